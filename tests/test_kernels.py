@@ -187,6 +187,30 @@ def test_gemm_plain_is_true_32_bit_and_batch_invariant(K):
     assert torch.equal(a[37], b[0])
 
 
+@pytest.mark.parametrize("K_dim", [1, 36, 131, 260])
+@pytest.mark.parametrize("M, N", [(1, 70), (4, 10007), (3, 4801), (8, 130), (7, 33), (16, 97), (17, 65), (33, 2113), (70, 131),
+                                  (1200, 1001), (2000, 2803)])
+def test_gemm_plain_shapes_agree_bit_for_bit(K, M, N, K_dim):
+    """Every shape of the 32-bit product (few rows, narrow and wide blocks, the three tile sizes, whole 16-byte pieces and
+    not) gives each row the bits that the row gets alone, and those lie within the error of K sums in 32 bits of the
+    64-bit product: |err| <= K 2^-24 sum |x w|, the bound of a chain of K fused multiply-adds."""
+    x, w = torch.randn(M, K_dim), torch.randn(N, K_dim)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    xd, wd = x.to(DEV), w.to(DEV)
+    K.gemm_plain(out, xd, wd)
+    err = (out.cpu().double() - x.double() @ w.double().T).abs()
+    assert bool((err <= (K_dim + 1) * 2.0 ** -24 * (x.abs().double() @ w.abs().double().T)).all())
+    for r in sorted({0, M // 2, M - 1}):
+        one = torch.empty(1, N, device=DEV)
+        K.gemm_plain(one, xd[r:r + 1].contiguous(), wd)
+        assert torch.equal(one[0], out[r])
+    wide = torch.empty(M, 3 * K_dim + 1, device=DEV)[:, :K_dim]       # rows apart, and not on 16 bytes
+    wide.copy_(xd)
+    again = torch.empty_like(out)
+    K.gemm_plain(again, wide, wd)
+    assert torch.equal(again, out)
+
+
 def _paged(k, v, order, n_pages, dtype):
     """Scatter k, v [T, nkv, hd] of one sequence into pages in the given order."""
     T, nkv, hd = k.shape
