@@ -1979,6 +1979,67 @@ def _delta_chunks(batch):
     return batch.aux["delta_chunks"]
 
 
+STATE_CHUNKS_AT_ONCE = 512     # chunks of 32 tokens whose scratch (up to 138 KB a head) is held at a time
+
+
+def state_chunks_supported(dk: int, dv: int, rank: int = 1) -> bool:
+    """Whether :func:`state_chunks` takes heads of these sizes (and a low-rank factor of ``rank`` rows)."""
+    return bool(_lib().af_state_chunks_supported(c_int(dk), c_int(dv), c_int(rank)))
+
+
+def state_chunks(mode: str, out, r, k, v, state, batch, heads: int, dk: int, dv: int, decay=None, silu: bool = False, a=None,
+                 low=None, a_bias=None, w0=None, w2t=None, decay_scale: float = 0.0, key_eps: float = 0.0) -> None:
+    """:func:`state_scan`'s rules ``decay`` and ``delta`` for a prefill step, the sequences cut into chunks of 32 tokens; every
+    sum in 32 bits, in another order.  ``delta`` works out unit keys, decays and removals itself, from the key rows, the
+    removals' logits ``a`` [T, heads * dk], the low-rank rows ``low`` [T, rank] and their weights (as :func:`delta_prep`)."""
+    T = out.shape[0]
+    n = heads * dk
+    delta = mode == "delta"
+    if mode not in ("decay", "delta"):
+        raise KernelError(f"state_chunks: unknown mode '{mode}'")
+    if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, dv, dk) or not state.is_contiguous():
+        raise KernelError(f"state_chunks: state must be contiguous float32 [slots, {heads}, {dv}, {dk}]")
+    for t, name, width in ((r, "r", n), (k, "k", n), (v, "v", heads * dv), (out, "out", heads * dv)) + (((a, "a", n),) if delta else ()):
+        if t is None or tuple(t.shape) != (T, width):
+            raise KernelError(f"state_chunks: {name} must be [{T}, {width}]")
+    f32, i32 = torch.float32, torch.int32
+    null = (ctypes.c_void_p(0), c_longlong(0))
+    if delta:
+        rank = w2t.shape[0]
+        if tuple(low.shape) != (T, rank) or tuple(w2t.shape) != (rank, n) or a_bias.numel() != n or w0.numel() != n:
+            raise KernelError(f"state_chunks: low [{T}, {rank}], w2t [{rank}, {n}] and biases of {n}")
+        extra = (*_f32_rows(a, "a"), *_f32_rows(low, "low"), _ptr(a_bias, "a_bias", f32), _ptr(w0, "w0", f32), _ptr(w2t, "w2t", f32),
+                 c_int(rank), c_float(decay_scale), c_float(key_eps), ctypes.c_void_p(0))
+    else:
+        if decay is None or decay.numel() != heads:
+            raise KernelError("state_chunks: one decay per head")
+        none = ctypes.c_void_p(0)
+        extra = (*null, *null, none, none, none, c_int(0), c_float(0.0), c_float(0.0), _ptr(decay, "decay", f32))
+    starts, first, _ = _delta_chunks(batch)
+    lib = _lib()
+    size = int(lib.af_state_chunks_size())
+    lib.af_state_chunks_scratch.restype = c_longlong
+    # the step's sequences in runs whose scratch fits what is held at a time (one launch pair a run; nearly always one run)
+    runs, chunk = [], 0
+    for s, length in enumerate(batch.seq_lens):
+        c = -(-length // size)
+        if runs and runs[-1][3] + c <= STATE_CHUNKS_AT_ONCE:
+            runs[-1][1] += 1
+            runs[-1][3] += c
+        else:
+            runs.append([s, 1, chunk, c])
+        chunk += c
+    most = max(run[3] for run in runs) * heads
+    blob, tiles = (torch.empty(most * lib.af_state_chunks_scratch(c_int(int(delta)), c_int(dk), c_int(dv), c_int(w)), dtype=f32,
+                               device=out.device) for w in (0, 1))
+    rp, kp, vp, op = (_f32_rows(t, name) for t, name in ((r, "r"), (k, "k"), (v, "v"), (out, "out")))
+    for s0, seqs, c0, chunks in runs:
+        _check(lib.af_state_chunks(c_int(int(delta)), *op, *rp, *kp, *vp, *extra, c_int(1 if silu else 0), _ptr(state), _ptr(blob),
+                                   _ptr(tiles), _ptr(starts[c0:], "chunk_starts", i32), _ptr(first[s0:], "seq_first_chunk", i32),
+                                   _ptr(batch.slots[s0:], "slots", i32), c_int(chunks), c_int(seqs), c_int(heads), c_int(dk),
+                                   c_int(dv), _ptr(error_word(out.device), "err", i32), _stream()))
+
+
 def delta_prompt(out, q, k, v, beta, z, dt_bias, rate, state, batch, heads: int, dk: int, dv: int, tile: int = 0) -> None:
     """:func:`state_scan`'s rule ``gated`` for a prefill step on the tensor cores, the sequences cut into chunks, with the
     decays exp(-rate softplus(z + dt_bias)) worked out from their logits ``z`` float32 [T, heads * dk]: q, k, v float32

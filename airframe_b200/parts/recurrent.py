@@ -1,7 +1,7 @@
 """Mixers that keep a state of fixed size per sequence instead of keys and
 values.  The state lives in the cache's per-sequence state (32-bit floats, zero
 when a sequence starts) and is carried from step to step; a prompt in one step
-and the same tokens one by one run the same recurrence token after token.
+and the same tokens one by one run the same recurrence (long bfloat16 prompts in chunks).
 
 ``general_delta``: the generalized delta rule.  Per head, with r, k, v of the
 token, a decay w per key channel, a removal rate a per key channel and the unit
@@ -93,6 +93,18 @@ class _StateMixer(Mixer):
         return torch.cat(mats, dim=0).contiguous(), offsets
 
 
+# Tokens of the longest prompt of a bfloat16 step whose recurrence goes in chunks.  The whole call, token by token against
+# in chunks, us: delta rule, 18 heads of 128: one prompt of 64 56 / 67, of 128 91 / 75, of 2,048 1,191 / 391; 16 prompts of
+# 33 235 / 236, of 128 866 / 418; linear attention 30 / 42, 50 / 45, 628 / 260, 84 / 105, 249 / 180; with 16 heads of 64 the
+# lines cross between 64 and 128 tokens as well.  (32-bit mode goes token by token: it is the plain recurrence.)
+CHUNKS_FROM = 128
+
+
+def _in_chunks(x, batch, dk: int, dv: int, rank: int = 1) -> bool:
+    return (x.dtype == torch.bfloat16 and batch.is_prefill and batch.max_len >= CHUNKS_FROM
+            and kernels.state_chunks_supported(dk, dv, rank))
+
+
 @register_part("mixer", "general_delta")
 class GeneralDelta(_StateMixer):
     """Parameters: ``hidden_size``, ``num_heads``, ``head_dim`` (keys and values),
@@ -149,13 +161,19 @@ class GeneralDelta(_StateMixer):
     def forward(self, x, batch, view):
         T, n, off = x.shape[0], self.n, self.off
         proj = linear(x, self.w_in, out_dtype=torch.float32)
-        pre = torch.empty(T, 3, n, dtype=torch.float32, device=x.device)
-        kernels.delta_prep(pre, proj, off["k"], off["a"], off["w1"], self.a_bias, self.w0, self.w2t, self.heads,
-                           self.hd, self.decay_scale, self.key_eps)
+        r, k, v = (proj[:, off[c]: off[c] + n] for c in ("r", "k", "v"))
         o = torch.empty(T, n, dtype=torch.float32, device=x.device)
-        kernels.state_scan("delta", o, proj[:, off["r"]: off["r"] + n], proj[:, off["k"]: off["k"] + n],
-                           proj[:, off["v"]: off["v"] + n], view.state, batch, self.heads, self.hd, self.hd,
-                           w=pre[:, 0], u=pre[:, 1], au=pre[:, 2])
+        if _in_chunks(x, batch, self.hd, self.hd, self.rank):
+            kernels.state_chunks("delta", o, r, k, v, view.state, batch, self.heads, self.hd, self.hd,
+                                 a=proj[:, off["a"]: off["a"] + n], low=proj[:, off["w1"]: off["w1"] + self.rank],
+                                 a_bias=self.a_bias, w0=self.w0, w2t=self.w2t, decay_scale=self.decay_scale,
+                                 key_eps=self.key_eps)
+        else:
+            pre = torch.empty(T, 3, n, dtype=torch.float32, device=x.device)
+            kernels.delta_prep(pre, proj, off["k"], off["a"], off["w1"], self.a_bias, self.w0, self.w2t, self.heads,
+                               self.hd, self.decay_scale, self.key_eps)
+            kernels.state_scan("delta", o, r, k, v, view.state, batch, self.heads, self.hd, self.hd,
+                               w=pre[:, 0], u=pre[:, 1], au=pre[:, 2])
         y = torch.empty(T, n, dtype=x.dtype, device=x.device)
         kernels.gated_group_norm(y, o, self.norm_w, proj[:, off["g"]: off["g"] + n], self.hd, self.eps)
         return linear_split(y, self.w_o, wide=self.wide)
@@ -209,9 +227,9 @@ class LightningAttention(_StateMixer):
         nk, nv = self.heads * self.dk, self.heads * self.dv
         proj = linear(x, self.w_in, out_dtype=torch.float32)
         o = torch.empty(T, nv, dtype=torch.float32, device=x.device)
-        kernels.state_scan("decay", o, proj[:, off["q"]: off["q"] + nk], proj[:, off["k"]: off["k"] + nk],
-                           proj[:, off["v"]: off["v"] + nv], view.state, batch, self.heads, self.dk, self.dv,
-                           decay=self.decay, silu=True)
+        scan = kernels.state_chunks if _in_chunks(x, batch, self.dk, self.dv) else kernels.state_scan
+        scan("decay", o, proj[:, off["q"]: off["q"] + nk], proj[:, off["k"]: off["k"] + nk],
+             proj[:, off["v"]: off["v"] + nv], view.state, batch, self.heads, self.dk, self.dv, decay=self.decay, silu=True)
         y = torch.empty(T, nv, dtype=x.dtype, device=x.device)
         kernels.gated_group_norm(y, o, self.norm_w, proj[:, off["g"]: off["g"] + nv], nv, self.eps)
         return linear_split(y, self.w_o, wide=self.wide)

@@ -230,3 +230,108 @@ def test_weighted_residual_sum_and_norm():
     x = x0.to(DEV)
     kernels.add_scaled_rmsnorm(x, [(parts.to(DEV), 1.0), (a.to(DEV), 1.0), (a.to(DEV), -1.0)])
     close(x, x0.double() + parts.double().sum(0), 1e-6)
+
+
+CHUNK_LENS = [1, 16, 17, 31, 32, 33, 64, 95, 230]      # tokens at and around the borders of groups of 16 and chunks of 32
+
+
+def prompt_batch(lens, slots):
+    b = batch_of(lens, slots)
+    b.seq_lens, b.tokens, b.aux = lens, b.slots, {}
+    return b
+
+
+def in_order(lens):
+    at = 0
+    for n in lens:
+        yield slice(at, at + n), n
+        at += n
+
+
+@pytest.mark.parametrize("at_once", [512, 3])
+@pytest.mark.parametrize("heads,dk,dv,rank,scale", [(2, 16, 16, 5, math.exp(-0.5)), (3, 48, 32, 64, 0.01), (1, 64, 80, 128, 2.0),
+                                                    (2, 128, 128, 64, math.exp(-0.5)), (1, 112, 16, 1, 200.0)])
+def test_general_delta_in_chunks(heads, dk, dv, rank, scale, at_once, monkeypatch):
+    """Prompts in chunks against the plain rule in 64 bits and against the token-by-token kernels, then more tokens from the
+    states they left; decays from none to (scale 200) all at once; sequences in one launch and in several.  Bounds: the
+    recurrence's sums are of up to 128 products of 32 bits, a few thousand roundings of 2^-24 at most: 2e-5 of the largest value."""
+    from airframe_b200 import kernels
+    assert kernels.state_chunks_supported(dk, dv, rank) and not kernels.state_chunks_supported(dk + 8, dv, rank)
+    assert not kernels.state_chunks_supported(dk, dv + 8, rank) and not kernels.state_chunks_supported(dk, dv, 129)
+    monkeypatch.setattr(kernels, "STATE_CHUNKS_AT_ONCE", at_once)
+    T, n = sum(CHUNK_LENS), heads * dk
+    g = torch.Generator().manual_seed(dk + rank)
+    widths = {"r": n, "k": n, "v": heads * dv, "a": n, "w1": rank}
+    cols, at = {}, 4
+    for name, w in widths.items():
+        cols[name] = slice(at, at + w)
+        at += (w + 3) // 4 * 4
+    proj = torch.randn(T, (at + 3) // 4 * 4, generator=g)
+    a_bias, w0 = torch.randn(n, generator=g), torch.randn(n, generator=g)
+    w2 = torch.randn(n, rank, generator=g) * rank ** -0.5
+    slots = [4, 0, 8, 2, 1, 3, 7, 5, 6]
+    state = torch.zeros(10, heads, dv, dk, device=DEV)
+    p = {name: proj.to(DEV)[:, c] for name, c in cols.items()}
+    consts = {"a_bias": a_bias.to(DEV), "w0": w0.to(DEV), "w2t": w2.t().contiguous().to(DEV)}
+    out = torch.full((T, heads * dv), 7.0, device=DEV)
+
+    def chunks(rows, o, lens, where):
+        kernels.state_chunks("delta", o, p["r"][rows], p["k"][rows], p["v"][rows], state, prompt_batch(lens, where), heads, dk, dv,
+                             a=p["a"][rows], low=p["w1"][rows], decay_scale=scale, key_eps=1e-6, **consts)
+
+    chunks(slice(0, T), out, CHUNK_LENS, slots)
+    pd = {name: proj.double()[:, c] for name, c in cols.items()}
+    w = torch.exp(-scale * plain.sigmoid(torch.tanh(pd["w1"]) @ w2.double().T + w0.double()))
+    a = plain.sigmoid(pd["a"] + a_bias.double())
+    for (s, length), slot in zip(in_order(CHUNK_LENS), slots):
+        o, S = plain.delta_rule(*(t[s].view(length, heads, -1) for t in (pd["r"], pd["k"], pd["v"], w, a)))
+        close(out[s], o.reshape(length, -1))
+        close(state[slot].transpose(1, 2), S)
+    assert float(state[9].abs().sum()) == 0
+    # token by token, and the last prompt again in two steps
+    pre = torch.empty(T, 3, n, device=DEV)
+    kernels.delta_prep(pre, proj.to(DEV), cols["k"].start, cols["a"].start, cols["w1"].start, consts["a_bias"], consts["w0"],
+                       consts["w2t"], heads, dk, scale, 1e-6)
+    twin, other = torch.empty_like(out), torch.zeros_like(state)
+    kernels.state_scan("delta", twin, p["r"], p["k"], p["v"], other, batch_of(CHUNK_LENS, slots), heads, dk, dv, w=pre[:, 0],
+                       u=pre[:, 1], au=pre[:, 2])
+    close(out, twin.cpu())
+    close(state, other.cpu())
+    last = list(in_order(CHUNK_LENS))[-1][0]
+    whole = out[last].clone()
+    state[6].zero_()
+    for rows in (slice(last.start, last.start + 77), slice(last.start + 77, last.stop)):
+        o = torch.empty(rows.stop - rows.start, heads * dv, device=DEV)
+        chunks(rows, o, [len(o)], [6])
+        close(o, whole[rows.start - last.start: rows.stop - last.start].cpu())
+
+
+@pytest.mark.parametrize("heads,dk,dv,silu", [(3, 16, 32, True), (2, 64, 64, False), (4, 128, 128, True), (2, 96, 144, True)])
+def test_decay_attention_in_chunks(heads, dk, dv, silu):
+    """Prompts in chunks against the plain rule in 64 bits, sections of one wider row; the states go on in a second step."""
+    from airframe_b200 import kernels
+    T, n = sum(CHUNK_LENS), heads * dk
+    g = torch.Generator().manual_seed(dk + 7 * dv)
+    proj = torch.randn(T, 8 + 2 * n + heads * dv, generator=g)
+    cols = slice(4, 4 + n), slice(4 + n, 4 + 2 * n), slice(8 + 2 * n, None)
+    decay = torch.tensor([1.0, 0.0, 0.97, 0.999][:heads])
+    slots = [4, 0, 8, 2, 1, 3, 7, 5, 6]
+    state = torch.zeros(10, heads, dv, dk, device=DEV)
+    out = torch.full((T, heads * dv), 7.0, device=DEV)
+    dev = [proj.to(DEV)[:, c] for c in cols]
+    act = plain.silu if silu else (lambda x: x)
+    ref = [act(proj.double()[:, c]) for c in cols]
+
+    def run(rows, lens, where):
+        kernels.state_chunks("decay", out[rows], *(t[rows] for t in dev), state, prompt_batch(lens, where), heads, dk, dv,
+                             decay=decay.to(DEV), silu=silu)
+
+    run(slice(0, T), CHUNK_LENS, slots)
+    for s, length in in_order(CHUNK_LENS):
+        close(out[s], plain.decay_linear_attention(*(t[s].view(length, heads, -1) for t in ref), decay.double()).reshape(length, -1))
+    last = list(in_order(CHUNK_LENS))[-1][0]
+    whole = out[last].clone()
+    state[6].zero_()
+    for rows in (slice(last.start, last.start + 77), slice(last.start + 77, last.stop)):
+        run(rows, [rows.stop - rows.start], [6])
+    close(out[last], whole.cpu())
