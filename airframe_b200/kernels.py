@@ -200,6 +200,39 @@ def gemm_plain(out, x, w, cap: float = 0.0) -> None:
                                 _stream()))
 
 
+# From how many rows, and how many multiply-adds, a 32-bit product goes to the tensor cores.  The CUDA cores' kernel and this
+# one, us (N x K, rows): 18432 x 2304: 32 94 / 92, 64 159 / 102, 301 597 / 182; 2304 x 9216: 32 89 / 87, 64 175 / 102, 301
+# 444 / 115; 4096 x 2304: 64 60 / 70, 128 89 / 72, 301 192 / 83; 2304 x 2048: 128 56 / 56, 160 80 / 65; 8192 x 512: 64 30 / 40,
+# 301 86 / 51; 1024 x 1024: 301 46 / 57, 1000 78 / 55: the lines cross at some 10^9.
+F32_TC_ROWS = 64
+F32_TC_WORK = 1 << 30
+
+
+def gemm_f32_tc_supported(x, w, out) -> bool:
+    """Whether :func:`gemm_f32_tc` takes these and is the kernel for them."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32
+            and F32_TC_ROWS <= x.shape[0] <= 65535 and x.shape[0] * w.numel() >= F32_TC_WORK
+            and x.shape[1] % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1
+            and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and (x.data_ptr() | w.data_ptr()) % 16 == 0)
+
+
+def gemm_f32_tc(out, x, w, cap: float = 0.0) -> None:
+    """out[M, N] = x[M, K] @ w[N, K]^T, all float32, on the tensor cores: operands in three bfloat16 parts that hold all 24 bits,
+    sums of 64 products joined in 32 bits in index order."""
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K or out.shape != (M, N) or not (x.dtype == w.dtype == out.dtype == torch.float32):
+        raise KernelError(f"gemm_f32_tc: shapes {tuple(x.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)}, all float32")
+    splits = _lib().af_gemm_f32_tc_splits(c_int(N), c_int(K))
+    if splits < 1:
+        _check(splits or -1)
+    parts = torch.empty(3 * M * ((K + 63) // 64 * 64), dtype=torch.bfloat16, device=x.device)
+    sums = torch.empty(splits * M * N, dtype=torch.float32, device=x.device) if splits > 1 else None
+    _check(_lib().af_gemm_f32_tc(_ptr(out), c_longlong(_rows(out, "out")), _ptr(x), c_longlong(_rows(x, "x")), _ptr(w),
+                                 c_longlong(_rows(w, "w")), c_int(M), c_int(N), c_int(K), c_float(cap), _ptr(parts),
+                                 _ptr(sums, allow_none=True), _ptr(error_word(x.device), "err", torch.int32), _stream()))
+
+
 # ---------------------------------------------------------------- attention
 
 def kv_keep(kv) -> int:

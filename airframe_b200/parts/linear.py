@@ -1,6 +1,7 @@
 """y = x W^T for a weight [out, in]: picks the matrix-product kernel.
 
-float32: the plain CUDA-core kernel (true 32-bit).  bfloat16: the tensor-core
+float32: the plain CUDA-core kernel (true 32-bit), and for prompts the tensor
+cores with operands in three parts that hold all their bits.  bfloat16: the tensor-core
 kernels where they take the sizes, the plain kernel (bfloat16 operands, 32-bit
 accumulators) otherwise.
 """
@@ -20,6 +21,8 @@ def linear(x, w, out_dtype=None, cap: float = 0.0, out=None):
         out = torch.empty(M, N, dtype=out_dtype or x.dtype, device=x.device)
     if kernels.gemm_tc_supported(x, w, out):
         kernels.gemm_tc(out, x, w, cap, checked=True)
+    elif kernels.gemm_f32_tc_supported(x, w, out):
+        kernels.gemm_f32_tc(out, x, w, cap)
     else:
         kernels.gemm_plain(out, x, w, cap)
     return out

@@ -211,6 +211,58 @@ def test_gemm_plain_shapes_agree_bit_for_bit(K, M, N, K_dim):
     assert torch.equal(again, out)
 
 
+@pytest.mark.parametrize("K_dim", [4, 60, 64, 132, 1000, 2304, 9216])
+@pytest.mark.parametrize("M, N", [(1, 128), (32, 1), (33, 129), (100, 260), (160, 127), (161, 4096), (301, 2304)])
+def test_gemm_f32_on_the_tensor_cores(K, M, N, K_dim):
+    """Edges of tiles, K blocks, splits and their joins; rows apart; a row's bits do not depend on the rows beside it.  Bound: a
+    product loses 2^-22 at most (what the parts leave out), a block of 64 is 24 additions that round towards zero (2^-23 of
+    the block's sum of |x w| each), the blocks are joined by K / 64 additions that round to nearest: together below
+    (56 + K / 64) 2^-24 sum |x w|.  And in the 2-norm it is no further off than the chain of fused multiply-adds."""
+    x, w = torch.randn(M, K_dim), torch.randn(N, K_dim) * 0.02
+    ref, size = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
+    wide = torch.full((M, K_dim + 8), float("nan"), device=DEV)
+    wide[:, 4:4 + K_dim] = x
+    xd, wd = wide[:, 4:4 + K_dim], w.to(DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    K.gemm_f32_tc(out, xd, wd)
+    assert bool(((out.cpu().double() - ref).abs() <= (56 + K_dim / 64) * 2.0 ** -24 * size).all())
+    chain = torch.empty_like(out)
+    K.gemm_plain(chain, xd, wd)
+    off, off_chain = (float((t.cpu().double() - ref).norm()) for t in (out, chain))
+    if K_dim >= 1000 and M * N > 1000:
+        assert off <= off_chain, (off, off_chain)
+    K.gemm_f32_tc(chain, xd, wd, cap=2.0)
+    close(chain, plain.softcap(ref, 2.0), torch.float32)
+    one = torch.empty(1, N, device=DEV)
+    for r in sorted({0, M // 2, M - 1}):
+        K.gemm_f32_tc(one, xd[r:r + 1], wd)
+        assert torch.equal(one[0], out[r])
+
+
+def test_gemm_f32_on_the_tensor_cores_beyond_finite_values(K):
+    """Infinities, NaN, sums that overflow and the largest values come out as a chain of multiply-adds has them; values near
+    the smallest lose nothing that counts (the parts reach as far down as the values)."""
+    x, w = torch.randn(40, 200), torch.randn(130, 200)
+    x[1, 3], x[2, 7], x[3, 190], x[4, 5], x[4, 6] = math.inf, -math.inf, math.nan, math.inf, -math.inf
+    x[5], x[6, 0] = 3e38, 3.4028234e38
+    x[7] *= 1e-30
+    w[0], w[1, 3], w[2, 100] = 1.0, 0.0, math.inf
+    w[3] = 2.0 ** torch.randint(-3, 3, (200,)).float()
+    out, chain = torch.empty(40, 130, device=DEV), torch.empty(40, 130, device=DEV)
+    K.gemm_f32_tc(out, x.to(DEV), w.to(DEV))
+    K.gemm_plain(chain, x.to(DEV), w.to(DEV))
+    out, chain = out.cpu(), chain.cpu()
+    rows = [r for r in range(40) if r not in (5, 6)]      # (a chain may overflow on its way to a finite sum: another order need not)
+    assert torch.equal(out[rows].isnan(), chain[rows].isnan()) and torch.equal(out[rows].isinf(), chain[rows].isinf())
+    assert torch.equal(out[rows][chain[rows].isinf()], chain[rows][chain[rows].isinf()])
+    assert bool(out[5, 0] == math.inf) and bool(out[5, 2].isinf() or out[5, 2].isnan())
+    fin = chain.isfinite()
+    fin[[5, 6]] = False
+    ref = x.double() @ w.double().T
+    size = x.abs().double() @ w.abs().double().T
+    assert bool(((out.double() - ref).abs()[fin] <= 64 * 2.0 ** -24 * size[fin]).all())
+
+
 def _paged(k, v, order, n_pages, dtype):
     """Scatter k, v [T, nkv, hd] of one sequence into pages in the given order."""
     T, nkv, hd = k.shape
