@@ -13,17 +13,20 @@
 //   warps 0 .. 7   weights: global -> registers (a stage ahead) -> three swizzled tiles; the sums: TMEM -> registers
 //   warp 8         TMEM, MMA issue (one lane)
 //   warp 9         TMA (one lane)
-// Two stages of 64 of K, two accumulators in turn.  Bound by shared memory (an MMA of 128 x 160 x 16 reads 9 KB of it in 80
-// cycles of products; the parts are written besides): 301 x 18432 x 2304 in 182 us (140 TFLOP/s
-// of 32-bit products), where the CUDA cores' kernel (gemm_plain.cu), which keeps the few rows and the small products, takes
-// 597.
+// Two stages of 64 of K, two accumulators in turn.  Bound by the worker warps' instructions (taking a value apart, five and a
+// half each) and, with 160 tokens, by shared memory (an MMA of 128 x 160 x 16 reads 9 KB of it in 80 cycles of products; the
+// parts are written besides).  301 x 18432 x 2304: 132 us (194 TFLOP/s of 32-bit products), where the CUDA cores' kernel
+// (gemm_plain.cu), which keeps the few rows and the small products, takes 592; before the rare values left the way (182 us:
+// a test a value, and the exact chain unrolled into the epilogue), weights were asked into L2 ahead, and TMEM was read
+// 32 columns at a time.
 //
-// An output that is not finite is made again as a plain chain of fmaf: inf times a part that is zero would be NaN.
+// An output that is not finite is made again as a plain chain of fmaf (the parts of an infinity are NaN).
 #include "umma.cuh"
 
 namespace {
 
 constexpr int FT_BM = 128, FT_BK = 64, FT_STAGES = 2;
+constexpr int FT_AHEAD = 4;                                // K blocks between a weight's way into L2 and into registers
 constexpr int FT_WORKERS = 256, FT_THREADS = FT_WORKERS + 64;
 constexpr int FT_PART = FT_BM * FT_BK * 2;                 // bytes of a part of a weight tile
 
@@ -49,11 +52,7 @@ __device__ __forceinline__ void ft_split(float x, uint32_t& hi, uint32_t& mid, u
   hi = b & 0xffff0000u;
   const float r1 = x - __uint_as_float(hi);
   mid = __float_as_uint(r1) & 0xffff0000u;
-  lo = __float_as_uint(r1 - __uint_as_float(mid));
-  if ((b & 0x7f800000u) == 0x7f800000u) {                  // inf, NaN: whole in the first part
-    hi = (b & 0x007fffffu) ? 0x7fc00000u : b;
-    mid = lo = 0u;
-  }
+  lo = __float_as_uint(r1 - __uint_as_float(mid));         // (inf and NaN leave NaN: their outputs are made again)
 }
 __device__ __forceinline__ uint32_t ft_pack(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
 
@@ -133,6 +132,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, FtArgs a) {
         q[i] = (n0 + wr + 16 * i < a.N && k + wk < a.K) ? *reinterpret_cast<const float4*>(src + (size_t)(16 * i) * a.ldw + k)
                                                          : make_float4(0.f, 0.f, 0.f, 0.f);
     };
+    // (and asked into L2 well ahead: a line a thread)
+    const float* line = a.w + (size_t)(n0 + (tid >> 1)) * a.ldw + (tid & 1) * 32;
+    auto ask = [&](int kb) {
+      const int k = (kb0 + kb) * FT_BK;
+      if (kb < count && n0 + (tid >> 1) < a.N && k + (tid & 1) * 32 < a.K) prefetch_l2(line + k);
+    };
     const int quarter = warp & 3, col0 = (warp >> 2) * HALF;
     float acc[HALF];
 #pragma unroll
@@ -146,18 +151,20 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, FtArgs a) {
       tc_fence_after();
       const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col0;
 #pragma unroll
-      for (int c = 0; c < HALF; c += 16) {
-        float v[16];
+      for (int c = 0; c < HALF; c += 32) {
+        float v[32];
         tmem_ld16(at + c, v);
+        if (c + 16 < HALF) tmem_ld16(at + c + 16, v + 16);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[c + j] += v[j];
+        for (int j = 0; j < 32 && c + j < HALF; ++j) acc[c + j] += v[j];
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);
     };
     fetch(0);                                              // (weights: they wait for nothing)
+    for (int kb = 1; kb < FT_AHEAD; ++kb) ask(kb);
     pdl_wait();
     for (int kb = 0; kb < count && ok; ++kb) {
       const int s = kb % FT_STAGES;
@@ -178,6 +185,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, FtArgs a) {
       __syncwarp();
       if (lane == 0) mbar_arrive(&full_w[s]);
       if (kb + 1 < count) fetch(kb + 1);
+      ask(kb + FT_AHEAD);
       if (kb > 0) add_up(kb - 1);
     }
     if (ok && count > 0) add_up(count - 1);
@@ -185,17 +193,25 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, FtArgs a) {
     if (ok && f < a.N) {
       float* o = a.out + (size_t)blockIdx.z * a.split_stride + f;
       const int k0 = kb0 * FT_BK, k1 = min(a.K, k0 + count * FT_BK);
+      bool again = a.cap > 0.f;
 #pragma unroll
       for (int j = 0; j < HALF; ++j) {
-        const int m = m0 + col0 + j;
-        if (m >= a.M) continue;
-        float v = acc[j];
-        if (!isfinite(v)) {
-          const float *xr = a.x + (size_t)m * a.ldx, *wrow = a.w + (size_t)f * a.ldw;
-          v = 0.f;
-          for (int k = k0; k < k1 && !isnan(v); ++k) v = fmaf(xr[k], wrow[k], v);
+        if (m0 + col0 + j < a.M) o[(size_t)(m0 + col0 + j) * a.ldo] = acc[j];
+        again = again || !isfinite(acc[j]);
+      }
+      // what is seldom: in a rolled loop over what was just written (as straight code in the loop above it cost every
+      // block 25 us of instruction fetches)
+      if (again) {
+#pragma unroll 1
+        for (int m = m0 + col0; m < min(a.M, m0 + col0 + HALF); ++m) {
+          float v = o[(size_t)m * a.ldo];
+          if (!isfinite(v)) {
+            const float *xr = a.x + (size_t)m * a.ldx, *wrow = a.w + (size_t)f * a.ldw;
+            v = 0.f;
+            for (int k = k0; k < k1 && !isnan(v); ++k) v = fmaf(xr[k], wrow[k], v);
+          }
+          o[(size_t)m * a.ldo] = softcap_f32(v, a.cap);
         }
-        o[(size_t)m * a.ldo] = softcap_f32(v, a.cap);
       }
     }
   } else if (warp == 8) {

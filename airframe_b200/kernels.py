@@ -201,11 +201,11 @@ def gemm_plain(out, x, w, cap: float = 0.0) -> None:
 
 
 # From how many rows, and how many multiply-adds, a 32-bit product goes to the tensor cores.  The CUDA cores' kernel and this
-# one, us (N x K, rows): 18432 x 2304: 32 94 / 92, 64 159 / 102, 301 597 / 182; 2304 x 9216: 32 89 / 87, 64 175 / 102, 301
-# 444 / 115; 4096 x 2304: 64 60 / 70, 128 89 / 72, 301 192 / 83; 2304 x 2048: 128 56 / 56, 160 80 / 65; 8192 x 512: 64 30 / 40,
-# 301 86 / 51; 1024 x 1024: 301 46 / 57, 1000 78 / 55: the lines cross at some 10^9.
-F32_TC_ROWS = 64
-F32_TC_WORK = 1 << 30
+# one, us (N x K, rows): 18432 x 2304: 32 91 / 74, 64 158 / 73, 301 592 / 132; 2304 x 9216: 32 88 / 68, 301 438 / 82;
+# 4096 x 2304: 32 54 / 47, 64 59 / 48, 301 192 / 61; 2304 x 2048: 32 34 / 37, 64 48 / 36, 301 108 / 41; 1024 x 1024: 160 32 / 37,
+# 301 45 / 36: the lines cross between 2^27 and 2^28.
+F32_TC_ROWS = 32
+F32_TC_WORK = 1 << 28
 
 
 def gemm_f32_tc_supported(x, w, out) -> bool:
