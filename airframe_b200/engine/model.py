@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from ..config.base import ConfigError, ModelSpec
-from ..parts import Block, BuildContext, build_part
+from ..parts import Block, BuildContext, build_part, prompt_run
 
 
 def _build_layers(spec: ModelSpec, ctx: BuildContext):
@@ -41,6 +41,7 @@ class Model:
                 raise ConfigError(f"a block of kind '{b.kind}' keeps {getattr(b, 'streams', 1)} residual streams, "
                                   f"the model {self.streams}")
         self.loaded = False
+        self.prompts_as_one = False      # (a prompt's layers launched by one call: see parts/prompt_run.py)
 
     # ------------------------------------------------------------------ weights
 
@@ -70,6 +71,7 @@ class Model:
                 by_class.setdefault(type(part), []).append(part)
         for cls, parts in by_class.items():
             cls.link(parts)
+        self.prompts_as_one = self.ctx.device.type == "cuda" and prompt_run.supported(self)
         self.loaded = True
 
     @property
@@ -128,6 +130,8 @@ class Model:
             one = x
             x = torch.empty(one.shape[0], self.streams * one.shape[1], dtype=torch.float32, device=one.device)
             kernels.stream_copy(x, one, self.streams)
+        if batch.is_prefill and probe is None and self.prompts_as_one and prompt_run.run(self, x, batch, cache):
+            return x
         sched = self.spec.schedule
         # a junction sees the embedding's output beside the stream (which the layers rewrite in place)
         x0 = x.clone() if any(e.enter is not None for e in sched) else None

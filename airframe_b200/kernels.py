@@ -479,6 +479,23 @@ def gemm_tc_splits(M: int, N: int, K: int) -> int:
     return (kb + per - 1) // per
 
 
+def gemm_tc_accumulators(M: int, rows: int, K: int, splits: int) -> int:
+    """Weight tiles a block of the product works at once: 1, 2, or 4 for the kernel on pairs of SMs.
+
+    Many tokens: two weight tiles per block halve the bytes a block stages per flop; worth it once the
+    tiles of 256 x 256 fill the GPU.  With fewer tiles and a long K a tile runs on a pair of SMs (the same
+    bytes per flop, 128 rows a block); with a short K the pair's set-up costs what it saves.  Measured at
+    2,048 tokens on a B200: 18432 x 2304 gated 122 us / 124 us / 132 us (two tiles / pair / one tile),
+    2304 x 9216 90 / 59 / 63, 2304 x 2048 25 / 17 / 15, 4096 x 2304 31 / 31 / 31."""
+    if M > 128 and splits == 1:
+        blocks2 = ((rows + 255) // 256) * ((M + 255) // 256)
+        if blocks2 >= 120:
+            return 2
+        if blocks2 >= 60 and K >= 4096:
+            return 4
+    return 1
+
+
 # Blocks per SM of the weight-bound product (up to 64 tokens): 0 lets the library choose.
 GEMM_TC_PER_SM = 0
 
@@ -508,18 +525,7 @@ def gemm_tc(out, x, w, cap: float = 0.0, splits: int = 1, gated: bool = False, a
             raise KernelError(f"gemm_tc: output shape {tuple(out.shape)}, expected {(M, N)}")
         ldo, part = out.stride(0), 0
     if n_acc == 0:
-        # Many tokens.  Two weight tiles per block halve the bytes a block stages per flop; worth it once the
-        # tiles of 256 x 256 fill the GPU.  With fewer tiles and a long K a tile runs on a pair of SMs (the same
-        # bytes per flop, 128 rows a block); with a short K the pair's set-up costs what it saves.  Measured at
-        # 2,048 tokens on a B200: 18432 x 2304 gated 122 us / 124 us / 132 us (two tiles / pair / one tile),
-        # 2304 x 9216 90 / 59 / 63, 2304 x 2048 25 / 17 / 15, 4096 x 2304 31 / 31 / 31.
-        blocks2 = ((rows + 255) // 256) * ((M + 255) // 256)
-        n_acc = 1
-        if M > 128 and splits == 1:
-            if blocks2 >= 120:
-                n_acc = 2
-            elif blocks2 >= 60 and K >= 4096:
-                n_acc = 4
+        n_acc = gemm_tc_accumulators(M, rows, K, splits)
     if n_acc == 4:
         if splits > 1:
             raise KernelError("gemm_tc: the kernel on pairs of SMs does not split K")
@@ -679,6 +685,19 @@ def attn_prefill_mma(out, q, k, v, seq_starts, n_seqs: int, max_len: int, nq, nk
         c_longlong(_rows(k, "k")), _ptr(v), c_longlong(_rows(v, "v")), _ptr(seq_starts, "seq_starts", torch.int32),
         c_int(n_seqs), c_int(max_len), c_int(nq), c_int(nkv), c_int(hd), c_float(scale), c_float(cap), c_int(window),
         c_int(keep), _ptr(sinks, "sinks", torch.float32, allow_none=True), gp, gs, _stream()))
+
+
+def attn_prefill_tc_supported(hd: int) -> bool:
+    """Whether :func:`attn_prefill_tc` takes heads of this size."""
+    return bool(_lib().af_attn_prefill_tc_supported(c_int(hd)))
+
+
+def prompt_layers(step: bytes, runs: bytes, n_runs: int) -> None:
+    """All launches of a prompt's layers (``step`` and ``runs`` as ``csrc/prompt_layers.cu`` lays them out)."""
+    lib = _lib()
+    if len(step) != lib.af_prompt_layers_sizes(c_int(1)) or len(runs) != n_runs * lib.af_prompt_layers_sizes(c_int(0)):
+        raise KernelError("prompt_layers: records of another size than the library's")
+    _check(lib.af_prompt_layers(ctypes.c_char_p(step), ctypes.c_char_p(runs), c_int(n_runs), _stream()))
 
 
 def attn_prefill_tc(out, q, k, v, seq_starts, n_seqs: int, max_len: int, nq, nkv, hd, scale, cap, window,

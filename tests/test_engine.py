@@ -115,6 +115,38 @@ def test_the_same_work_gives_the_same_bits(case, dtype):
     assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("lens", [[1], [17], [64], [130], [210], [3, 64, 1, 40, 33], [5, 5]])
+def test_prompt_layers_launched_by_one_call(case, lens):
+    """Where a model's prompts go through one call into the library, logits and cache pages are those of the same kernels
+    launched part by part, bit for bit, and as many kernels run; other models do not go that way."""
+    from airframe_b200 import kernels
+    from airframe_b200.engine import StepEntry
+    rt = runtime(case, "bfloat16")
+    model, engine = rt.model, rt.engine
+    assert model.prompts_as_one == (case["cfg"]["head_dim"] in (128, 256) and case["cfg"]["hidden_size"] % 8 == 0
+                                    and case["cfg"]["intermediate_size"] % 16 == 0)
+    assert not runtime(case, "float32").model.prompts_as_one
+    if not model.prompts_as_one:
+        return
+    prompts = [replay.random_ids(case["cfg"]["vocab_size"], min(n, case["cfg"]["max_position_embeddings"]), 7 + i) for i, n in enumerate(lens)]
+    got = []
+    for as_one in (True, False):
+        model.prompts_as_one = as_one
+        try:
+            rt.reset()
+            slots = [engine.take_slot() for _ in prompts]
+            before = kernels.launch_count()
+            logits = rt.step([StepEntry(s, p, [0, len(p) - 1]) for s, p in zip(slots, prompts)])
+            launched = kernels.launch_count() - before
+            more = rt.step([StepEntry(s, [5], [0]) for s in slots]).clone()       # reads the pages that the prompts left
+            got.append((logits, more, launched))
+        finally:
+            model.prompts_as_one = True
+            for s in slots:
+                engine.free_slot(s)
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and got[0][2] == got[1][2] > 0
+
+
 def test_decode_steps_fed_from_the_device(case, dtype):
     """``decode_rows``: the step's tokens lie on the device, rows keep their places and a row may be
     unused; the logits are those of the same step fed from the host."""
