@@ -777,22 +777,23 @@ AF_EXPORT int af_gated_group_norm(void* y, int y_dtype, const float* o, const fl
 
 // Per channel: z = sigmoid(pz + bz), c = px + bx, candidate = c + 1/2 where c >= 0 and sigmoid(c) below,
 // S <- (1 - z) S + z candidate, y = S * silu(pg).  pz, px, pg are sections of the packed projection row.
-// A block owns 32 channels of a sequence (a lane each) and walks its tokens 128 at a time: warp w takes 16
-// tokens in a row, works out what they do to any state that enters them (S_out = A S_in + B: the map of a
-// token is affine, and so is their composition), the warps exchange these pairs, each warp composes the pairs
-// of the warps before it onto the state carried so far, and then walks its 16 tokens once more from the state
-// that really enters them.  The gates and candidates of the 16 tokens stay in registers between the passes.
-#define AF_GS_WARPS 8
-#define AF_GS_RUN 16
-template <typename TY>
-__global__ void __launch_bounds__(AF_GS_WARPS * 32)
+// A block owns CH channels of a sequence and walks its tokens RUNS * RUN at a time: a thread takes a run of RUN
+// tokens of a channel, works out what they do to any state that enters them (S_out = A S_in + B: the map of a
+// token is affine, and so is their composition), the threads exchange these pairs, each composes the pairs
+// of the runs before its own onto the state carried so far, and then walks its tokens once more from the state
+// that really enters them.  The gates and candidates of a run stay in registers between the passes.
+// Two shapes: 32 channels by 8 runs of 16 for few tokens a sequence; for prompts 16 channels by 32 runs of 8, a block of
+// 512 threads: twice the blocks, twice the warps in each, half the chain.  One prompt of 2,048 tokens of 2,304 channels (66 MB:
+// 10 us): 124 -> 63 us.
+template <typename TY, int CH, int RUNS, int RUN>
+__global__ void __launch_bounds__(CH * RUNS)
 gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long ld, int off_z, int off_x, int off_g,
                   const float* __restrict__ bz, const float* __restrict__ bx, float* __restrict__ state,
                   const int* __restrict__ seq_starts, const int* __restrict__ slots, int width) {
   pdl_launch_dependents();
-  __shared__ float comp[AF_GS_WARPS][32][2];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
+  __shared__ float2 comp[RUNS][CH];
+  const int lane = threadIdx.x % CH, w = threadIdx.x / CH;
+  const int c = blockIdx.x * CH + lane;
   const int b = blockIdx.y;
   const bool on = c < width;
   const int first = seq_starts[b], last = seq_starts[b + 1];
@@ -801,16 +802,16 @@ gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long 
   pdl_wait();
   if (slot < 0) {
     if (on)
-      for (int t = first + w; t < last; t += AF_GS_WARPS) y[(size_t)t * width + c] = from_f32<TY>(0.f);
+      for (int t = first + w; t < last; t += RUNS) y[(size_t)t * width + c] = from_f32<TY>(0.f);
     return;
   }
   float carry = on ? state[(size_t)slot * width + c] : 0.f;
-  for (int base = first; base < last; base += AF_GS_WARPS * AF_GS_RUN) {
-    const int t0 = base + w * AF_GS_RUN;
-    const int n = max(0, min(AF_GS_RUN, last - t0));
-    float z[AF_GS_RUN], cd[AF_GS_RUN], g[AF_GS_RUN];
+  for (int base = first; base < last; base += RUNS * RUN) {
+    const int t0 = base + w * RUN;
+    const int n = max(0, min(RUN, last - t0));
+    float z[RUN], cd[RUN], g[RUN];
 #pragma unroll
-    for (int e = 0; e < AF_GS_RUN; ++e) {
+    for (int e = 0; e < RUN; ++e) {
       const bool in = on && e < n;
       const float* row = proj + (size_t)(t0 + e) * ld + c;
       z[e] = in ? row[off_z] : 0.f;
@@ -819,7 +820,7 @@ gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long 
     }
     float A = 1.f, B = 0.f;
 #pragma unroll
-    for (int e = 0; e < AF_GS_RUN; ++e) {
+    for (int e = 0; e < RUN; ++e) {
       if (e < n) {
         const float zz = 1.f / (1.f + expf(-(z[e] + zb)));
         const float u = cd[e] + xb;
@@ -829,18 +830,19 @@ gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long 
         B = (1.f - zz) * B + zz * cd[e];
       }
     }
-    comp[w][lane][0] = A;
-    comp[w][lane][1] = B;
+    comp[w][lane] = make_float2(A, B);
     __syncthreads();
-    // the state that enters this warp's tokens, and the one that leaves the stretch (the same in every warp)
+    // the state that enters this run, and the one that leaves the stretch (the same in every thread of a channel)
     float S = carry, full = carry;
-    for (int v = 0; v < AF_GS_WARPS; ++v) {
+#pragma unroll 8
+    for (int v = 0; v < RUNS; ++v) {
       if (v == w) S = full;
-      full = comp[v][lane][0] * full + comp[v][lane][1];
+      const float2 m = comp[v][lane];
+      full = m.x * full + m.y;
     }
     carry = full;
 #pragma unroll
-    for (int e = 0; e < AF_GS_RUN; ++e) {
+    for (int e = 0; e < RUN; ++e) {
       if (e < n) {
         S = (1.f - z[e]) * S + z[e] * cd[e];
         if (on) y[(size_t)(t0 + e) * width + c] = from_f32<TY>(S * (g[e] / (1.f + expf(-g[e]))));
@@ -853,11 +855,16 @@ gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long 
 
 AF_EXPORT int af_gated_scan(void* y, int y_dtype, const float* proj, long long ld, int off_z, int off_x, int off_g,
                             const float* bz, const float* bx, float* state, const int* seq_starts, const int* slots,
-                            int n_seqs, int width, cudaStream_t stream) {
+                            int n_seqs, int n_tokens, int width, cudaStream_t stream) {
   if (n_seqs == 0) return 0;
   AF_REQUIRE(n_seqs > 0 && n_seqs < 65536 && width > 0, "af_gated_scan: bad sizes");
-  AF_DISPATCH_DTYPE(y_dtype, TY, af_launch(gated_scan_kernel<TY>, dim3((width + 31) / 32, n_seqs), dim3(AF_GS_WARPS * 32), 0, stream,
-                                           (TY*)y, proj, ld, off_z, off_x, off_g, bz, bx, state, seq_starts, slots, width));
+  // (sequences of more tokens than the narrow shape takes at a time: the wide one)
+  const bool wide = n_tokens > 128ll * n_seqs;
+  const int ch = wide ? 16 : 32;
+  AF_DISPATCH_DTYPE(y_dtype, TY,
+                    auto kernel = wide ? gated_scan_kernel<TY, 16, 32, 8> : gated_scan_kernel<TY, 32, 8, 16>;
+                    af_launch(kernel, dim3((width + ch - 1) / ch, n_seqs), dim3(wide ? 512 : 256), 0, stream, (TY*)y, proj, ld,
+                              off_z, off_x, off_g, bz, bx, state, seq_starts, slots, width));
   AF_CHECK_LAUNCH("af_gated_scan");
 }
 

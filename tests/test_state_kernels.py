@@ -156,6 +156,33 @@ def test_gated_scan(width):
             at += n
 
 
+@pytest.mark.parametrize("width", [5, 16, 300])
+@pytest.mark.parametrize("lens", [[129], [257, 700, 1], [256], [512, 255]])
+def test_gated_scan_of_prompts(width, lens):
+    """Sequences of more than 128 tokens on average take the shape for prompts: stretches of 256 tokens that end inside a run, at
+    its border and at the stretch's; bounds as for short ones (a state is a mean of what entered it: its error does not grow)."""
+    from airframe_b200 import kernels
+    T = sum(lens)
+    g = torch.Generator().manual_seed(width)
+    proj = torch.randn(T, 3 * width, generator=g) * 2
+    bz, bx = torch.randn(width, generator=g), torch.randn(width, generator=g)
+    state = torch.zeros(4, width, device=DEV)
+    state[1:] = torch.randn(3, width, generator=g).to(DEV)
+    before, slots = state.clone().cpu().double(), [3, 0, 2][:len(lens)]
+    y = torch.empty(T, width, device=DEV)
+    kernels.gated_scan(y, proj.to(DEV), 0, width, 2 * width, bz.to(DEV), bx.to(DEV), state, batch_of(lens, slots))
+    for (s, n), slot in zip(in_order(lens), slots):
+        p = proj[s].double()
+        z, c = plain.sigmoid(p[:, :width] + bz.double()), p[:, width:2 * width] + bx.double()
+        cand, S, out = torch.where(c >= 0, c + 0.5, plain.sigmoid(c)), before[slot], []
+        for t in range(n):
+            S = (1 - z[t]) * S + z[t] * cand[t]
+            out.append(S)
+        close(y[s], torch.stack(out) * plain.silu(p[:, 2 * width:]), 2e-6)
+        close(state[slot], S, 2e-6)
+    assert torch.equal(state[1].cpu().double(), before[1])
+
+
 @pytest.mark.parametrize("n,group", [(48, 24), (60, 60), (256, 128), (24, 8)])
 def test_gated_group_norm(n, group):
     from airframe_b200 import kernels
