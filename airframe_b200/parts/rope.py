@@ -116,7 +116,7 @@ class Rope(PositionEncoding):
                               "(kernels.qk_norm_rope_store), which this path is not")
 
     def rotary_table(self, batch, hd):
-        key = ("rope_table", self.theta, self.rotary_dim, self.inv_freq.data_ptr())
+        key = ("rope_table", self._table_key)       # (by the frequencies' values: one table a step, not one a layer)
         if key not in batch.aux:
             batch.aux[key] = kernels.rope_table(batch.positions, self.inv_freq)
         return batch.aux[key]
