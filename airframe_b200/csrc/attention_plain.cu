@@ -378,11 +378,12 @@ __device__ __forceinline__ void attn_keys(WarpAttn<NS>& st, const T* const (&k)[
     s[n] = softcap_f32(s[n] * scale, cap) + bias[n];
     m_new = fmaxf(m_new, s[n]);
   }
-  const float corr = expf(st.m - m_new);  // exp(-inf) = 0 on the first key
+  const float ref = m_new == -INFINITY ? 0.f : m_new;      // (no score above -inf yet: they weigh nothing)
+  const float corr = expf(st.m - ref);    // exp(-inf) = 0 on the first key
   st.l *= corr;
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    s[n] = expf(s[n] - m_new);
+    s[n] = expf(s[n] - ref);
     st.l += s[n];
   }
 #pragma unroll
@@ -418,11 +419,15 @@ __device__ __forceinline__ float gate_factor(const float* gate, long long gate_s
 }
 
 // Prompts that start at position 0: keys and values are the step's own rows.
-// Warp w of the grid handles (token, head) = (w / nq, w % nq).  `hd` is the key size, `dv` the value
+// Block w of the grid handles (token, head) = (w / nq, w % nq): one warp, or from AF_PLAIN_SPLIT visible keys on four, a quarter
+// of the keys each, joined through shared memory (a token's number of keys alone decides).  A warp's chain from keys to keys
+// is what takes the time: the last tokens' walk was as long as the kernel while most warps were done.  301 tokens, 8 heads of
+// 256 in 32 bits: 105 -> @@ us.  `hd` is the key size, `dv` the value
 // size; the first `keep` positions stay visible whatever the window; `sinks` (float [nq]) and `gate` (float logits, row t and column h at gate[t * gate_stride + h]:
 // the head's output is multiplied by their sigmoid) may be null.
+#define AF_PLAIN_SPLIT 64
 template <typename T, int NS>
-__global__ void attn_prefill_plain_kernel(T* __restrict__ out, int out_stride, const T* __restrict__ q,
+__global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__ out, int out_stride, const T* __restrict__ q,
                                           int q_stride, const T* __restrict__ k, int k_stride,
                                           const T* __restrict__ v, int v_stride,
                                           const int* __restrict__ positions,
@@ -432,23 +437,24 @@ __global__ void attn_prefill_plain_kernel(T* __restrict__ out, int out_stride, c
                                           long long gate_stride) {
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= (long long)n_tokens * nq) return;
-  const int t = (int)(w / nq), h = (int)(w % nq);
+  const int lane = threadIdx.x & 31, split = threadIdx.x >> 5;
+  const int t = n_tokens - 1 - (int)(blockIdx.x / nq), h = (int)(blockIdx.x % nq);      // (the last tokens, which see most, first)
   const int g = h / (nq / nkv);
   const int pos = positions[t];          // position inside its sequence
   const int first_row = t - pos;         // row of the sequence's position 0
   using Attn = WarpAttn<NS>;
   constexpr int KEYS = Attn::KEYS;
   Attn st;
-  attn_load_q(st, q + (size_t)t * q_stride + (size_t)h * hd, hd, lane, sinks ? sinks[h] : -INFINITY);
+  attn_load_q(st, q + (size_t)t * q_stride + (size_t)h * hd, hd, lane, sinks && split == 0 ? sinks[h] : -INFINITY);
   const int lo = first_visible(pos, window, mask_kind);
   const float slope = slopes ? slopes[h] : 0.f;
   const int kept = min(keep, lo);         // the first tokens that stay visible before the window
   const int n_vis = kept + pos - lo + 1;
-  int x = 0;
-  for (; KEYS > 1 && x + KEYS <= n_vis; x += KEYS) {
+  const int splits = n_vis >= AF_PLAIN_SPLIT ? 4 : 1;
+  if (split >= splits) return;
+  const int per = ((n_vis + splits - 1) / splits + 3) / 4 * 4, end = min(n_vis, (split + 1) * per);
+  int x = split * per;
+  for (; KEYS > 1 && x + KEYS <= end; x += KEYS) {
     const T *ks[KEYS], *vs[KEYS];
     float bias[KEYS];
 #pragma unroll
@@ -460,11 +466,34 @@ __global__ void attn_prefill_plain_kernel(T* __restrict__ out, int out_stride, c
     }
     attn_keys<KEYS>(st, ks, vs, hd, dv, lane, scale, cap, bias);
   }
-  for (; x < n_vis; ++x) {
+  for (; x < end; ++x) {
     const int j = x < kept ? x : lo + x - kept;
     const size_t r = (size_t)(first_row + j);
     attn_key(st, k + r * k_stride + (size_t)g * hd, v + r * v_stride + (size_t)g * dv, hd, dv, lane, scale,
              cap, slope * (float)(j - pos));
+  }
+  if (splits > 1) {
+    __shared__ float o_s[3][32 * NS], m_s[4], l_s[4];
+    if (split > 0) {
+#pragma unroll
+      for (int e = 0; e < NS; ++e) o_s[split - 1][lane + 32 * e] = st.o[e];
+    }
+    if (lane == 0) m_s[split] = st.m, l_s[split] = st.l;
+    __syncthreads();
+    if (split > 0) return;
+    float top = fmaxf(fmaxf(m_s[0], m_s[1]), fmaxf(m_s[2], m_s[3]));
+    if (top == -INFINITY) top = 0.f;
+    const float f0 = expf(st.m - top);
+    st.l *= f0;
+#pragma unroll
+    for (int e = 0; e < NS; ++e) st.o[e] *= f0;
+#pragma unroll 1
+    for (int s = 1; s < 4; ++s) {
+      const float f = expf(m_s[s] - top);
+      st.l += l_s[s] * f;
+#pragma unroll
+      for (int e = 0; e < NS; ++e) st.o[e] += o_s[s - 1][lane + 32 * e] * f;
+    }
   }
   attn_store(st, out + (size_t)t * out_stride + (size_t)h * dv, dv, lane, gate_factor(gate, gate_stride, t, h));
 }
@@ -481,14 +510,13 @@ AF_EXPORT int af_attn_prefill_plain(void* out, int out_stride, const void* q, in
              "af_attn_prefill_plain: key size %d or value size %d beyond %d", hd, dv, AF_MAX_HD);
   AF_REQUIRE(mask_kind == AF_MASK_WINDOW || mask_kind == AF_MASK_CHUNK, "af_attn_prefill_plain: mask kind %d", mask_kind);
   AF_REQUIRE(keep >= 0, "af_attn_prefill_plain: %d kept tokens", keep);
-  const long long warps = (long long)n_tokens * nq;
-  const int wpb = 4, slices = (max(hd, dv) + 31) / 32;
-  const long long blocks = (warps + wpb - 1) / wpb;
+  const long long blocks = (long long)n_tokens * nq;
+  const int slices = (max(hd, dv) + 31) / 32;
   AF_REQUIRE(blocks < (1ll << 31), "af_attn_prefill_plain: too many rows");
   AF_DISPATCH_DTYPE(dtype, T,
                     auto kernel = slices <= 4 ? attn_prefill_plain_kernel<T, 4> : slices <= 8 ? attn_prefill_plain_kernel<T, 8>
                                                                            : attn_prefill_plain_kernel<T, AF_HD_SLICES>;
-                    af_launch(kernel, dim3((unsigned)blocks), dim3(wpb * 32), 0, stream, 
+                    af_launch(kernel, dim3((unsigned)blocks), dim3(128), 0, stream, 
                         (T*)out, out_stride, (const T*)q, q_stride, (const T*)k, k_stride, (const T*)v,
                         v_stride, positions, n_tokens, nq, nkv, hd, dv, scale, cap, window, mask_kind, keep, slopes,
                         sinks, gate, gate_stride));

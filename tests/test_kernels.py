@@ -411,6 +411,38 @@ def test_ring_keeps_the_last_rows_of_a_long_prompt(K):
         page = [3, 1][r // PAGE]
         assert torch.equal(vc[page, 0, r % PAGE].cpu(), v[p]), p
 
+@pytest.mark.parametrize("hd, dv", [(64, 64), (200, 136), (256, 256), (300, 520)])
+def test_attention_prefill_plain_in_quarters(K, hd, dv):
+    """Around the number of keys from which four warps share a query (64), remainders of four, heads of every register shape;
+    windows that keep first tokens, a sink, scores of minus infinity.  Bound: sums of up to 200 32-bit terms."""
+    torch.manual_seed(hd)
+    nq, nkv, lens, window, keep = 4, 2, [63, 64, 65, 67, 200], 70, 5
+    T = sum(lens)
+    q, k, v = torch.randn(T, nq * hd), torch.randn(T, nkv * hd), torch.randn(T, nkv * dv)
+    sinks, slopes = torch.randn(nq), torch.rand(nq)
+    k.view(T, nkv, hd)[T - 190:T - 150, 1, 0] = -1e30          # (of the last sequence; its early tokens' quarters see them)
+    q.view(T, nq, hd)[:, 2, 0] = 1e30
+    pos = torch.tensor([i for n in lens for i in range(n)], dtype=torch.int32)
+    for win, kept in ((0, 0), (window, keep)):
+        out = torch.full((T, nq * dv), float("nan"), device=DEV)
+        K.attn_prefill_plain(out, q.to(DEV), k.to(DEV), v.to(DEV), pos.to(DEV), nq, nkv, hd, hd ** -0.5, 0.0, win, slopes.to(DEV),
+                             dv=dv, sinks=sinks.to(DEV), keep=kept)
+        at = 0
+        for n in lens:
+            s = slice(at, at + n)
+            i, j = torch.arange(n)[:, None], torch.arange(n)[None, :]
+            seen = (j <= i) & ((i - j < win) | (j < kept) if win else True)
+            for h in (0, 1, 3):                     # (head 2's products leave 32 bits: below)
+                qq, kk, vv = (t[s].double().view(n, -1, d)[:, g] for t, g, d in ((q, h, hd), (k, h // 2, hd), (v, h // 2, dv)))
+                sc = (qq @ kk.T) * hd ** -0.5 + slopes[h].double() * (j - i)
+                sc = torch.cat([sc.masked_fill(~seen, -math.inf), sinks[h].double().expand(n, 1)], 1).softmax(1)[:, :n]
+                close(out[s].view(n, nq, dv)[:, h], sc @ vv, torch.float32)
+            at += n
+        # keys whose score is minus infinity weigh nothing
+        h2 = out[-200:].view(200, nq, dv)[:, 2]
+        assert bool(h2[10:].isfinite().all())
+
+
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hd,nq,nkv,window,cap", [(16, 4, 2, 0, 50.0), (80, 6, 2, 7, 0.0), (256, 3, 3, 33, 30.0),
