@@ -422,7 +422,7 @@ __device__ __forceinline__ float gate_factor(const float* gate, long long gate_s
 // Block w of the grid handles (token, head) = (w / nq, w % nq): one warp, or from AF_PLAIN_SPLIT visible keys on four, a quarter
 // of the keys each, joined through shared memory (a token's number of keys alone decides).  A warp's chain from keys to keys
 // is what takes the time: the last tokens' walk was as long as the kernel while most warps were done.  301 tokens, 8 heads of
-// 256 in 32 bits: 105 -> @@ us.  `hd` is the key size, `dv` the value
+// 256 in 32 bits: 105 -> 67 us.  `hd` is the key size, `dv` the value
 // size; the first `keep` positions stay visible whatever the window; `sinks` (float [nq]) and `gate` (float logits, row t and column h at gate[t * gate_stride + h]:
 // the head's output is multiplied by their sigmoid) may be null.
 #define AF_PLAIN_SPLIT 64
