@@ -2,7 +2,8 @@
 // 32-bit multiply-adds and 32-bit accumulators (no tensor cores, no reduced
 // precision mode).  Every output element adds its K products in index order,
 // whatever M and N are, so a row's result does not depend on the batch it is
-// in.  It is the matrix product of the 32-bit path and the twin of the
+// in.  It is the 32-bit path's matrix product of few rows, of small and of
+// unaligned sizes (gemm_f32_tc.cu takes the prompts') and the twin of the
 // tensor-core kernels.
 //
 // float operands run the two gemm_f32 kernels (the reads from shared memory bound them for many rows, an output's chain
