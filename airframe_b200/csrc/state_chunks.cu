@@ -91,22 +91,27 @@ __device__ __forceinline__ float sc_sum32(float* v) {
   return v[0];
 }
 
-// out[r0 + i][column] = sum over k <= r0 + 3 of m[k][r0 + i] x[k][column] for four rows i and up to eight columns of a lane
-// (four from `col`, four from col + 64 where `second`): m lower triangular, transposed, rows of SC_PM.
+// out[r0 + i][column] = sum over k <= r0 + i of m[k][r0 + i] x[k][column] for four rows i and up to eight columns of a lane
+// (four from `col`, four from col + 64 where `second`): m lower triangular, transposed, rows of SC_PM.  No row meets a later
+// token's values: zero times an infinity would be NaN.
 __device__ __forceinline__ void sc_lower_rows(const float* m, int r0, const float* x, int ldx, bool second, float (&out)[4][8]) {
   unsigned long long acc[4][4] = {};
-#pragma unroll 2
-  for (int k = 0; k < r0 + 4; ++k) {
+  auto step = [&](int k, int from) {               // rows from .. 3 of the four take token k's values
     const float4 f = *reinterpret_cast<const float4*>(m + k * SC_PM + r0);
     const unsigned long long fd[4] = {sc_both(f.x), sc_both(f.y), sc_both(f.z), sc_both(f.w)};
     const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(x + k * ldx);
     const ulonglong2 hi = second ? *reinterpret_cast<const ulonglong2*>(x + k * ldx + 64) : make_ulonglong2(0, 0);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+      if (i < from) continue;
       sc_fma2(acc[i][0], fd[i], lo.x), sc_fma2(acc[i][1], fd[i], lo.y);
       sc_fma2(acc[i][2], fd[i], hi.x), sc_fma2(acc[i][3], fd[i], hi.y);
     }
-  }
+  };
+#pragma unroll 2
+  for (int k = 0; k < r0; ++k) step(k, 0);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) step(r0 + i, i);
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll

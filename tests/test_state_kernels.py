@@ -362,3 +362,51 @@ def test_decay_attention_in_chunks(heads, dk, dv, silu):
     for rows in (slice(last.start, last.start + 77), slice(last.start + 77, last.stop)):
         run(rows, [rows.stop - rows.start], [6])
     close(out[last], whole.cpu())
+
+
+@pytest.mark.parametrize("what", ["r", "k", "v", "a", "w1"])
+@pytest.mark.parametrize("mode", ["delta", "decay"])
+def test_chunks_of_values_that_are_not_finite(mode, what):
+    """An infinity or a NaN at a token leaves the tokens before it as they are, bit for bit, and reaches the tokens behind it as
+    token by token it does: at places within a group of four rows, of 16 tokens and of a chunk of 32."""
+    from airframe_b200 import kernels
+    if mode == "decay" and what in ("a", "w1"):
+        return
+    heads, dk, dv, rank, lens, slots = 2, 32, 32, 8, [70, 40], [1, 0]
+    T, n = sum(lens), heads * dk
+    g = torch.Generator().manual_seed(3)
+    data = {name: torch.randn(T, w, generator=g) for name, w in (("r", n), ("k", n), ("v", heads * dv), ("a", n), ("w1", rank))}
+    a_bias, w0 = torch.randn(n, generator=g).to(DEV), torch.randn(n, generator=g).to(DEV)
+    w2t = torch.randn(rank, n, generator=g).to(DEV)
+    decay = torch.tensor([0.9, 1.0], device=DEV)
+
+    def run(chunked):
+        d = {name: t.to(DEV) for name, t in data.items()}
+        state, out = torch.zeros(2, heads, dv, dk, device=DEV), torch.empty(T, heads * dv, device=DEV)
+        args = (mode, out, d["r"], d["k"], d["v"], state)
+        if chunked:
+            more = (dict(a=d["a"], low=d["w1"], a_bias=a_bias, w0=w0, w2t=w2t, decay_scale=0.5, key_eps=1e-6) if mode == "delta"
+                    else dict(decay=decay))
+            kernels.state_chunks(*args, prompt_batch(lens, slots), heads, dk, dv, **more)
+        elif mode == "decay":
+            kernels.state_scan(*args, batch_of(lens, slots), heads, dk, dv, decay=decay)
+        else:
+            proj = torch.cat([d["k"], d["a"], d["w1"]], 1)
+            pre = torch.empty(T, 3, n, device=DEV)
+            kernels.delta_prep(pre, proj, 0, n, 2 * n, a_bias, w0, w2t, heads, dk, 0.5, 1e-6)
+            kernels.state_scan(*args, batch_of(lens, slots), heads, dk, dv, w=pre[:, 0], u=pre[:, 1], au=pre[:, 2])
+        return out
+
+    clean = run(True)
+    assert bool(clean.isfinite().all())
+    for t in (0, 2, 3, 17, 30, 35, 69):
+        for bad in (math.inf, -math.inf, math.nan):
+            if what in ("a", "w1") and bad == bad:
+                continue                               # (a sigmoid or tanh of an infinity is finite)
+            kept = data[what][t, 5].item()
+            data[what][t, 5] = bad
+            got, twin = run(True), run(False)
+            data[what][t, 5] = kept
+            assert torch.equal(got[:t], clean[:t]) and torch.equal(got[lens[0]:], clean[lens[0]:]), (t, bad)
+            assert torch.equal(got.isfinite(), twin.isfinite()), (t, bad)
+            assert not bool(got[t].isfinite().all())
