@@ -670,7 +670,15 @@ state_walk_kernel(StateChunkArgs a) {
   const int j0 = blockIdx.x * SC_N;
   const int base = a.seq_first_chunk[0], ch0 = a.seq_first_chunk[b] - base, ch1 = a.seq_first_chunk[b + 1] - base;
   const int slot = a.slots[b];
-  if (slot < 0 || ch0 >= ch1) return;
+  if (ch0 >= ch1) return;
+  if (slot < 0) {                                  // (a padding row: zeros, and no state)
+    pdl_wait();
+    const int first = a.chunk_starts[ch0], count = (a.chunk_starts[ch1] - first) * (SC_N / 4);
+    for (int i = tid; i < count; i += 256)
+      *reinterpret_cast<float4*>(a.out + (size_t)(first + i / (SC_N / 4)) * a.out_ts + (size_t)h * dv + j0 + i % (SC_N / 4) * 4) =
+          make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
+  }
   if (tid == 0) {
     mbar_init(&full[0], 1);
     mbar_init(&full[1], 1);

@@ -410,3 +410,24 @@ def test_chunks_of_values_that_are_not_finite(mode, what):
             assert torch.equal(got[:t], clean[:t]) and torch.equal(got[lens[0]:], clean[lens[0]:]), (t, bad)
             assert torch.equal(got.isfinite(), twin.isfinite()), (t, bad)
             assert not bool(got[t].isfinite().all())
+
+
+@pytest.mark.parametrize("mode", ["delta", "decay"])
+def test_chunks_of_padding_rows(mode):
+    """A sequence without a slot leaves zeros and no state, as token by token."""
+    from airframe_b200 import kernels
+    heads, dk, dv, rank, lens, slots = 2, 32, 48, 8, [40, 33, 5], [1, -1, 0]
+    T, n = sum(lens), heads * dk
+    g = torch.Generator().manual_seed(5)
+    r, k, v, a, low = (torch.randn(T, w, generator=g).to(DEV) for w in (n, n, heads * dv, n, rank))
+    more = (dict(a=a, low=low, a_bias=r[0], w0=k[0], w2t=torch.randn(rank, n, generator=g).to(DEV), decay_scale=0.5, key_eps=1e-6)
+            if mode == "delta" else dict(decay=torch.tensor([0.9, 1.0], device=DEV)))
+    outs, states = [], []
+    for where in (slots, [1, 2, 0]):
+        state, out = torch.zeros(3, heads, dv, dk, device=DEV), torch.full((T, heads * dv), float("nan"), device=DEV)
+        kernels.state_chunks(mode, out, r, k, v, state, prompt_batch(lens, where), heads, dk, dv, **more)
+        outs.append(out), states.append(state)
+    assert bool((outs[0][40:73] == 0).all()) and float(states[0][2].abs().sum()) == 0
+    for rows in (slice(0, 40), slice(73, T)):
+        assert torch.equal(outs[0][rows], outs[1][rows])
+    assert torch.equal(states[0][:2], states[1][:2])
