@@ -2014,22 +2014,22 @@ def delta_prompt_supported(dk: int, dv: int) -> bool:
     return bool(_lib().af_delta_prompt_supported(c_int(dk), c_int(dv)))
 
 
-def _delta_chunks(batch):
-    """The chunks of a prefill step's sequences (made on the host once a step, kept in ``batch.aux``): device tensors
-    chunk_starts [n_chunks + 1] and seq_first_chunk [n_seqs + 1], and how many chunks there are."""
-    if "delta_chunks" not in batch.aux:
-        chunk = int(_lib().af_delta_prompt_chunk())
+def _chunk_table(batch, size: int):
+    """The chunks of ``size`` tokens of a prefill step's sequences (made on the host once a step, kept in ``batch.aux`` by their
+    size): device tensors chunk_starts [n_chunks + 1] and seq_first_chunk [n_seqs + 1], and how many chunks there are."""
+    key = ("chunk_table", size)
+    if key not in batch.aux:
         starts, first, row = [], [0], 0
         for n in batch.seq_lens:
-            starts.extend(range(row, row + n, chunk))
+            starts.extend(range(row, row + n, size))
             row += n
             first.append(len(starts))
         starts.append(row)
         host = torch.tensor(starts + first, dtype=torch.int32).pin_memory()
         dev = host.to(batch.tokens.device, non_blocking=True)
         transfers.count_h2d(host)
-        batch.aux["delta_chunks"] = (dev[:len(starts)], dev[len(starts):], len(starts) - 1)
-    return batch.aux["delta_chunks"]
+        batch.aux[key] = (dev[:len(starts)], dev[len(starts):], len(starts) - 1)
+    return batch.aux[key]
 
 
 STATE_CHUNKS_AT_ONCE = 512     # chunks of 32 tokens whose scratch (up to 138 KB a head) is held at a time
@@ -2068,9 +2068,9 @@ def state_chunks(mode: str, out, r, k, v, state, batch, heads: int, dk: int, dv:
             raise KernelError("state_chunks: one decay per head")
         none = ctypes.c_void_p(0)
         extra = (*null, *null, none, none, none, c_int(0), c_float(0.0), c_float(0.0), _ptr(decay, "decay", f32))
-    starts, first, _ = _delta_chunks(batch)
     lib = _lib()
     size = int(lib.af_state_chunks_size())
+    starts, first, _ = _chunk_table(batch, size)
     lib.af_state_chunks_scratch.restype = c_longlong
     # the step's sequences in runs whose scratch fits what is held at a time (one launch pair a run; nearly always one run)
     runs, chunk = [], 0
@@ -2108,7 +2108,7 @@ def delta_prompt(out, q, k, v, beta, z, dt_bias, rate, state, batch, heads: int,
             or tuple(state.shape[1:]) != (heads, dv, dk) or not state.is_contiguous() or dt_bias.numel() != heads * dk \
             or rate.numel() != heads * dk:
         raise KernelError(f"delta_prompt: out contiguous float32 [{T}, {heads * dv}], state float32 [slots, {heads}, {dv}, {dk}]")
-    starts, first, n = _delta_chunks(batch)
+    starts, first, n = _chunk_table(batch, int(_lib().af_delta_prompt_chunk()))
     dev, f32, i32 = out.device, torch.float32, torch.int32
     # blocks of 32 value columns, or of 16 while those all run at once (a block an SM)
     tile = tile or (16 if batch.n_seqs * heads * -(-dv // 16) <= sm_count() else 32)

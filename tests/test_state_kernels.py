@@ -431,3 +431,23 @@ def test_chunks_of_padding_rows(mode):
     for rows in (slice(0, 40), slice(73, T)):
         assert torch.equal(outs[0][rows], outs[1][rows])
     assert torch.equal(states[0][:2], states[1][:2])
+
+
+def test_chunk_tables_of_other_sizes_in_a_step():
+    """A step's tables of chunks go by their size: what another kernel cut into chunks of 64 tokens is not taken for its own."""
+    from airframe_b200 import kernels
+    heads, dk, dv, lens = 2, 16, 16, [70, 33]
+    T, n = sum(lens), heads * dk
+    g = torch.Generator().manual_seed(6)
+    r, k, v = (torch.randn(T, w, generator=g).to(DEV) for w in (n, n, heads * dv))
+    decay, outs = torch.tensor([0.9, 1.0], device=DEV), []
+    for other in (None, 64, 16):
+        batch = prompt_batch(lens, [1, 0])
+        if other is not None:
+            starts, first, count = kernels._chunk_table(batch, other)
+            assert count == sum(-(-x // other) for x in lens)
+            assert starts.tolist() == [*range(0, 70, other), *range(70, 103, other), 103] and first.tolist() == [0, -(-70 // other), count]
+        state, out = torch.zeros(2, heads, dv, dk, device=DEV), torch.empty(T, heads * dv, device=DEV)
+        kernels.state_chunks("decay", out, r, k, v, state, batch, heads, dk, dv, decay=decay)
+        outs.append((out, state))
+    assert all(torch.equal(o, outs[0][0]) and torch.equal(s, outs[0][1]) for o, s in outs)
