@@ -46,6 +46,7 @@ struct StateChunkArgs {
   float* out;                   // [tokens][H * dv], rows out_ts apart
   long long out_ts;
   const int *chunk_starts, *seq_first_chunk, *slots;   // of this launch's first chunk and sequence on
+  int chunk0, n_chunks;         // this launch's chunks of the step (a sequence may begin before them and go on behind them)
   int H, dk, dv;
   int* err;
 };
@@ -668,7 +669,7 @@ state_walk_kernel(StateChunkArgs a) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y, b = blockIdx.z, tiles = gridDim.x;
   const int j0 = blockIdx.x * SC_N;
-  const int base = a.seq_first_chunk[0], ch0 = a.seq_first_chunk[b] - base, ch1 = a.seq_first_chunk[b + 1] - base;
+  const int ch0 = max(a.seq_first_chunk[b] - a.chunk0, 0), ch1 = min(a.seq_first_chunk[b + 1] - a.chunk0, a.n_chunks);
   const int slot = a.slots[b];
   if (ch0 >= ch1) return;
   if (slot < 0) {                                  // (a padding row: zeros, and no state)
@@ -821,24 +822,25 @@ AF_EXPORT long long af_state_chunks_scratch(int delta, int dk, int dv, int which
   return which == 0 ? sc_blob(delta != 0, dk) : (long long)(dv / SC_N) * sc_tile(delta != 0);
 }
 
-// A prefill step's recurrence over n_chunks chunks of n_seqs whole sequences.  chunk_starts, seq_first_chunk and slots begin
-// at the first of them (seq_first_chunk counts from the step's first chunk).  `delta`: the generalized delta rule from r, k, v,
+// A prefill step's recurrence over the n_chunks chunks from chunk0 on, which lie in n_seqs sequences; chunk_starts, slots and
+// seq_first_chunk begin at the first of them (seq_first_chunk counts from the step's first chunk).  A sequence may be cut by
+// the range: the next launch goes on from the state that this one leaves.  `delta`: the generalized delta rule from r, k, v,
 // the removals' logits a, the low-rank rows `low` [rank] and their weights; else linear attention with a decay per head.
 AF_EXPORT int af_state_chunks(int delta, float* out, long long out_ts, const float* r, long long r_ts, const float* k,
                               long long k_ts, const float* v, long long v_ts, const float* la, long long la_ts,
                               const float* low, long long low_ts, const float* a_bias, const float* w0, const float* w2t,
                               int rank, float decay_scale, float key_eps, const float* decay, int silu, float* state,
                               float* blob, float* tiles, const int* chunk_starts, const int* seq_first_chunk, const int* slots,
-                              int n_chunks, int n_seqs, int H, int dk, int dv, int* err, cudaStream_t stream) {
+                              int chunk0, int n_chunks, int n_seqs, int H, int dk, int dv, int* err, cudaStream_t stream) {
   if (n_chunks == 0) return 0;
   AF_REQUIRE(af_state_chunks_supported(dk, dv, delta ? rank : 1), "af_state_chunks: heads of %d keys and %d values, rank %d", dk, dv, rank);
-  AF_REQUIRE(n_chunks > 0 && n_seqs > 0 && n_seqs < 65536 && H > 0 && H < 65536 && (!delta || rank > 0), "af_state_chunks: bad sizes");
+  AF_REQUIRE(chunk0 >= 0 && n_chunks > 0 && n_seqs > 0 && n_seqs < 65536 && H > 0 && H < 65536 && (!delta || rank > 0), "af_state_chunks: bad sizes");
   AF_REQUIRE(((r_ts | k_ts | v_ts | la_ts | out_ts) & 3) == 0 &&
                  (((uintptr_t)r | (uintptr_t)k | (uintptr_t)v | (uintptr_t)la | (uintptr_t)blob | (uintptr_t)tiles | (uintptr_t)out |
                    (uintptr_t)state | (uintptr_t)w2t) & 15) == 0,
              "af_state_chunks: rows of whole 16-byte pieces");
   StateChunkArgs a{r, k, v, r_ts, k_ts, v_ts, la, low, la_ts, low_ts, a_bias, w0, w2t, rank, decay_scale, key_eps, decay, silu,
-                   blob, tiles, state, out, out_ts, chunk_starts, seq_first_chunk, slots, H, dk, dv, err};
+                   blob, tiles, state, out, out_ts, chunk_starts, seq_first_chunk, slots, chunk0, n_chunks, H, dk, dv, err};
   static bool raised[5][AF_MAX_DEVICES];
   const dim3 chunks(n_chunks, H), walk(dv / SC_N, H, n_seqs);
   int e;

@@ -2032,7 +2032,27 @@ def _chunk_table(batch, size: int):
     return batch.aux[key]
 
 
-STATE_CHUNKS_AT_ONCE = 512     # chunks of 32 tokens whose scratch (up to 138 KB a head) is held at a time
+# Chunks of 32 tokens whose scratch is held at a time: at most so many, and of at most so many bytes (a chunk of 18 heads of 128 keys
+# and values takes 2.1 MB for the delta rule, 1.2 MB for linear attention: 127 and 220 chunks).
+STATE_CHUNKS_AT_ONCE = 512
+STATE_CHUNKS_BYTES = 256 << 20
+
+
+def _chunk_runs(seq_lens, size: int, most: int) -> list:
+    """[first sequence, sequences, first chunk, chunks] of the launches that hold at most ``most`` chunks of ``size`` tokens each:
+    sequences that fit stay whole, longer ones are cut and go on in the next."""
+    runs, chunk = [], 0
+    for s, length in enumerate(seq_lens):
+        left = -(-length // size)
+        while left:
+            if not runs or runs[-1][3] + min(left, most) > most:
+                runs.append([s, 0, chunk, 0])
+            c = min(left, most)
+            runs[-1][1] += 1
+            runs[-1][3] += c
+            chunk += c
+            left -= c
+    return runs
 
 
 def state_chunks_supported(dk: int, dv: int, rank: int = 1) -> bool:
@@ -2072,25 +2092,17 @@ def state_chunks(mode: str, out, r, k, v, state, batch, heads: int, dk: int, dv:
     size = int(lib.af_state_chunks_size())
     starts, first, _ = _chunk_table(batch, size)
     lib.af_state_chunks_scratch.restype = c_longlong
-    # the step's sequences in runs whose scratch fits what is held at a time (one launch pair a run; nearly always one run)
-    runs, chunk = [], 0
-    for s, length in enumerate(batch.seq_lens):
-        c = -(-length // size)
-        if runs and runs[-1][3] + c <= STATE_CHUNKS_AT_ONCE:
-            runs[-1][1] += 1
-            runs[-1][3] += c
-        else:
-            runs.append([s, 1, chunk, c])
-        chunk += c
-    most = max(run[3] for run in runs) * heads
-    blob, tiles = (torch.empty(most * lib.af_state_chunks_scratch(c_int(int(delta)), c_int(dk), c_int(dv), c_int(w)), dtype=f32,
-                               device=out.device) for w in (0, 1))
+    # the step's chunks in runs whose scratch fits what is held at a time (one launch pair a run; nearly always one run)
+    floats = [lib.af_state_chunks_scratch(c_int(int(delta)), c_int(dk), c_int(dv), c_int(w)) * heads for w in (0, 1)]
+    runs = _chunk_runs(batch.seq_lens, size, max(1, min(STATE_CHUNKS_AT_ONCE, STATE_CHUNKS_BYTES // (4 * sum(floats)))))
+    most = max(run[3] for run in runs)
+    blob, tiles = (torch.empty(most * n, dtype=f32, device=out.device) for n in floats)
     rp, kp, vp, op = (_f32_rows(t, name) for t, name in ((r, "r"), (k, "k"), (v, "v"), (out, "out")))
     for s0, seqs, c0, chunks in runs:
         _check(lib.af_state_chunks(c_int(int(delta)), *op, *rp, *kp, *vp, *extra, c_int(1 if silu else 0), _ptr(state), _ptr(blob),
                                    _ptr(tiles), _ptr(starts[c0:], "chunk_starts", i32), _ptr(first[s0:], "seq_first_chunk", i32),
-                                   _ptr(batch.slots[s0:], "slots", i32), c_int(chunks), c_int(seqs), c_int(heads), c_int(dk),
-                                   c_int(dv), _ptr(error_word(out.device), "err", i32), _stream()))
+                                   _ptr(batch.slots[s0:], "slots", i32), c_int(c0), c_int(chunks), c_int(seqs), c_int(heads),
+                                   c_int(dk), c_int(dv), _ptr(error_word(out.device), "err", i32), _stream()))
 
 
 def delta_prompt(out, q, k, v, beta, z, dt_bias, rate, state, batch, heads: int, dk: int, dv: int, tile: int = 0) -> None:

@@ -451,3 +451,38 @@ def test_chunk_tables_of_other_sizes_in_a_step():
         kernels.state_chunks("decay", out, r, k, v, state, batch, heads, dk, dv, decay=decay)
         outs.append((out, state))
     assert all(torch.equal(o, outs[0][0]) and torch.equal(s, outs[0][1]) for o, s in outs)
+
+
+@pytest.mark.parametrize("mode", ["delta", "decay"])
+def test_long_sequences_in_several_launches(mode, monkeypatch):
+    """Sequences of more chunks than are held at a time are cut and go on from the state in memory: the same bits as in one launch,
+    for outputs and states, and no more scratch than allowed."""
+    from airframe_b200 import kernels
+    heads, dk, dv, rank, lens, slots = 3, 64, 32, 16, [40, 32 * 9 + 5, 1, 7 * 32, 64], [3, 0, 4, 1, 2]
+    T, n = sum(lens), heads * dk
+    g = torch.Generator().manual_seed(8)
+    r, k, v, a, low = (torch.randn(T, w, generator=g).to(DEV) for w in (n, n, heads * dv, n, rank))
+    more = (dict(a=a, low=low, a_bias=r[0], w0=k[0], w2t=torch.randn(rank, n, generator=g).to(DEV), decay_scale=0.05, key_eps=1e-6)
+            if mode == "delta" else dict(decay=torch.tensor([0.9, 0.99, 1.0], device=DEV)))
+    start, got = torch.randn(5, heads, dv, dk, generator=g).to(DEV), []
+
+    def run():
+        state, out = start.clone(), torch.full((T, heads * dv), float("nan"), device=DEV)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        kernels.state_chunks(mode, out, r, k, v, state, prompt_batch(lens, slots), heads, dk, dv, **more)
+        return out, state, torch.cuda.max_memory_allocated() - before
+
+    whole = run()
+    chunk = whole[2] // sum(-(-x // 32) for x in lens)
+    for most in (1, 2, 3, 5, 8):
+        with monkeypatch.context() as m:
+            m.setattr(kernels, "STATE_CHUNKS_AT_ONCE", most)
+            got = run()
+        assert torch.equal(got[0], whole[0]) and torch.equal(got[1], whole[1]), most
+        with monkeypatch.context() as m:
+            m.setattr(kernels, "STATE_CHUNKS_BYTES", most * chunk)
+            got = run()
+        assert torch.equal(got[0], whole[0]) and torch.equal(got[1], whole[1]), most
+        assert got[2] <= most * chunk + 8192
