@@ -93,16 +93,29 @@ class _StateMixer(Mixer):
         return torch.cat(mats, dim=0).contiguous(), offsets
 
 
-# Tokens of the longest prompt of a bfloat16 step whose recurrence goes in chunks.  The whole call, token by token against
-# in chunks, us: delta rule, 18 heads of 128: one prompt of 64 56 / 67, of 128 91 / 75, of 2,048 1,191 / 391; 16 prompts of
-# 33 235 / 236, of 128 866 / 418; linear attention 30 / 42, 50 / 45, 628 / 260, 84 / 105, 249 / 180; with 16 heads of 64 the
-# lines cross between 64 and 128 tokens as well.  (32-bit mode goes token by token: it is the plain recurrence.)
+# When a bfloat16 step's recurrence goes in chunks (32-bit mode goes token by token: it is the plain recurrence): its longest
+# prompt has CHUNKS_FROM tokens, and its chunks are not mostly empty.  Token by token the longest sequence's chain and all
+# sequences' tokens take the time, in chunks every chunk does, however few tokens it holds.  The whole call, token by token against
+# in chunks, us (18 heads of 128; delta rule, linear attention): one prompt of 128 tokens 110 / 73, 58 / 36, of 2,048 1,223 / 417,
+# 694 / 275; 16 of 33 263 / 226, 86 / 97; 16 of 128 869 / 407, 248 / 171; 64 of 160 3,991 / 1,908, 1,187 / 761; one of 130 and 63 of
+# 40 1,135 / 841, 354 / 351; one of 130 and 63 of 17 572 / 521, 205 / 228; one of 128 and 60 of 8 329 / 464, 122 / 206; one of 128 and 255
+# single tokens 488 / 1,802, 291 / 786; one of 2,048 and 64 single tokens 1,529 / 820, 723 / 339.  With 16 heads of 64 the lines lie where
+# these do.
 CHUNKS_FROM = 128
+CHUNK_WORTH = 20        # tokens that a chunk's time is worth
+
+
+def chunks_pay(seq_lens) -> bool:
+    """Whether sequences of these lengths are faster in chunks of 32 tokens than token by token."""
+    longest = max(seq_lens)
+    if longest < CHUNKS_FROM:
+        return False
+    return CHUNK_WORTH * sum(-(-n // 32) for n in seq_lens) <= max(sum(seq_lens), 2 * longest)
 
 
 def _in_chunks(x, batch, dk: int, dv: int, rank: int = 1) -> bool:
-    return (x.dtype == torch.bfloat16 and batch.is_prefill and batch.max_len >= CHUNKS_FROM
-            and kernels.state_chunks_supported(dk, dv, rank))
+    return (x.dtype == torch.bfloat16 and batch.is_prefill and kernels.state_chunks_supported(dk, dv, rank)
+            and chunks_pay(batch.seq_lens))
 
 
 @register_part("mixer", "general_delta")

@@ -18,3 +18,13 @@ def test_runs_of_chunks():
             for s, c in enumerate(chunks):
                 met = sum(s0 <= s < s0 + seqs for s0, seqs, _, _ in runs)
                 assert met == -(-c // most)
+
+
+def test_which_steps_go_in_chunks():
+    """Steps whose recurrence is faster in chunks, and steps whose chunks would be mostly empty (measured: see the rule)."""
+    from airframe_b200.parts.recurrent import chunks_pay
+    for lens in ([128], [129], [2048], [128] * 16, [160] * 64, [129] * 8, [128, 40] * 8, [512] + [8] * 15, [2048] + [1] * 16, [2048] + [1] * 64,
+                 [130] + [40] * 63, [513] * 4):
+        assert chunks_pay(lens), lens
+    for lens in ([1], [127], [64] * 16, [33] * 16, [128] + [1] * 63, [128] + [1] * 255, [128] + [8] * 60, [130] + [17] * 63, [2048] + [1] * 400):
+        assert not chunks_pay(lens), lens
