@@ -2033,9 +2033,9 @@ def _chunk_table(batch, size: int):
 
 
 # Chunks of 32 tokens whose scratch is held at a time: at most so many, and of at most so many bytes (a chunk of 18 heads of 128 keys
-# and values takes 2.1 MB for the delta rule, 1.2 MB for linear attention: 127 and 220 chunks).
+# and values takes 2.1 MB for the delta rule, 1.2 MB for linear attention: 190 and 331 chunks).
 STATE_CHUNKS_AT_ONCE = 512
-STATE_CHUNKS_BYTES = 256 << 20
+STATE_CHUNKS_BYTES = 384 << 20
 
 
 def _chunk_runs(seq_lens, size: int, most: int) -> list:
