@@ -782,14 +782,17 @@ AF_EXPORT int af_gated_group_norm(void* y, int y_dtype, const float* o, const fl
 // token is affine, and so is their composition), the threads exchange these pairs, each composes the pairs
 // of the runs before its own onto the state carried so far, and then walks its tokens once more from the state
 // that really enters them.  The gates and candidates of a run stay in registers between the passes.
-// Two shapes: 32 channels by 8 runs of 16 for few tokens a sequence; for prompts 16 channels by 32 runs of 8, a block of
-// 512 threads: twice the blocks, twice the warps in each, half the chain.  One prompt of 2,048 tokens of 2,304 channels (66 MB:
-// 10 us): 124 -> 63 us.
+// Two shapes, chosen by a sequence's own length, so that its bits do not depend on what is beside it: up to AF_GS_LONG tokens
+// 32 channels by 8 runs of 16; longer ones 16 channels by 32 runs of 8, a block of 512 threads: twice the blocks, four times the
+// warps in each, half the chain.  A step that has both is two launches, each over the sequences of `from` to `to` tokens (both
+// shapes in one kernel have the registers of both: 8 prompts of 2,048 227 -> 352 us).  2,304 channels, us: one prompt of 2,048
+// tokens (66 MB: 10 us) 111 by 8 runs, 53 by 32; 16 of 129 51 / 59; 4 of 200 22 / 22; one of 300 27 / 17.
+#define AF_GS_LONG 192
 template <typename TY, int CH, int RUNS, int RUN>
 __global__ void __launch_bounds__(CH * RUNS)
 gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long ld, int off_z, int off_x, int off_g,
                   const float* __restrict__ bz, const float* __restrict__ bx, float* __restrict__ state,
-                  const int* __restrict__ seq_starts, const int* __restrict__ slots, int width) {
+                  const int* __restrict__ seq_starts, const int* __restrict__ slots, int width, int from, int to) {
   pdl_launch_dependents();
   __shared__ float2 comp[RUNS][CH];
   const int lane = threadIdx.x % CH, w = threadIdx.x / CH;
@@ -800,6 +803,7 @@ gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long 
   const int slot = slots[b];
   const float zb = on ? bz[c] : 0.f, xb = on ? bx[c] : 0.f;
   pdl_wait();
+  if (last - first < from || last - first > to) return;        // (of another launch)
   if (slot < 0) {
     if (on)
       for (int t = first + w; t < last; t += RUNS) y[(size_t)t * width + c] = from_f32<TY>(0.f);
@@ -853,19 +857,22 @@ gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long 
   if (on && w == 0) state[(size_t)slot * width + c] = carry;
 }
 
+// `min_len`, `max_len`: the step's shortest and longest sequence lie within these.
 AF_EXPORT int af_gated_scan(void* y, int y_dtype, const float* proj, long long ld, int off_z, int off_x, int off_g,
                             const float* bz, const float* bx, float* state, const int* seq_starts, const int* slots,
-                            int n_seqs, int n_tokens, int width, cudaStream_t stream) {
+                            int n_seqs, int min_len, int max_len, int width, cudaStream_t stream) {
   if (n_seqs == 0) return 0;
   AF_REQUIRE(n_seqs > 0 && n_seqs < 65536 && width > 0, "af_gated_scan: bad sizes");
-  // (sequences of more tokens than the narrow shape takes at a time: the wide one)
-  const bool wide = n_tokens > 128ll * n_seqs;
-  const int ch = wide ? 16 : 32;
-  AF_DISPATCH_DTYPE(y_dtype, TY,
-                    auto kernel = wide ? gated_scan_kernel<TY, 16, 32, 8> : gated_scan_kernel<TY, 32, 8, 16>;
-                    af_launch(kernel, dim3((width + ch - 1) / ch, n_seqs), dim3(wide ? 512 : 256), 0, stream, (TY*)y, proj, ld,
-                              off_z, off_x, off_g, bz, bx, state, seq_starts, slots, width));
-  AF_CHECK_LAUNCH("af_gated_scan");
+  for (int wide = max_len > AF_GS_LONG ? 1 : 0; wide >= (min_len > AF_GS_LONG ? 1 : 0); --wide) {
+    const int ch = wide ? 16 : 32;
+    AF_DISPATCH_DTYPE(y_dtype, TY,
+                      auto kernel = wide ? gated_scan_kernel<TY, 16, 32, 8> : gated_scan_kernel<TY, 32, 8, 16>;
+                      af_launch(kernel, dim3((width + ch - 1) / ch, n_seqs), dim3(wide ? 512 : 256), 0, stream, (TY*)y, proj, ld,
+                                off_z, off_x, off_g, bz, bx, state, seq_starts, slots, width, wide ? AF_GS_LONG + 1 : 0,
+                                wide ? 0x7fffffff : AF_GS_LONG));
+    AF_COUNT_LAUNCH("af_gated_scan");
+  }
+  return 0;
 }
 
 // ---------------------------------------------------------------- decays of gated linear attention

@@ -1054,11 +1054,12 @@ def gated_scan(y, proj, off_z: int, off_x: int, off_g: int, bz, bx, state, batch
     if max(off_z, off_x, off_g) + width > proj.shape[1] or bz.numel() != width or bx.numel() != width:
         raise KernelError("gated_scan: a section lies outside the projection row, or a bias of another size")
     pp, ld = _f32_rows(proj, "proj")
+    lens = getattr(batch, "seq_lens", None) or (0, T)        # (0 to T: any)
     _check(_lib().af_gated_scan(_ptr(y), c_int(dtype_code(y.dtype)), pp, ld, c_int(off_z), c_int(off_x), c_int(off_g),
                                 _ptr(bz, "bz", torch.float32), _ptr(bx, "bx", torch.float32),
                                 _ptr(state, "state", torch.float32), _ptr(batch.seq_starts, "seq_starts", torch.int32),
-                                _ptr(batch.slots, "slots", torch.int32), c_int(batch.n_seqs), c_int(y.shape[0]), c_int(width),
-                                _stream()))
+                                _ptr(batch.slots, "slots", torch.int32), c_int(batch.n_seqs), c_int(min(lens)),
+                                c_int(max(lens)), c_int(width), _stream()))
 
 
 def qk_norm_rope_store(qkv, proj, batch, nq: int, nkv: int, hd: int, inv_freq, rot_dim: int, pairing: str,

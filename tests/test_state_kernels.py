@@ -159,8 +159,8 @@ def test_gated_scan(width):
 @pytest.mark.parametrize("width", [5, 16, 300])
 @pytest.mark.parametrize("lens", [[129], [257, 700, 1], [256], [512, 255]])
 def test_gated_scan_of_prompts(width, lens):
-    """Sequences of more than 128 tokens on average take the shape for prompts: stretches of 256 tokens that end inside a run, at
-    its border and at the stretch's; bounds as for short ones (a state is a mean of what entered it: its error does not grow)."""
+    """Steps with prompts: stretches of 256 tokens (of sequences of more than 192) that end inside a run, at its border and at the
+    stretch's, shorter sequences beside them; bounds as for short ones (a state is a mean of what entered it: its error does not grow)."""
     from airframe_b200 import kernels
     T = sum(lens)
     g = torch.Generator().manual_seed(width)
@@ -486,3 +486,31 @@ def test_long_sequences_in_several_launches(mode, monkeypatch):
             got = run()
         assert torch.equal(got[0], whole[0]) and torch.equal(got[1], whole[1]), most
         assert got[2] <= most * chunk + 8192
+
+
+@pytest.mark.parametrize("width", [5, 40, 300])
+def test_gated_scan_alone_and_in_a_batch(width):
+    """A sequence's rows and state are the same bits alone and beside others, shorter and longer: its own length decides how its
+    tokens are composed (up to 192 one way, from 193 on another), not the step's."""
+    from airframe_b200 import kernels
+    lens, slots = [1, 1000, 17, 128, 129, 192, 193, 300], [3, 0, 2, 7, 1, 4, 6, 5]
+    T = sum(lens)
+    g = torch.Generator().manual_seed(width)
+    proj = (torch.randn(T, 3 * width, generator=g) * 2).to(DEV)
+    bz, bx, start = (torch.randn(*s, generator=g).to(DEV) for s in ((width,), (width,), (8, width)))
+
+    def run(rows, some, where):
+        state, y = start.clone(), torch.full((rows.stop - rows.start, width), float("nan"), device=DEV)
+        kernels.gated_scan(y, proj[rows], 0, width, 2 * width, bz, bx, state, prompt_batch(some, where))
+        return y, state
+
+    y, state = run(slice(0, T), lens, slots)
+    pieces = list(in_order(lens))
+    for (rows, n), slot in zip(pieces, slots):
+        alone, left = run(rows, [n], [slot])
+        assert torch.equal(alone, y[rows]) and torch.equal(left[slot], state[slot]), n
+    for some in ([0, 2, 3], [4, 5], [6, 0], [7, 3]):          # (neighbours in another step)
+        data = torch.cat([proj[pieces[i][0]] for i in some])
+        st, out = start.clone(), torch.empty(len(data), width, device=DEV)
+        kernels.gated_scan(out, data, 0, width, 2 * width, bz, bx, st, prompt_batch([lens[i] for i in some], [slots[i] for i in some]))
+        assert torch.equal(out, torch.cat([y[pieces[i][0]] for i in some]))
