@@ -1,12 +1,14 @@
 // 32-bit matrix product out[M, N] = x[M, K] * w[N, K]^T for prompts, on the 5th-generation tensor cores.
 //
-// Every operand is taken apart, without a rounding, into three bfloat16 parts: x = hi + mid + lo, each the leading 8 bits
-// of what the parts before it leave (24 bits in all: the whole mantissa).  Of the nine products of parts six are taken, from
-// the smallest up: lo hi, hi lo, mid mid, mid hi, hi mid, hi hi; what is left out is below 2^-23 of a product.  The
+// Every operand is taken apart into three bfloat16 parts: x = hi + mid + lo, each the nearest to what the parts before it leave.
+// The remainders are exact and have a sign, so the three hold all 24 bits where 2^-110 <= |x| < 3.38e38 (bfloat16 ends at
+// 2^-133: below, lo is off by up to 2^-134; above, hi is infinite: see the end).  Of the nine products of parts six are
+// taken, from the smallest up: lo hi, hi lo, mid mid, mid hi, hi mid, hi hi; what is left out (mid lo, lo mid, lo lo) is at most
+// 2^-24 of a product, of either sign (parts cut off instead of rounded leave out up to 2^-21, always of the product's sign).  The
 // tensor cores' accumulator rounds towards zero, which over a long sum would drift: it holds 64 products of K at a time
 // and the blocks' sums are added up in registers, in index order, by 32-bit additions that round to nearest.  Distance from
-// the product in 64 bits (2-norm, normal values): 1.2e-7 to 1.7e-7 for K of 64 to 9,216, where the chain of fmaf is 1.5e-7 to
-// 1.7e-6 away.
+// the product in 64 bits (2-norm) for K of 64 to 9,216: normal values 7.7e-8 to 1.3e-7, where the chain of fmaf is 1.4e-7 to
+// 1.7e-6 away; positive ones from 1 to 2 6.1e-8 to 7.6e-8 (on average -0.9 x 2^-24, the accumulator's), the chain 1.2e-7 to 1.5e-6.
 //
 // A block makes 128 features (weight rows: the MMA's A operand, TMEM lanes) by NT tokens.  The tokens' parts come from a
 // small kernel and by TMA; the weights stay as they are in memory and are taken apart on their way into shared memory:
@@ -20,7 +22,8 @@
 // a test a value, and the exact chain unrolled into the epilogue), weights were asked into L2 ahead, and TMEM was read
 // 32 columns at a time.
 //
-// An output that is not finite is made again as a plain chain of fmaf (the parts of an infinity are NaN).
+// An output that is not finite is made again as a plain chain of fmaf (the parts of an infinity, and of a value that rounds to
+// one, are NaN).
 #include "umma.cuh"
 
 namespace {
@@ -46,26 +49,24 @@ struct FtArgs {
   int* err;
 };
 
-// The leading 8 bits of x and of what they leave, as bfloat16 bits in the upper halves.
-__device__ __forceinline__ void ft_split(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const uint32_t b = __float_as_uint(x);
-  hi = b & 0xffff0000u;
-  const float r1 = x - __uint_as_float(hi);
-  mid = __float_as_uint(r1) & 0xffff0000u;
-  lo = __float_as_uint(r1 - __uint_as_float(mid));         // (inf and NaN leave NaN: their outputs are made again)
+// Two values into their parts, a pair of bfloat16 each (x below): rounded two at a time.
+__device__ __forceinline__ uint32_t ft_nearest(float x, float y) {
+  uint32_t p;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(y), "f"(x));
+  return p;
 }
-__device__ __forceinline__ uint32_t ft_pack(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
+__device__ __forceinline__ void ft_split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = ft_nearest(x, y);
+  x -= __uint_as_float(hi << 16), y -= __uint_as_float(hi & 0xffff0000u);
+  mid = ft_nearest(x, y);
+  x -= __uint_as_float(mid << 16), y -= __uint_as_float(mid & 0xffff0000u);
+  lo = ft_nearest(x, y);                                   // (what is not finite leaves NaN: its outputs are made again)
+}
 
 // Four values into three tiles of packed parts.
 __device__ __forceinline__ void ft_split4(float4 v, uint2 (&p)[3]) {
-  uint32_t h[4], m[4], l[4];
-  ft_split(v.x, h[0], m[0], l[0]);
-  ft_split(v.y, h[1], m[1], l[1]);
-  ft_split(v.z, h[2], m[2], l[2]);
-  ft_split(v.w, h[3], m[3], l[3]);
-  p[0] = make_uint2(ft_pack(h[0], h[1]), ft_pack(h[2], h[3]));
-  p[1] = make_uint2(ft_pack(m[0], m[1]), ft_pack(m[2], m[3]));
-  p[2] = make_uint2(ft_pack(l[0], l[1]), ft_pack(l[2], l[3]));
+  ft_split2(v.x, v.y, p[0].x, p[1].x, p[2].x);
+  ft_split2(v.z, v.w, p[0].y, p[1].y, p[2].y);
 }
 
 // The tokens' parts: [3][rows][Kp] bfloat16, zeros from K on.

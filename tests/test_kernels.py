@@ -215,9 +215,9 @@ def test_gemm_plain_shapes_agree_bit_for_bit(K, M, N, K_dim):
 @pytest.mark.parametrize("M, N", [(1, 128), (32, 1), (33, 129), (100, 260), (160, 127), (161, 4096), (301, 2304)])
 def test_gemm_f32_on_the_tensor_cores(K, M, N, K_dim):
     """Edges of tiles, K blocks, splits and their joins; rows apart; a row's bits do not depend on the rows beside it.  Bound: a
-    product loses 2^-22 at most (what the parts leave out), a block of 64 is 24 additions that round towards zero (2^-23 of
+    product loses 2^-24 at most (what the parts leave out), a block of 64 is 24 additions that round towards zero (2^-23 of
     the block's sum of |x w| each), the blocks are joined by K / 64 additions that round to nearest: together below
-    (56 + K / 64) 2^-24 sum |x w|.  And in the 2-norm it is no further off than the chain of fused multiply-adds."""
+    (50 + K / 64) 2^-24 sum |x w|.  And in the 2-norm it is no further off than the chain of fused multiply-adds."""
     x, w = torch.randn(M, K_dim), torch.randn(N, K_dim) * 0.02
     ref, size = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
     wide = torch.full((M, K_dim + 8), float("nan"), device=DEV)
@@ -225,7 +225,7 @@ def test_gemm_f32_on_the_tensor_cores(K, M, N, K_dim):
     xd, wd = wide[:, 4:4 + K_dim], w.to(DEV)
     out = torch.full((M, N), float("nan"), device=DEV)
     K.gemm_f32_tc(out, xd, wd)
-    assert bool(((out.cpu().double() - ref).abs() <= (56 + K_dim / 64) * 2.0 ** -24 * size).all())
+    assert bool(((out.cpu().double() - ref).abs() <= (50 + K_dim / 64) * 2.0 ** -24 * size).all())
     chain = torch.empty_like(out)
     K.gemm_plain(chain, xd, wd)
     off, off_chain = (float((t.cpu().double() - ref).norm()) for t in (out, chain))
@@ -240,8 +240,8 @@ def test_gemm_f32_on_the_tensor_cores(K, M, N, K_dim):
 
 
 def test_gemm_f32_on_the_tensor_cores_beyond_finite_values(K):
-    """Infinities, NaN, sums that overflow and the largest values come out as a chain of multiply-adds has them; values near
-    the smallest lose nothing that counts (the parts reach as far down as the values)."""
+    """Infinities, NaN, sums that overflow and the largest values come out as a chain of multiply-adds has them; values of 1e-30
+    lose nothing (the parts hold all bits down to 2^-110)."""
     x, w = torch.randn(40, 200), torch.randn(130, 200)
     x[1, 3], x[2, 7], x[3, 190], x[4, 5], x[4, 6] = math.inf, -math.inf, math.nan, math.inf, -math.inf
     x[5], x[6, 0] = 3e38, 3.4028234e38
@@ -261,6 +261,39 @@ def test_gemm_f32_on_the_tensor_cores_beyond_finite_values(K):
     ref = x.double() @ w.double().T
     size = x.abs().double() @ w.abs().double().T
     assert bool(((out.double() - ref).abs()[fin] <= 64 * 2.0 ** -24 * size[fin]).all())
+
+
+@pytest.mark.parametrize("K_dim", [64, 256, 2304])
+@pytest.mark.parametrize("mantissas", [(0x80ffff, 0x80ffff), (0x80ff00, 0x80ffff), (0x800000, 0xffffff)])
+def test_gemm_f32_on_the_tensor_cores_of_one_sign(K, mantissas, K_dim):
+    """Operands from 1 to 2, all positive, of the mantissas whose parts, cut off instead of rounded, leave out most (2^-21 of a product)
+    and of any: nothing cancels.  Bound, in 2^-24 of the sum: the parts leave out 1; the last four of a block's 24
+    additions meet a quarter, a half, three quarters and all of its sum and round it towards zero, by 2 at most (5 together),
+    the twenty before them 2^-6 of it at most (1 together); the K / 64 blocks are joined by additions of 1.  On average the
+    parts leave out nothing and an addition half as much: 3 together, and the joins, which round to nearest, nothing
+    (values alike round alike: no average there)."""
+    lo, hi = (m - 0x800000 + 0x3f800000 for m in mantissas)
+    x, w = (torch.randint(lo, hi + 1, (n, K_dim), dtype=torch.int32).view(torch.float32) for n in (40, 130))
+    out = torch.empty(40, 130, device=DEV)
+    K.gemm_f32_tc(out, x.to(DEV), w.to(DEV))
+    ref = x.double() @ w.double().T
+    off = (out.cpu().double() - ref) / ref * 2.0 ** 24
+    assert float(off.abs().max()) <= 7 + (K_dim / 64 if K_dim > 64 else 0), float(off.abs().max())
+    if lo != hi:
+        assert abs(float(off.mean())) <= 3, float(off.mean())
+
+
+@pytest.mark.parametrize("power", [-100, -108, -115, -125, -140])
+def test_gemm_f32_on_the_tensor_cores_of_small_values(K, power):
+    """Below 2^-110 the lowest part ends before the value does (bfloat16's last bit is 2^-133): an operand is off by 2^-134 at most
+    there, and a product by as much times the other operand; above, nothing is lost."""
+    x, w = torch.randn(40, 200) * 2.0 ** power, torch.randn(130, 200)
+    out = torch.empty(40, 130, device=DEV)
+    K.gemm_f32_tc(out, x.to(DEV), w.to(DEV))
+    xd, wd = x.double(), w.double()
+    size = xd.abs() @ wd.abs().T
+    least = 0 if power >= -100 else 2.0 ** -133 * wd.abs().sum(1)[None]      # (a rounding of the smallest sums is as large again)
+    assert bool(((out.cpu().double() - xd @ wd.T).abs() <= (50 + 4) * 2.0 ** -24 * size + least).all())
 
 
 def _paged(k, v, order, n_pages, dtype):
