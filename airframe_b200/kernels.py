@@ -206,12 +206,14 @@ def gemm_plain(out, x, w, cap: float = 0.0) -> None:
 # 301 45 / 36: the lines cross between 2^27 and 2^28.
 F32_TC_ROWS = 32
 F32_TC_WORK = 1 << 28
+# Scratch that a product holds (the parts of its rows, and partial sums where K is cut): more rows than fit go in several launches.
+F32_TC_BYTES = 128 << 20
 
 
 def gemm_f32_tc_supported(x, w, out) -> bool:
     """Whether :func:`gemm_f32_tc` takes these and is the kernel for them."""
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32
-            and F32_TC_ROWS <= x.shape[0] <= 65535 and x.shape[0] * w.numel() >= F32_TC_WORK
+            and x.shape[0] >= F32_TC_ROWS and x.shape[0] * w.numel() >= F32_TC_WORK
             and x.shape[1] % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1
             and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and (x.data_ptr() | w.data_ptr()) % 16 == 0)
 
@@ -226,11 +228,16 @@ def gemm_f32_tc(out, x, w, cap: float = 0.0) -> None:
     splits = _lib().af_gemm_f32_tc_splits(c_int(N), c_int(K))
     if splits < 1:
         _check(splits or -1)
-    parts = torch.empty(3 * M * ((K + 63) // 64 * 64), dtype=torch.bfloat16, device=x.device)
-    sums = torch.empty(splits * M * N, dtype=torch.float32, device=x.device) if splits > 1 else None
-    _check(_lib().af_gemm_f32_tc(_ptr(out), c_longlong(_rows(out, "out")), _ptr(x), c_longlong(_rows(x, "x")), _ptr(w),
-                                 c_longlong(_rows(w, "w")), c_int(M), c_int(N), c_int(K), c_float(cap), _ptr(parts),
-                                 _ptr(sums, allow_none=True), _ptr(error_word(x.device), "err", torch.int32), _stream()))
+    Kp = (K + 63) // 64 * 64
+    a_row = 6 * Kp + (4 * splits * N if splits > 1 else 0)
+    most = min(M, 65535, max(160, F32_TC_BYTES // a_row // 160 * 160))         # (160: the rows of a tile)
+    parts = torch.empty(3 * most * Kp, dtype=torch.bfloat16, device=x.device)
+    sums = torch.empty(splits * most * N, dtype=torch.float32, device=x.device) if splits > 1 else None
+    for r in range(0, M, max(most, 1)):
+        some, to = (x, out) if most == M else (x[r:r + most], out[r:r + most])
+        _check(_lib().af_gemm_f32_tc(_ptr(to), c_longlong(_rows(out, "out")), _ptr(some), c_longlong(_rows(x, "x")), _ptr(w),
+                                     c_longlong(_rows(w, "w")), c_int(some.shape[0]), c_int(N), c_int(K), c_float(cap), _ptr(parts),
+                                     _ptr(sums, allow_none=True), _ptr(error_word(x.device), "err", torch.int32), _stream()))
 
 
 # ---------------------------------------------------------------- attention

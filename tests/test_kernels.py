@@ -296,6 +296,30 @@ def test_gemm_f32_on_the_tensor_cores_of_small_values(K, power):
     assert bool(((out.cpu().double() - xd @ wd.T).abs() <= (50 + 4) * 2.0 ** -24 * size + least).all())
 
 
+def test_gemm_f32_on_the_tensor_cores_of_many_rows(K, monkeypatch):
+    """More rows than the scratch holds go in several launches: the same bits, and no more scratch than allowed; more rows than a
+    grid's second axis takes too."""
+    x, w = torch.randn(500, 2048, device=DEV), torch.randn(256, 2048, device=DEV)
+    whole, got = torch.empty(500, 256, device=DEV), torch.empty(500, 300, device=DEV)[:, 20:276]
+    K.gemm_f32_tc(whole, x, w, cap=30.0)
+    monkeypatch.setattr(K, "F32_TC_BYTES", 1)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    K.gemm_f32_tc(got, x, w, cap=30.0)
+    splits = K._lib().af_gemm_f32_tc_splits(256, 2048)
+    assert splits > 1 and torch.cuda.max_memory_allocated() - before <= 160 * (6 * 2048 + 4 * splits * 256) + 2048
+    assert torch.equal(got, whole)
+    monkeypatch.undo()
+    x, w = torch.randn(65536 + 200, 64, device=DEV), torch.randn(8, 64, device=DEV)
+    out = torch.empty(len(x), 8, device=DEV)
+    K.gemm_f32_tc(out, x, w)
+    for r in (0, 65534, 65535, 65536, len(x) - 1):
+        one = torch.empty(1, 8, device=DEV)
+        K.gemm_f32_tc(one, x[r:r + 1], w)
+        assert torch.equal(one[0], out[r]), r
+
+
 def _paged(k, v, order, n_pages, dtype):
     """Scatter k, v [T, nkv, hd] of one sequence into pages in the given order."""
     T, nkv, hd = k.shape
