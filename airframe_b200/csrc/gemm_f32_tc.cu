@@ -18,7 +18,7 @@
 // Two stages of 64 of K, two accumulators in turn.  Bound by the worker warps' instructions (taking a value apart, five and a
 // half each) and, with 160 tokens, by shared memory (an MMA of 128 x 160 x 16 reads 9 KB of it in 80 cycles of products; the
 // parts are written besides).  301 x 18432 x 2304: 132 us (194 TFLOP/s of 32-bit products), where the CUDA cores' kernel
-// (gemm_plain.cu), which keeps the few rows and the small products, takes 592; before the rare values left the way (182 us:
+// (gemm_plain.cu), which keeps the single tokens' and the small weights' products, takes 592; before the rare values left the way (182 us:
 // a test a value, and the exact chain unrolled into the epilogue), weights were asked into L2 ahead, and TMEM was read
 // 32 columns at a time.
 //

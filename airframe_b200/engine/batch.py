@@ -38,6 +38,7 @@ class StepBatch:
     want_rows: Optional[torch.Tensor]   # int32 [R] rows whose logits are wanted
     n_want: int = 0
     max_len_after: int = 0              # host: longest sequence after the step
+    want_counts: Optional[list] = None  # host: rows wanted per sequence
     step_kv: dict = field(default_factory=dict)   # cache id -> (k, v) of this step, for runs that share a cache
     # what parts make once per forward pass and share between layers (a table of rotary cosines and sines,
     # the tokens' rows in a group's cache pages); emptied when a pass begins
@@ -89,4 +90,4 @@ def build_batch(entries, lens_before, device, pad_to: int = 0) -> StepBatch:
         is_prefill=is_prefill, n_tokens=T, n_seqs=Bp, max_len=max(seq_lens), seq_lens=seq_lens,
         tokens=cut(T), positions=cut(T), seq_of_token=cut(T), slots=cut(Bp), len_after=cut(Bp),
         seq_starts=cut(Bp + 1), want_rows=cut(R) if R else None, n_want=R,
-        max_len_after=max(len_after))
+        max_len_after=max(len_after), want_counts=[len(e.want) for e in entries])

@@ -157,10 +157,12 @@ class Model:
         kernels.stream_sum(out, x, self.streams)
         return out
 
-    def logits(self, x, want_rows) -> torch.Tensor:
-        """float32 logits [R, V] at the wanted rows of the residual stream."""
+    def logits(self, x, want_rows, counts=None) -> torch.Tensor:
+        """float32 logits [R, V] at the wanted rows of the residual stream.  ``counts``: a prefill step's wanted rows per
+        sequence (a head may take rows of sequences that want many another way)."""
         y = self.final_norm.forward(x, self.ctx.compute_dtype, rows=want_rows)
-        return self.head.forward(y)
+        prompt = getattr(self.head, "prompt_logits", None) if counts else None
+        return self.head.forward(y) if prompt is None else prompt(y, counts)
 
     def greedy_tokens(self, x, want_rows) -> torch.Tensor:
         """int32 [R]: the arg-max token at the wanted rows (a head that can, finds
@@ -180,7 +182,9 @@ class Model:
         x = self.hidden(batch, cache, probe)
         if batch.want_rows is None:
             return None
-        return self.greedy_tokens(x, batch.want_rows) if greedy else self.logits(x, batch.want_rows)
+        if greedy:
+            return self.greedy_tokens(x, batch.want_rows)
+        return self.logits(x, batch.want_rows, batch.want_counts if batch.is_prefill else None)
 
 
 def declared_weights(spec: ModelSpec) -> list:

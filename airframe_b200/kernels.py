@@ -200,21 +200,20 @@ def gemm_plain(out, x, w, cap: float = 0.0) -> None:
                                 _stream()))
 
 
-# From how many rows, and how many multiply-adds, a 32-bit product goes to the tensor cores.  The CUDA cores' kernel and this
-# one, us (N x K, rows): 18432 x 2304: 32 91 / 74, 64 158 / 73, 301 592 / 132; 2304 x 9216: 32 88 / 68, 301 438 / 82;
-# 4096 x 2304: 32 54 / 47, 64 59 / 48, 301 192 / 61; 2304 x 2048: 32 34 / 37, 64 48 / 36, 301 108 / 41; 1024 x 1024: 160 32 / 37,
-# 301 45 / 36: the lines cross between 2^27 and 2^28.
-F32_TC_ROWS = 32
-F32_TC_WORK = 1 << 28
+# From how many values of the weight on a prompt's 32-bit product goes to the tensor cores: the weight alone decides, so that a row's
+# bits do not depend on how many rows the step has.  A decode step's goes to the CUDA cores' kernel, whatever its rows.  The
+# CUDA cores' kernel and this one, us (N x K: 1, 16, 64, 301 rows): 18432 x 2304 53 / 56, 88 / 58, 152 / 60, 588 / 128; 2304 x 9216
+# 39 / 55, 57 / 58, 172 / 59, 447 / 83; 4096 x 2304 16 / 32, 29 / 32, 53 / 36, 184 / 46; 2304 x 2048 14 / 22, 18 / 22, 43 / 24, 105 / 30;
+# 1024 x 1024 10 / 20, 12 / 19, 16 / 20, 39 / 26 (1,024 rows: 74 / 30).
+F32_TC_WEIGHT = 1 << 20
 # Scratch that a product holds (the parts of its rows, and partial sums where K is cut): more rows than fit go in several launches.
 F32_TC_BYTES = 128 << 20
 
 
 def gemm_f32_tc_supported(x, w, out) -> bool:
-    """Whether :func:`gemm_f32_tc` takes these and is the kernel for them."""
+    """Whether :func:`gemm_f32_tc` takes these and is a prompt's kernel for them."""
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32
-            and x.shape[0] >= F32_TC_ROWS and x.shape[0] * w.numel() >= F32_TC_WORK
-            and x.shape[1] % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1
+            and w.numel() >= F32_TC_WEIGHT and x.shape[1] % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1
             and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and (x.data_ptr() | w.data_ptr()) % 16 == 0)
 
 

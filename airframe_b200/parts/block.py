@@ -217,24 +217,24 @@ class NormedSumBlock(Block):
     def first_read(self, view, batch):
         return ShiftedReader(self, view, batch)
 
-    def _gate(self, which: int, y):
+    def _gate(self, which: int, y, batch):
         """The arguments that put this sublayer's gate into the kernel of its residual sum."""
         if self.gates[which] is None:
             return {}
         w, b = self.gates[which]
-        z = linear_split(y, w, wide=True)
+        z = linear_split(y, w, wide=True, prompt=batch.is_prefill)
         return {"gate": z.parts if isinstance(z, PartialSums) else z, "gate_bias": b}
 
     def forward(self, x, batch, view, normed=None, next_pre=None):
         dt = self.ctx.compute_dtype
         y, h = normed if normed is not None else ShiftedReader(self, view, batch).forward(x, dt)
-        gate = self._gate(0, y)
+        gate = self._gate(0, y, batch)
         a = self.mixer.forward(h, batch, view)
         if not self.feed_forward.present:
             return self._close(self.norms["mixer_sum"], x, a, gate, batch, next_pre)
         y = x if dt == torch.float32 else torch.empty_like(x, dtype=dt)
         self.norms["mixer_sum"].of_sum(x, a, self.alpha, y=None if y is x else y, **gate)
-        gate = self._gate(1, y)
+        gate = self._gate(1, y, batch)
         return self._close(self.norms["feed_forward_sum"], x, self.feed_forward.forward(y, batch), gate, batch, next_pre)
 
     def _close(self, norm, x, a, gate, batch, next_pre):

@@ -9,6 +9,8 @@ no separate matrix exists, ``src/runtime/gpu.rs:763-795``).
 """
 from __future__ import annotations
 
+import itertools
+
 import torch
 
 from .. import kernels
@@ -100,6 +102,26 @@ class LmHead(Part):
     def forward(self, y):
         """y [R, H] compute dtype (after the final norm) -> float32 logits [R, V]."""
         logits = linear(y, self.w, out_dtype=torch.float32, cap=self.softcap)
+        if self.scale != 1.0:
+            kernels.scale_(logits, self.scale)
+        return logits
+
+    SCORE_ROWS = 32      # rows that a sequence wants at least to be scored rather than continued
+
+    def prompt_logits(self, y, counts):
+        """:meth:`forward` of a prefill step's rows, ``counts`` of them a sequence, one after the other.  In 32 bits the rows of
+        a sequence that wants many go to the product for prompts, those of one that wants a few (its last) to the one for
+        few rows: what a sequence asks for decides, not the step, so that its bits do not depend on its neighbours.
+        256000 x 2304, one row 365 us against 630 with the prompts' product, 301 rows 7,530 against 1,840."""
+        if y.dtype != torch.float32 or max(counts) < self.SCORE_ROWS:
+            return self.forward(y)
+        logits = torch.empty(y.shape[0], self.vocab, dtype=torch.float32, device=y.device)
+        at = 0
+        for many, run in itertools.groupby(counts, lambda n: n >= self.SCORE_ROWS):
+            n = sum(run)
+            if n:
+                linear(y[at: at + n], self.w, cap=self.softcap, out=logits[at: at + n], prompt=many)
+            at += n
         if self.scale != 1.0:
             kernels.scale_(logits, self.scale)
         return logits

@@ -49,7 +49,7 @@ class Reinject(Junction):
     def forward(self, x, x0, index, batch, then=None, out_dtype=None):
         both = torch.empty(x.shape[0], 2 * self.hidden, dtype=self.ctx.compute_dtype, device=x.device)
         kernels.concat_cast(both, x, x0)
-        z = linear_split(both, self.w, wide=True)
+        z = linear_split(both, self.w, wide=True, prompt=batch.is_prefill)
         z = z.parts if isinstance(z, PartialSums) else z
         if then is None or not isinstance(then, TanhNorm):
             kernels.set_sum_row(x, z, self.steps[index])

@@ -90,8 +90,8 @@ class GatedMlp(FeedForward):
         return 2 * sum(lens) * 3 * self.hidden * self.inter
 
     def forward(self, x, batch):
-        h = gated_linear(x, self.w_gu, self.inter, self.activation, self.interleaved)
-        return linear_split(h, self.w_down, wide=bool(self.params.get("wide_output", False)))
+        h = gated_linear(x, self.w_gu, self.inter, self.activation, self.interleaved, prompt=batch.is_prefill)
+        return linear_split(h, self.w_down, wide=bool(self.params.get("wide_output", False)), prompt=batch.is_prefill)
 
 
 @register_part("feed_forward", "none")
@@ -144,11 +144,11 @@ class TokenSide(FeedForward):
         return 4 * sum(lens) * self.hidden * self.dim
 
     def forward(self, x, batch):
-        z = linear_split(x, self.w_gate, wide=True)
+        z = linear_split(x, self.w_gate, wide=True, prompt=batch.is_prefill)
         g = torch.empty(x.shape[0], self.dim, dtype=x.dtype, device=x.device)
         kernels.token_gate(g, z.parts if isinstance(z, PartialSums) else z, self.table, self.index * self.dim, batch.tokens,
                            self.activation)
-        return linear_split(g, self.w_proj, wide=True)
+        return linear_split(g, self.w_proj, wide=True, prompt=batch.is_prefill)
 
 
 @register_part("feed_forward", "routed_experts")

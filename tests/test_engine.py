@@ -115,6 +115,57 @@ def test_the_same_work_gives_the_same_bits(case, dtype):
     assert torch.equal(a, b)
 
 
+def test_32_bit_prompts_alone_and_in_a_batch(case):
+    """In 32 bits a prompt's logits are the same bits alone and beside others, whether its last row is wanted or all: what is in
+    the step besides decides neither a product's kernel nor an order of sums.  (Steps of less than 256 rows: from there on the
+    norm of a residual sum has half the threads a row, another order of the row's one sum.)"""
+    from airframe_b200.engine import StepEntry
+    rt = runtime(case, "float32")
+    reqs = []
+    for r in sorted(case["requests"], key=len):
+        if sum(map(len, reqs)) + len(r) < 256:
+            reqs.append(r)
+    reqs = reqs[::2] + reqs[1::2]
+    longest = max(range(len(reqs)), key=lambda i: len(reqs[i]))
+    wants = [list(range(len(r))) if i == longest else [len(r) - 1] for i, r in enumerate(reqs)]
+
+    def run(which):
+        slots = [rt.engine.take_slot() for _ in which]
+        try:
+            out = rt.step([StepEntry(s, reqs[i], wants[i]) for s, i in zip(slots, which)])
+        finally:
+            for s in slots:
+                rt.engine.free_slot(s)
+        return list(out.split([len(wants[i]) for i in which]))
+
+    together = run(range(len(reqs)))
+    for i in range(len(reqs)):
+        assert torch.equal(run([i])[0], together[i]), len(reqs[i])
+    assert torch.equal(run([1, longest])[1], together[longest])
+
+
+def test_32_bit_decode_of_many_sequences(case):
+    """A captured 32-bit step of 40 sequences against the same sequences eight at a time: the products of single tokens run on one
+    kernel whatever the batch (the attention's cut of the keys goes by the batch, so not bit for bit)."""
+    from airframe_b200.engine import GpuRuntime, StepEntry
+    if case["name"] != "D":
+        return
+    rt = GpuRuntime.load(case["folder"], dtype="float32", max_tokens=64 * 48)
+    ids = [replay.random_ids(case["cfg"]["vocab_size"], 6, 300 + i) for i in range(40)]
+
+    def run(group):
+        slots, got = [rt.engine.take_slot() for _ in group], []
+        rt.step([StepEntry(s, r[:3], []) for s, r in zip(slots, group)])
+        for t in range(3, 6):
+            got.append(rt.step([StepEntry(s, [r[t]], [0]) for s, r in zip(slots, group)]).clone())
+        for s in slots:
+            rt.engine.free_slot(s)
+        return torch.stack(got, 1)
+
+    many, few = run(ids), torch.cat([run(ids[i:i + 8]) for i in range(0, 40, 8)])
+    assert rel_err(many, few.cpu()) < SPLITS["float32"]
+
+
 @pytest.mark.parametrize("lens", [[1], [17], [64], [130], [210], [3, 64, 1, 40, 33], [5, 5]])
 def test_prompt_layers_launched_by_one_call(case, lens):
     """Where a model's prompts go through one call into the library, logits and cache pages are those of the same kernels

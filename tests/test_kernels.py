@@ -320,6 +320,21 @@ def test_gemm_f32_on_the_tensor_cores_of_many_rows(K, monkeypatch):
         assert torch.equal(one[0], out[r]), r
 
 
+@pytest.mark.parametrize("N, K_dim, cores", [(1024, 1024, True), (1023, 1024, False), (300, 4096, True), (1100, 1023, False)])
+def test_which_32_bit_product(K, N, K_dim, cores):
+    """A prompt's product goes to the tensor cores from a weight of 2^20 values on (rows in whole 16-byte pieces), any other to the
+    CUDA cores: the number of rows decides nothing, so that a row has the bits that it has alone."""
+    from airframe_b200.parts.linear import linear
+    x, w = torch.randn(300, K_dim, device=DEV), torch.randn(N, K_dim, device=DEV)
+    alone = {}
+    for M in (1, 31, 32, 33, 255, 256, 300):
+        for prompt in (False, True):
+            want, got = torch.empty(M, N, device=DEV), linear(x[:M], w, prompt=prompt)
+            (K.gemm_f32_tc if prompt and cores else K.gemm_plain)(want, x[:M], w)
+            assert torch.equal(got, want), (M, prompt)
+            assert torch.equal(got[0], alone.setdefault(prompt, got[0])), (M, prompt)
+
+
 def _paged(k, v, order, n_pages, dtype):
     """Scatter k, v [T, nkv, hd] of one sequence into pages in the given order."""
     T, nkv, hd = k.shape
