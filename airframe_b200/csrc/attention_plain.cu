@@ -419,14 +419,15 @@ __device__ __forceinline__ float gate_factor(const float* gate, long long gate_s
 }
 
 // Prompts that start at position 0: keys and values are the step's own rows.
-// Block w of the grid handles (token, head) = (w / nq, w % nq): one warp, or from AF_PLAIN_SPLIT visible keys on four, a quarter
-// of the keys each, joined through shared memory (a token's number of keys alone decides).  A warp's chain from keys to keys
-// is what takes the time: the last tokens' walk was as long as the kernel while most warps were done.  301 tokens, 8 heads of
-// 256 in 32 bits: 105 -> 67 us.  `hd` is the key size, `dv` the value
+// A block handles a (token, head), the last tokens first: one of its warps, or from AF_PLAIN_SPLIT visible keys on all four, a
+// quarter of the keys each, joined through shared memory (a token's number of keys alone decides).  A warp's chain from keys to
+// keys is what takes the time: the last tokens' walk was as long as the kernel while most warps were done.  301 tokens, 8 heads
+// of 256 in 32 bits: 105 -> 67 us.  FEW: no token of the step sees so many, and a block's warps take a (token, head) each; where
+// three of four warps had nothing to do, 64 prompts of 30 tokens took 80 us for 55.  `hd` is the key size, `dv` the value
 // size; the first `keep` positions stay visible whatever the window; `sinks` (float [nq]) and `gate` (float logits, row t and column h at gate[t * gate_stride + h]:
 // the head's output is multiplied by their sigmoid) may be null.
 #define AF_PLAIN_SPLIT 64
-template <typename T, int NS>
+template <typename T, int NS, bool FEW>
 __global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__ out, int out_stride, const T* __restrict__ q,
                                           int q_stride, const T* __restrict__ k, int k_stride,
                                           const T* __restrict__ v, int v_stride,
@@ -437,8 +438,10 @@ __global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__
                                           long long gate_stride) {
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31, split = threadIdx.x >> 5;
-  const int t = n_tokens - 1 - (int)(blockIdx.x / nq), h = (int)(blockIdx.x % nq);      // (the last tokens, which see most, first)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, split = FEW ? 0 : warp;
+  const long long unit = FEW ? (long long)blockIdx.x * 4 + warp : blockIdx.x;
+  if (FEW && unit >= (long long)n_tokens * nq) return;
+  const int t = n_tokens - 1 - (int)(unit / nq), h = (int)(unit % nq);      // (the last tokens, which see most, first)
   const int g = h / (nq / nkv);
   const int pos = positions[t];          // position inside its sequence
   const int first_row = t - pos;         // row of the sequence's position 0
@@ -450,7 +453,7 @@ __global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__
   const float slope = slopes ? slopes[h] : 0.f;
   const int kept = min(keep, lo);         // the first tokens that stay visible before the window
   const int n_vis = kept + pos - lo + 1;
-  const int splits = n_vis >= AF_PLAIN_SPLIT ? 4 : 1;
+  const int splits = !FEW && n_vis >= AF_PLAIN_SPLIT ? 4 : 1;
   if (split >= splits) return;
   const int per = ((n_vis + splits - 1) / splits + 3) / 4 * 4, end = min(n_vis, (split + 1) * per);
   int x = split * per;
@@ -472,7 +475,7 @@ __global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__
     attn_key(st, k + r * k_stride + (size_t)g * hd, v + r * v_stride + (size_t)g * dv, hd, dv, lane, scale,
              cap, slope * (float)(j - pos));
   }
-  if (splits > 1) {
+  if (!FEW && splits > 1) {
     __shared__ float o_s[3][32 * NS], m_s[4], l_s[4];
     if (split > 0) {
 #pragma unroll
@@ -498,11 +501,12 @@ __global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__
   attn_store(st, out + (size_t)t * out_stride + (size_t)h * dv, dv, lane, gate_factor(gate, gate_stride, t, h));
 }
 
+// `max_keys`: no token sees more.
 AF_EXPORT int af_attn_prefill_plain(void* out, int out_stride, const void* q, int q_stride,
                                     const void* k, int k_stride, const void* v, int v_stride, int dtype,
                                     const int* positions, int n_tokens, int nq, int nkv, int hd, int dv,
                                     float scale, float cap, int window, int mask_kind, int keep, const float* slopes,
-                                    const float* sinks, const float* gate, long long gate_stride,
+                                    const float* sinks, const float* gate, long long gate_stride, int max_keys,
                                     cudaStream_t stream) {
   if (n_tokens == 0) return 0;
   AF_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "af_attn_prefill_plain: heads %d, groups %d", nq, nkv);
@@ -510,12 +514,14 @@ AF_EXPORT int af_attn_prefill_plain(void* out, int out_stride, const void* q, in
              "af_attn_prefill_plain: key size %d or value size %d beyond %d", hd, dv, AF_MAX_HD);
   AF_REQUIRE(mask_kind == AF_MASK_WINDOW || mask_kind == AF_MASK_CHUNK, "af_attn_prefill_plain: mask kind %d", mask_kind);
   AF_REQUIRE(keep >= 0, "af_attn_prefill_plain: %d kept tokens", keep);
-  const long long blocks = (long long)n_tokens * nq;
+  const bool few = max_keys < AF_PLAIN_SPLIT;
+  const long long units = (long long)n_tokens * nq, blocks = few ? (units + 3) / 4 : units;
   const int slices = (max(hd, dv) + 31) / 32;
   AF_REQUIRE(blocks < (1ll << 31), "af_attn_prefill_plain: too many rows");
   AF_DISPATCH_DTYPE(dtype, T,
-                    auto kernel = slices <= 4 ? attn_prefill_plain_kernel<T, 4> : slices <= 8 ? attn_prefill_plain_kernel<T, 8>
-                                                                           : attn_prefill_plain_kernel<T, AF_HD_SLICES>;
+                    auto kernel = slices <= 4 ? (few ? attn_prefill_plain_kernel<T, 4, true> : attn_prefill_plain_kernel<T, 4, false>)
+                                  : slices <= 8 ? (few ? attn_prefill_plain_kernel<T, 8, true> : attn_prefill_plain_kernel<T, 8, false>)
+                                  : few ? attn_prefill_plain_kernel<T, AF_HD_SLICES, true> : attn_prefill_plain_kernel<T, AF_HD_SLICES, false>;
                     af_launch(kernel, dim3((unsigned)blocks), dim3(128), 0, stream, 
                         (T*)out, out_stride, (const T*)q, q_stride, (const T*)k, k_stride, (const T*)v,
                         v_stride, positions, n_tokens, nq, nkv, hd, dv, scale, cap, window, mask_kind, keep, slopes,

@@ -330,16 +330,22 @@ def _gate_args(gate, rows: int, nq: int, who: str):
     return _ptr(gate, "gate", torch.float32), c_longlong(gate.stride(0))
 
 
+def _most_keys(max_len: int, window: int, keep: int) -> int:
+    """The most keys that a token of prompts of up to ``max_len`` tokens sees."""
+    return min(max_len, window + keep) if window else max_len
+
+
 def attn_prefill_plain(out, q, k, v, positions, nq: int, nkv: int, hd: int, scale: float, cap: float,
                        window: int, slopes=None, dv=None, mask: str = "window", sinks=None, gate=None,
-                       keep: int = 0) -> None:
+                       keep: int = 0, max_len: int = 0) -> None:
     """Attention of prompts that start at position 0 over the step's own keys.
     q [T, nq*hd], k [T, nkv*hd], v [T, nkv*dv] are row views (any row stride; ``dv`` = hd by default).
     ``window`` > 0 with ``mask`` "window": a position sees the last ``window`` ones; "chunk": those of its
     own chunk of ``window`` positions; with either the sequence's first ``keep`` positions stay visible.  ``slopes`` (float32 [nq]): slope[h] * (key position - query position)
     is added to head h's scores after scale and cap (a position encoding that biases scores).  ``sinks``
     (float32 [nq]): exp(sink[h]) joins head h's softmax denominator without a key or a value.  ``gate``
-    (float32 [T, nq] logits): head h's output is multiplied by their sigmoid."""
+    (float32 [T, nq] logits): head h's output is multiplied by their sigmoid.  ``max_len``: no sequence is longer (0: unknown;
+    short prompts have kernels of their own, with the same bits)."""
     if slopes is not None and slopes.numel() != nq:
         raise KernelError(f"attn_prefill_plain: {slopes.numel()} slopes for {nq} heads")
     if sinks is not None and sinks.numel() != nq:
@@ -353,7 +359,8 @@ def attn_prefill_plain(out, q, k, v, positions, nq: int, nkv: int, hd: int, scal
         _ptr(v), c_int(_rows(v, "v")), c_int(dtype_code(q.dtype)), _ptr(positions, "positions", torch.int32),
         c_int(T), c_int(nq), c_int(nkv), c_int(hd), c_int(dv or hd), c_float(scale), c_float(cap), c_int(window),
         c_int(MASKS[mask]), c_int(keep), _ptr(slopes, "slopes", torch.float32, allow_none=True),
-        _ptr(sinks, "sinks", torch.float32, allow_none=True), gp, gs, _stream()))
+        _ptr(sinks, "sinks", torch.float32, allow_none=True), gp, gs,
+        c_int(_most_keys(max_len or T, window, keep)), _stream()))
 
 
 def plain_decode_splits(batch: int, nq: int, most_keys: int) -> int:
@@ -763,7 +770,7 @@ def attn_prefill(out, q, k, v, batch, nq, nkv, hd, scale, cap, window, slopes=No
         and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v))
     if not (use_tc or use_mma):
         attn_prefill_plain(out, q, k, v, batch.positions, nq, nkv, hd, scale, cap, window, slopes, dv=dv, mask=mask,
-                           sinks=sinks, gate=gate, keep=keep)
+                           sinks=sinks, gate=gate, keep=keep, max_len=getattr(batch, "max_len", 0))
         return
     starts, n_seqs, max_len, size = batch.seq_starts, batch.n_seqs, batch.max_len, window
     if mask == "chunk" and window:
@@ -771,7 +778,7 @@ def attn_prefill(out, q, k, v, batch, nq, nkv, hd, scale, cap, window, slopes=No
         window = 0
     if n_seqs > 65535:          # (more sequences than a grid's second axis takes)
         attn_prefill_plain(out, q, k, v, batch.positions, nq, nkv, hd, scale, cap, size, slopes, dv=dv, mask=mask,
-                           sinks=sinks, gate=gate, keep=keep)
+                           sinks=sinks, gate=gate, keep=keep, max_len=batch.max_len)
     elif use_tc:
         attn_prefill_tc(out, q, k, v, starts, n_seqs, max_len, nq, nkv, hd, scale, cap, window, sinks, gate, keep)
     else:

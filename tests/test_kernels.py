@@ -515,6 +515,30 @@ def test_attention_prefill_plain_in_quarters(K, hd, dv):
         assert bool(h2[10:].isfinite().all())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd, dv, nq, nkv", [(64, 64, 3, 1), (200, 136, 6, 2), (300, 520, 1, 1)])
+def test_attention_prefill_plain_of_short_prompts(K, hd, dv, nq, nkv, dtype, monkeypatch):
+    """Steps in which no token sees 64 keys run four (token, head) pairs a block: the bits of the kernel for any step, whether the
+    prompts' length or a window (with first tokens that stay visible) keeps the keys few, and pairs that fill no block."""
+    g = torch.Generator().manual_seed(hd)
+    for lens, window, keep, mask in (([63, 1, 40, 7], 0, 0, "window"), ([100, 30], 50, 13, "window"), ([90, 65], 40, 0, "chunk"), ([1], 0, 0, "window")):
+        T = sum(lens)
+        q, k, v = (torch.randn(T, n, generator=g).to(DEV, dtype) for n in (nq * hd, nkv * hd, nkv * dv))
+        pos = torch.tensor([i for n in lens for i in range(n)], dtype=torch.int32, device=DEV)
+        sinks, gate = torch.randn(nq, generator=g).to(DEV), torch.randn(T, nq, generator=g).to(DEV)
+        outs = []
+        for few in (True, False):
+            with monkeypatch.context() as m:
+                if not few:
+                    m.setattr(K, "_most_keys", lambda *_: 1 << 20)
+                else:
+                    assert K._most_keys(max(lens), window, keep) < 64
+                out = torch.full((T, nq * dv), float("nan"), device=DEV, dtype=dtype)
+                K.attn_prefill_plain(out, q, k, v, pos, nq, nkv, hd, hd ** -0.5, 0.0, window, dv=dv, mask=mask, sinks=sinks, gate=gate,
+                                     keep=keep, max_len=max(lens))
+            outs.append(out)
+        assert torch.equal(outs[0], outs[1]) and bool(outs[0].isfinite().all())
+
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hd,nq,nkv,window,cap", [(16, 4, 2, 0, 50.0), (80, 6, 2, 7, 0.0), (256, 3, 3, 33, 30.0),
