@@ -320,7 +320,11 @@ static int gp_launch(TO* out, int ldo, const float* x, int ldx, const float* w, 
 //   up to 8 rows 49 / 13 / 27 / 71; up to 16 rows 88 / 18 / 28 / 97 against 163 / 39 / 45 / 107 for 32 x 32 tiles, which
 //     are better from two blocks of 16 x 16 an SM on (32 rows: 101 / 25 / 52 / 195 against 165 / 39 / 45 / 109);
 //   301 rows: 32 x 32 tiles 431 / 99 / 179 / 695, 32 x 64 tiles 556 / 126 / 178 / 687 (from three and a half an SM on they
-//     are the better ones), 64 x 128 tiles of pairs 773 / 170 / 320 / 581 (from four and a half an SM on: 44 TFLOP/s).
+//     are the better ones), 64 x 128 tiles of pairs 773 / 170 / 320 / 581 (from four and a half an SM on: 44 TFLOP/s, where the
+//     64 rows are not mostly empty: a tile takes 1.66 times as long as one of 32 x 64 for the same columns).
+// So many rows come with the heads of decode steps (256000 x 2304: 17 to 32 rows 954 in tiles of 32 x 64 against 1,561, 33 to 64 rows
+// 1,870 against 1,565) and with prompts that the tensor cores do not take (18432 x 2302, 301 rows: 827 / 647; 1000 x 1000, 8,192
+// rows: 453 / 361).
 // The kernel that all of these replace, 64 x 64 tiles fetched and then multiplied, took 1,297 us at 301 x 18432 x 2304
 // (20 TFLOP/s) and 230 to 1,000 us for a few rows.
 template <bool VEC, typename TO>
@@ -336,7 +340,7 @@ static int gp_choose(TO* out, int ldo, const float* x, int ldx, const float* w, 
   }
   if (M <= 8) return gp_launch<GpShape<8, 16, 1, 1, 64, 4>, VEC, TO>(GP_ARGS);
   if (M <= 16 || tiles(16, 16) <= 2 * sms) return gp_launch<GpShape<16, 16, 2, 1, 128, 5>, VEC, TO>(GP_ARGS);
-  if (2 * tiles(64, 128) >= 9 * sms) return gp_pair_launch<GpShape<64, 128, 8, 8, 16, 3, 3>, VEC, TO>(GP_ARGS);
+  if (2 * tiles(64, 128) >= 9 * sms && 5 * ((M + 63) / 64) <= 3 * ((M + 31) / 32)) return gp_pair_launch<GpShape<64, 128, 8, 8, 16, 3, 3>, VEC, TO>(GP_ARGS);
   if (2 * tiles(32, 64) >= 7 * sms) return gp_launch<GpShape<32, 64, 4, 4, 32, 4>, VEC, TO>(GP_ARGS);
   return gp_launch<GpShape<32, 32, 4, 4, 32, 4>, VEC, TO>(GP_ARGS);
 #undef GP_ARGS

@@ -189,7 +189,7 @@ def test_gemm_plain_is_true_32_bit_and_batch_invariant(K):
 
 @pytest.mark.parametrize("K_dim", [1, 36, 131, 260])
 @pytest.mark.parametrize("M, N", [(1, 70), (4, 10007), (3, 4801), (8, 130), (7, 33), (16, 97), (17, 65), (33, 2113), (70, 131),
-                                  (1200, 1001), (2000, 2803)])
+                                  (1200, 1001), (2000, 2803), (24, 90001), (40, 90001), (70, 50001)])
 def test_gemm_plain_shapes_agree_bit_for_bit(K, M, N, K_dim):
     """Every shape of the 32-bit product (few rows, narrow and wide blocks, the three tile sizes, whole 16-byte pieces and
     not) gives each row the bits that the row gets alone, and those lie within the error of K sums in 32 bits of the
