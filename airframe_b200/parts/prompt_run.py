@@ -3,7 +3,8 @@
 A short prompt's time is the host's: a launch and what stands around it take some 17 us from Python, the kernel behind
 it less.  Where all runs of a model are of one kind (``sandwich`` blocks of attention with a rotary encoding, a gated
 feed-forward and RMS norms, in bfloat16, of sizes the tensor cores take), their launches are made in the library instead
-(``csrc/prompt_layers.cu``): the same kernels with the same arguments, in the same order.  A prompt of 37 tokens through 26
+(``csrc/prompt_layers.cu``): the same kernels with the same arguments, in the same order (a change of what ``SandwichBlock``,
+``Attention`` or ``GatedMlp`` launch is made there too).  A prompt of 37 tokens through 26
 layers: 3.68 ms part by part, 1.79 ms so (the kernels' own time).  Anything else runs part by part."""
 from __future__ import annotations
 
@@ -22,6 +23,15 @@ _RUN = struct.Struct("<13Q4q6d")
 _STEP = struct.Struct("<13Q18qd")
 
 
+def _matrix(w, rows: int, cols: int) -> bool:
+    """Whether a weight is what its product is told (the bindings, which look at every tensor, are passed by)."""
+    return w.dtype == torch.bfloat16 and tuple(w.shape) == (rows, cols) and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.is_cuda
+
+
+def _vector(w, n: int) -> bool:
+    return w.dtype == torch.float32 and w.numel() == n and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.is_cuda
+
+
 def _alike(block):
     """What the runs of a step have to have in common, or None where a block is not of the kind."""
     m, f = block.mixer, block.feed_forward
@@ -33,7 +43,10 @@ def _alike(block):
             and m.mask == "window" and f.interleaved and f.w_gu.shape[0] == 2 * f.inter
             and not (m.params.get("wide_output") or f.params.get("wide_output"))
             and all(type(n) is RmsNorm and n.offset == norms[0].offset for n in norms)
-            and rope.magnitude == 1.0 and 0 < rope.rotary_dim <= m.hd and m.hidden % 8 == 0 and f.inter % 8 == 0 and m.w_qkv.is_cuda
+            and rope.magnitude == 1.0 and 0 < rope.rotary_dim <= m.hd and m.hidden % 8 == 0 and f.inter % 8 == 0
+            and _matrix(m.w_qkv, (m.nq + 2 * m.nkv) * m.hd, m.hidden) and _matrix(m.w_o, m.hidden, m.nq * m.hd)
+            and _matrix(f.w_gu, 2 * f.inter, m.hidden) and _matrix(f.w_down, m.hidden, f.inter)
+            and all(_vector(n.w, m.hidden) for n in norms) and _vector(rope.inv_freq, rope.rotary_dim // 2)
             and kernels.attn_prefill_tc_supported(m.hd))
     if not fits:
         return None
@@ -49,10 +62,10 @@ def supported(model) -> bool:
 
 
 def run(model, x, batch, cache) -> bool:
-    """All runs of the schedule on the stream ``x`` (float32 [T, H], updated in place).  False: nothing was done, a run's view
-    of the cache is not a plain one."""
+    """All runs of the schedule on the stream ``x`` (float32 [T, H], updated in place).  False: nothing was done (a run's view
+    of the cache is not a plain one, or ``kernels.GEMM_TC_PER_SM`` asks for products of another shape)."""
     views = cache.views
-    if any(not v.writes or v.keep_step_kv for v in views) or batch.n_seqs > 65535:
+    if any(not v.writes or v.keep_step_kv for v in views) or batch.n_seqs > 65535 or kernels.GEMM_TC_PER_SM:
         return False
     blocks = [model.blocks[e.layer] for e in model.spec.schedule]
     first = blocks[0]

@@ -198,6 +198,31 @@ def test_prompt_layers_launched_by_one_call(case, lens):
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and got[0][2] == got[1][2] > 0
 
 
+def test_prompt_layers_that_the_one_call_does_not_take(case, monkeypatch):
+    """Weights off 16 bytes or in another order, which the parts take on their own, do not go through the one call; nor does a step
+    while the products' shape is set by hand."""
+    from airframe_b200 import kernels
+    from airframe_b200.parts import prompt_run
+    rt = runtime(case, "bfloat16")
+    if not rt.model.prompts_as_one:
+        return
+    m, f, n = rt.model.blocks[0].mixer, rt.model.blocks[0].feed_forward, rt.model.blocks[0].norms["post_mixer"]
+    assert prompt_run.supported(rt.model)
+    for part, name in ((m, "w_qkv"), (m, "w_o"), (f, "w_gu"), (f, "w_down"), (n, "w")):
+        w = getattr(part, name)
+        off = torch.empty(w.numel() + 1, dtype=w.dtype, device=w.device)[1:].view(w.shape)
+        with monkeypatch.context() as p:
+            p.setattr(part, name, off)
+            assert not prompt_run.supported(rt.model)
+            if w.dim() == 2:
+                p.setattr(part, name, w.t().contiguous().t())
+                assert not prompt_run.supported(rt.model)
+    with monkeypatch.context() as p:
+        p.setattr(kernels, "GEMM_TC_PER_SM", 1)
+        p.setattr(kernels, "prompt_layers", None)
+        assert replay.run_whole(rt, case["requests"][0]).isfinite().all()
+
+
 def test_decode_steps_fed_from_the_device(case, dtype):
     """``decode_rows``: the step's tokens lie on the device, rows keep their places and a row may be
     unused; the logits are those of the same step fed from the host."""
