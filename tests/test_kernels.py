@@ -504,15 +504,12 @@ def test_attention_prefill_plain_in_quarters(K, hd, dv):
             s = slice(at, at + n)
             i, j = torch.arange(n)[:, None], torch.arange(n)[None, :]
             seen = (j <= i) & ((i - j < win) | (j < kept) if win else True)
-            for h in (0, 1, 3):                     # (head 2's products leave 32 bits: below)
+            for h in range(nq):                     # (head 2's products with some keys leave 32 bits: minus infinity, weight zero)
                 qq, kk, vv = (t[s].double().view(n, -1, d)[:, g] for t, g, d in ((q, h, hd), (k, h // 2, hd), (v, h // 2, dv)))
                 sc = (qq @ kk.T) * hd ** -0.5 + slopes[h].double() * (j - i)
                 sc = torch.cat([sc.masked_fill(~seen, -math.inf), sinks[h].double().expand(n, 1)], 1).softmax(1)[:, :n]
                 close(out[s].view(n, nq, dv)[:, h], sc @ vv, torch.float32)
             at += n
-        # keys whose score is minus infinity weigh nothing
-        h2 = out[-200:].view(200, nq, dv)[:, 2]
-        assert bool(h2[10:].isfinite().all())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
