@@ -217,6 +217,21 @@ def gemm_f32_tc_supported(x, w, out) -> bool:
             and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and (x.data_ptr() | w.data_ptr()) % 16 == 0)
 
 
+_F32_TC_SPLITS = {}
+
+
+def _f32_tc_splits(N: int, K: int) -> int:
+    """Into how many ranges the product cuts K for a weight [N, K] (asked of the library once a size and device)."""
+    key = (_current_device(), N, K)
+    n = _F32_TC_SPLITS.get(key)
+    if n is None:
+        n = int(_lib().af_gemm_f32_tc_splits(c_int(N), c_int(K)))
+        if n < 1:
+            _check(n or -1)
+        _F32_TC_SPLITS[key] = n
+    return n
+
+
 def gemm_f32_tc(out, x, w, cap: float = 0.0) -> None:
     """out[M, N] = x[M, K] @ w[N, K]^T, all float32, on the tensor cores: operands in three bfloat16 parts that hold all 24 bits,
     sums of 64 products joined in 32 bits in index order."""
@@ -224,19 +239,21 @@ def gemm_f32_tc(out, x, w, cap: float = 0.0) -> None:
     N = w.shape[0]
     if w.shape[1] != K or out.shape != (M, N) or not (x.dtype == w.dtype == out.dtype == torch.float32):
         raise KernelError(f"gemm_f32_tc: shapes {tuple(x.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)}, all float32")
-    splits = _lib().af_gemm_f32_tc_splits(c_int(N), c_int(K))
-    if splits < 1:
-        _check(splits or -1)
+    splits = _f32_tc_splits(N, K)
     Kp = (K + 63) // 64 * 64
-    a_row = 6 * Kp + (4 * splits * N if splits > 1 else 0)
-    most = min(M, 65535, max(160, F32_TC_BYTES // a_row // 160 * 160))         # (160: the rows of a tile)
-    parts = torch.empty(3 * most * Kp, dtype=torch.bfloat16, device=x.device)
-    sums = torch.empty(splits * most * N, dtype=torch.float32, device=x.device) if splits > 1 else None
-    for r in range(0, M, max(most, 1)):
-        some, to = (x, out) if most == M else (x[r:r + most], out[r:r + most])
-        _check(_lib().af_gemm_f32_tc(_ptr(to), c_longlong(_rows(out, "out")), _ptr(some), c_longlong(_rows(x, "x")), _ptr(w),
-                                     c_longlong(_rows(w, "w")), c_int(some.shape[0]), c_int(N), c_int(K), c_float(cap), _ptr(parts),
-                                     _ptr(sums, allow_none=True), _ptr(error_word(x.device), "err", torch.int32), _stream()))
+    part_row, sum_row = 6 * Kp, 4 * splits * N if splits > 1 else 0
+    most = min(M, 65535, max(160, F32_TC_BYTES // (part_row + sum_row) // 160 * 160))         # (160: the rows of a tile)
+    scratch = torch.empty(most * (part_row + sum_row), dtype=torch.uint8, device=x.device)
+    parts = scratch.data_ptr()
+    more = (_ptr(w), c_longlong(_rows(w, "w")))
+    rest = (c_int(N), c_int(K), c_float(cap), c_void_p(parts), c_void_p(parts + most * part_row if sum_row else 0),
+            _ptr(error_word(x.device), "err", torch.int32), _stream())
+    ldo, ldx, run = c_longlong(_rows(out, "out")), c_longlong(_rows(x, "x")), _lib().af_gemm_f32_tc
+    if most == M:
+        _check(run(_ptr(out), ldo, _ptr(x), ldx, *more, c_int(M), *rest))
+        return
+    for r in range(0, M, most):
+        _check(run(_ptr(out[r:]), ldo, _ptr(x[r:]), ldx, *more, c_int(min(most, M - r)), *rest))
 
 
 # ---------------------------------------------------------------- attention
