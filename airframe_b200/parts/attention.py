@@ -34,7 +34,7 @@ from .. import kernels
 from ..config.base import ConfigError, PartSpec
 from ..weights.loader import WeightDecl
 from .base import KVNeed, Mixer, PositionEncoding, build_part, register_part
-from .linear import PartialSums, linear, linear_split
+from .linear import PartialSums, linear, linear_split, of_prompt
 from .rope import Rope
 
 
@@ -247,7 +247,7 @@ class Attention(Mixer):
         """The projection in 32-bit rows; q and k heads normed and rotated, the values taken
         (from the raw key projection, or their own heads), all packed and the cache written: one kernel."""
         nq, nkv, hd = self.nq, self.nkv, self.hd
-        proj = linear(x, self.w_qkv, out_dtype=torch.float32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_qkv, out_dtype=torch.float32, prompt=of_prompt(batch))
         width = (nq + 2 * nkv) * self.pad if self.pad else (nq + nkv) * hd + nkv * self.dv
         qkv = torch.empty(x.shape[0], width, dtype=x.dtype, device=x.device)
         rope = self.position if isinstance(self.position, Rope) else None
@@ -278,7 +278,7 @@ class Attention(Mixer):
         elif self.rope_epilogue:
             qkv = self._project_rotate_store(x, batch, view)
         else:
-            qkv = linear_split(x, self.w_qkv, prompt=batch.is_prefill)
+            qkv = linear_split(x, self.w_qkv, prompt=of_prompt(batch))
             parts = None
             if isinstance(qkv, PartialSums):
                 parts = qkv.parts
@@ -309,4 +309,4 @@ class Attention(Mixer):
                                  keep=self.keep, **more)
         else:
             kernels.attn_decode(ctx, q, kv, batch, nq, nkv, hd, self.scale, self.softcap, window, slopes, **more)
-        return linear_split(ctx, self.w_o, wide=bool(self.params.get("wide_output", False)), prompt=batch.is_prefill)
+        return linear_split(ctx, self.w_o, wide=bool(self.params.get("wide_output", False)), prompt=of_prompt(batch))

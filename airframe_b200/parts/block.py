@@ -29,7 +29,7 @@ from .. import kernels
 from ..config.base import ConfigError, PartSpec
 from ..weights.loader import WeightDecl
 from .base import Block, StateNeed, build_part, register_part
-from .linear import PartialSums, as_terms, linear_split
+from .linear import PartialSums, as_terms, linear_split, of_prompt
 from .norm import LayerNorm
 
 
@@ -222,7 +222,7 @@ class NormedSumBlock(Block):
         if self.gates[which] is None:
             return {}
         w, b = self.gates[which]
-        z = linear_split(y, w, wide=True, prompt=batch.is_prefill)
+        z = linear_split(y, w, wide=True, prompt=of_prompt(batch))
         return {"gate": z.parts if isinstance(z, PartialSums) else z, "gate_bias": b}
 
     def forward(self, x, batch, view, normed=None, next_pre=None):

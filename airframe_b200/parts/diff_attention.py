@@ -28,7 +28,7 @@ from .. import kernels
 from ..config.base import ConfigError
 from ..weights.loader import WeightDecl
 from .base import KVNeed, Mixer, StateNeed, register_part
-from .linear import linear, linear_split
+from .linear import linear, linear_split, of_prompt
 
 
 @register_part("mixer", "diff_attention")
@@ -161,7 +161,7 @@ class DiffAttention(Mixer):
 
     def forward(self, x, batch, view):
         T, H, G, pk, pv = x.shape[0], self.H, self.G, self.pk, self.pv
-        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=of_prompt(batch))
         qkv = torch.empty(T, (2 * H + 2 * G) * pk + 2 * G * pv, dtype=x.dtype, device=x.device)
         kernels.conv_pack(qkv, proj, batch, H, G, self.d, self.dv, pk, pv, bias=self.bias, taps_w=self.taps_w,
                           history=view.state, temp_coef=self.temp_coef, temp_every=self.temp_every,
@@ -184,4 +184,4 @@ class DiffAttention(Mixer):
         gate = proj[:, self.channels: self.channels + H * self.dv] if self.names.get("g") else None
         kernels.diff_join(y, ctx, gate, H, G, self.dv, pv, self.lam, self.eps, 1.0 - self.diff,
                           ones=1 if self.o_in != H * self.dv else 0)
-        return linear_split(y, self.w_o, wide=bool(self.params.get("wide_output", True)), prompt=batch.is_prefill)
+        return linear_split(y, self.w_o, wide=bool(self.params.get("wide_output", True)), prompt=of_prompt(batch))

@@ -15,7 +15,7 @@ import torch
 from .. import kernels
 from ..weights.loader import WeightDecl
 from .base import Junction, register_part
-from .linear import PartialSums, linear_split
+from .linear import PartialSums, linear_split, of_prompt
 from .norm import TanhNorm
 
 
@@ -49,7 +49,7 @@ class Reinject(Junction):
     def forward(self, x, x0, index, batch, then=None, out_dtype=None):
         both = torch.empty(x.shape[0], 2 * self.hidden, dtype=self.ctx.compute_dtype, device=x.device)
         kernels.concat_cast(both, x, x0)
-        z = linear_split(both, self.w, wide=True, prompt=batch.is_prefill)
+        z = linear_split(both, self.w, wide=True, prompt=of_prompt(batch))
         z = z.parts if isinstance(z, PartialSums) else z
         if then is None or not isinstance(then, TanhNorm):
             kernels.set_sum_row(x, z, self.steps[index])

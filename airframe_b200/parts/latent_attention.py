@@ -34,7 +34,7 @@ from .. import kernels
 from ..config.base import ConfigError, PartSpec
 from ..weights.loader import WeightDecl
 from .base import KVNeed, Mixer, build_part, register_part
-from .linear import PartialSums, linear, linear_split
+from .linear import PartialSums, linear, linear_split, of_prompt
 from .rope import Rope
 
 
@@ -189,7 +189,7 @@ class LatentAttention(Mixer):
         written to the cache), the logits of a gate per head and those of a gate per value (column sections, or None)."""
         H, dim, rot, rank = self.heads, self.dim, self.rot, self.rank
         T, dt, dev = x.shape[0], x.dtype, x.device
-        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=of_prompt(batch))
         q = torch.empty(T, H * pitch, dtype=dt, device=dev)
         kvrow = torch.empty(T, rank + rot, dtype=dt, device=dev)
         pos = self.position
@@ -201,7 +201,7 @@ class LatentAttention(Mixer):
             cq = torch.empty(T, self.q_rank, dtype=dt, device=dev)
             kernels.latent_prep(batch, H, dim, rot, rank, self.eps, side=cq, side_src=proj[:, : self.q_rank],
                                 side_w=self.q_norm_w, **kv_part, **turn)
-            up = linear_split(cq, self.w_uq, wide=True, prompt=batch.is_prefill)
+            up = linear_split(cq, self.w_uq, wide=True, prompt=of_prompt(batch))
             q_part["q_src"] = up.parts if isinstance(up, PartialSums) else up
             kernels.latent_prep(batch, H, dim, rot, rank, self.eps, **q_part, **turn)
         else:
@@ -254,4 +254,4 @@ class LatentAttention(Mixer):
         # back from the latent to the heads' values, then the output projection
         ctx = torch.empty(T, H * dv, dtype=dt, device=x.device)
         kernels.head_project(ctx, mix, self.w_uv, H, rank, dv, x_pitch=rank + rot if wide else rank, gate=values)
-        return linear_split(ctx, self.w_o, wide=bool(self.params.get("wide_output", False)), prompt=batch.is_prefill)
+        return linear_split(ctx, self.w_o, wide=bool(self.params.get("wide_output", False)), prompt=of_prompt(batch))

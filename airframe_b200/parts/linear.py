@@ -14,6 +14,11 @@ import torch
 from .. import kernels
 
 
+def of_prompt(batch) -> bool:
+    """Whether a part's rows are a prefill step's (a part called without a batch: no)."""
+    return getattr(batch, "is_prefill", False)
+
+
 def linear(x, w, out_dtype=None, cap: float = 0.0, out=None, prompt: bool = False):
     """x [M, K] (dense rows), w [N, K] -> [M, N] in ``out_dtype`` (x's by default).
     ``cap`` > 0 applies the softcap cap * tanh(y / cap) to the result.  ``prompt``: the

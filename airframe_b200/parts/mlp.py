@@ -42,7 +42,7 @@ from .. import kernels
 from ..config.base import ConfigError
 from ..weights.loader import WeightDecl
 from .base import FeedForward, register_part
-from .linear import PartialSums, WeightedSum, gated_linear, linear_split
+from .linear import PartialSums, WeightedSum, gated_linear, linear_split, of_prompt
 
 
 @register_part("feed_forward", "gated_mlp")
@@ -90,8 +90,8 @@ class GatedMlp(FeedForward):
         return 2 * sum(lens) * 3 * self.hidden * self.inter
 
     def forward(self, x, batch):
-        h = gated_linear(x, self.w_gu, self.inter, self.activation, self.interleaved, prompt=batch.is_prefill)
-        return linear_split(h, self.w_down, wide=bool(self.params.get("wide_output", False)), prompt=batch.is_prefill)
+        h = gated_linear(x, self.w_gu, self.inter, self.activation, self.interleaved, prompt=of_prompt(batch))
+        return linear_split(h, self.w_down, wide=bool(self.params.get("wide_output", False)), prompt=of_prompt(batch))
 
 
 @register_part("feed_forward", "none")
@@ -144,11 +144,11 @@ class TokenSide(FeedForward):
         return 4 * sum(lens) * self.hidden * self.dim
 
     def forward(self, x, batch):
-        z = linear_split(x, self.w_gate, wide=True, prompt=batch.is_prefill)
+        z = linear_split(x, self.w_gate, wide=True, prompt=of_prompt(batch))
         g = torch.empty(x.shape[0], self.dim, dtype=x.dtype, device=x.device)
         kernels.token_gate(g, z.parts if isinstance(z, PartialSums) else z, self.table, self.index * self.dim, batch.tokens,
                            self.activation)
-        return linear_split(g, self.w_proj, wide=True, prompt=batch.is_prefill)
+        return linear_split(g, self.w_proj, wide=True, prompt=of_prompt(batch))
 
 
 @register_part("feed_forward", "routed_experts")

@@ -52,7 +52,7 @@ from .. import kernels
 from ..config.base import ConfigError
 from ..weights.loader import WeightDecl
 from .base import Mixer, StateNeed, build_part, register_part
-from .linear import linear, linear_split
+from .linear import linear, linear_split, of_prompt
 from .rope import Rope
 
 
@@ -173,7 +173,7 @@ class GeneralDelta(_StateMixer):
 
     def forward(self, x, batch, view):
         T, n, off = x.shape[0], self.n, self.off
-        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=of_prompt(batch))
         r, k, v = (proj[:, off[c]: off[c] + n] for c in ("r", "k", "v"))
         o = torch.empty(T, n, dtype=torch.float32, device=x.device)
         if _in_chunks(x, batch, self.hd, self.hd, self.rank):
@@ -189,7 +189,7 @@ class GeneralDelta(_StateMixer):
                                w=pre[:, 0], u=pre[:, 1], au=pre[:, 2])
         y = torch.empty(T, n, dtype=x.dtype, device=x.device)
         kernels.gated_group_norm(y, o, self.norm_w, proj[:, off["g"]: off["g"] + n], self.hd, self.eps)
-        return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+        return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
 
 
 @register_part("mixer", "lightning_attention")
@@ -238,14 +238,14 @@ class LightningAttention(_StateMixer):
     def forward(self, x, batch, view):
         T, off = x.shape[0], self.off
         nk, nv = self.heads * self.dk, self.heads * self.dv
-        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=of_prompt(batch))
         o = torch.empty(T, nv, dtype=torch.float32, device=x.device)
         scan = kernels.state_chunks if _in_chunks(x, batch, self.dk, self.dv) else kernels.state_scan
         scan("decay", o, proj[:, off["q"]: off["q"] + nk], proj[:, off["k"]: off["k"] + nk],
              proj[:, off["v"]: off["v"] + nv], view.state, batch, self.heads, self.dk, self.dv, decay=self.decay, silu=True)
         y = torch.empty(T, nv, dtype=x.dtype, device=x.device)
         kernels.gated_group_norm(y, o, self.norm_w, proj[:, off["g"]: off["g"] + nv], nv, self.eps)
-        return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+        return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
 
 
 @register_part("mixer", "retention")
@@ -302,7 +302,7 @@ class Retention(_StateMixer):
     def forward(self, x, batch, view):
         T, off, pos, H, dk, dv = x.shape[0], self.off, self.position, self.heads, self.dk, self.dv
         nk, nv = H * dk, H * dv
-        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=of_prompt(batch))
         q, k, v, g = (proj[:, off[n]: off[n] + w] for n, w in (("q", nk), ("k", nk), ("v", nv), ("g", nv)))
         table = pos.step_table(batch) if pos.rotary_dim else None
         turn = {"pairing": pos.pairing, "magnitude": pos.magnitude}
@@ -310,7 +310,7 @@ class Retention(_StateMixer):
         if T == batch.n_seqs:            # single tokens: rotation, state, norm and gate in one kernel
             kernels.retention_step(y, q, k, v, g, table, self.decay, view.state, batch, H, dk, dv, self.key_scale, self.eps,
                                    gate_act=self.gate, **turn)
-            return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+            return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
         scale = self.key_scale
         if self._on_tensor_cores(x, batch):
             fused = dv <= 128            # (a head's values in one block: its norm and gate there too)
@@ -318,7 +318,7 @@ class Retention(_StateMixer):
             kernels.retention_prompt(o, q, k, v, g if fused else None, table, self._powers(), view.state, batch, H, dk, dv,
                                      scale, self.eps, gate_act=self.gate, **turn)
             if fused:
-                return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+                return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
             scale = 1.0
         else:                            # token after token, in 32 bits
             if table is not None:
@@ -326,7 +326,7 @@ class Retention(_StateMixer):
             o = torch.empty(T, nv, dtype=torch.float32, device=x.device)
             kernels.state_scan("decay", o, q, k, v, view.state, batch, H, dk, dv, decay=self.decay)
         kernels.gated_group_norm(y, o, None, g, dv, self.eps, gate_act=self.gate, in_scale=scale)
-        return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+        return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
 
     def _on_tensor_cores(self, x, batch) -> bool:
         """A bfloat16 prompt whose tokens fill a tile, cut into chunks on the tensor cores."""
@@ -375,10 +375,10 @@ class MinGru(_StateMixer):
 
     def forward(self, x, batch, view):
         off = self.off
-        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=torch.float32, prompt=of_prompt(batch))
         y = torch.empty(x.shape[0], self.width, dtype=x.dtype, device=x.device)
         kernels.gated_scan(y, proj, off["z"], off["x"], off["g"], self.z_bias, self.x_bias, view.state, batch)
-        return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+        return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
 
 
 @register_part("mixer", "rglru")
@@ -440,7 +440,7 @@ class RgLru(_StateMixer):
 
     def forward(self, x, batch, view):
         T, w, off, f32 = x.shape[0], self.width, self.off, torch.float32
-        proj = linear(x, self.w_in, out_dtype=f32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=f32, prompt=of_prompt(batch))
         u = torch.empty(T, w, dtype=f32, device=x.device)
         # many rows in bfloat16: the gates' block-diagonal products on the tensor cores, from u rounded as
         # every product's input is; few rows (a decode step) or 32-bit: on the CUDA cores from u itself
@@ -455,7 +455,7 @@ class RgLru(_StateMixer):
             kernels.gate_rows(decay, inp, u, self.w_a, self.w_i, self.a_bias, self.i_bias, self.rate)
         y = torch.empty(T, w, dtype=x.dtype, device=x.device)
         kernels.decay_scan(y, decay, inp, proj, off["y"], off["x"], self.y_bias, self.x_bias, view.state, batch)
-        return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+        return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
 
 
 @register_part("mixer", "gated_linear_attention")
@@ -543,7 +543,7 @@ class GatedLinearAttention(_StateMixer):
     def forward(self, x, batch, view):
         T, off, f32 = x.shape[0], self.off, torch.float32
         nk, nv = self.heads * self.dk, self.heads * self.dv
-        proj = linear(x, self.w_in, out_dtype=f32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=f32, prompt=of_prompt(batch))
         alpha = torch.empty(T, nk, dtype=f32, device=x.device)
         kernels.channel_decay(alpha, proj, off["a1"], self.w2t, self.a2_bias, self.tau)
         o = torch.empty(T, nv, dtype=f32, device=x.device)
@@ -558,7 +558,7 @@ class GatedLinearAttention(_StateMixer):
         y = torch.empty(T, nv, dtype=x.dtype, device=x.device)
         kernels.gated_group_norm(y, o, self.norm_w, proj[:, off["g"]: off["g"] + nv], self.dv, self.eps,
                                  gate_act=self.gate, in_scale=self.query_scale)
-        return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+        return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
 
 
 @register_part("mixer", "channel_delta")
@@ -637,7 +637,7 @@ class ChannelDelta(_StateMixer):
     def forward(self, x, batch, view):
         T, off, f32, nk, nv, H = x.shape[0], self.off, torch.float32, self.nk, self.nv, self.heads
         state, history = view.state if self.taps > 1 else (view.state[0], None)
-        proj = linear(x, self.w_in, out_dtype=f32, prompt=batch.is_prefill)
+        proj = linear(x, self.w_in, out_dtype=f32, prompt=of_prompt(batch))
         # [q | k | v | beta], rows of whole 16-byte pieces
         mixed = torch.empty(T, (self.channels + H + 3) // 4 * 4, dtype=f32, device=x.device)[:, : self.channels + H]
         q, k, v = mixed[:, :nk], mixed[:, nk: 2 * nk], mixed[:, 2 * nk: self.channels]
@@ -674,7 +674,7 @@ class ChannelDelta(_StateMixer):
             kernels.state_scan("gated", o, q, k, v, state, batch, H, self.dk, self.dv, w=decay, beta=beta)
         y = torch.empty(T, nv, dtype=x.dtype, device=x.device)
         kernels.gated_group_norm(y, o, self.norm_w, gate, self.dv, self.eps)
-        return linear_split(y, self.w_o, wide=self.wide, prompt=batch.is_prefill)
+        return linear_split(y, self.w_o, wide=self.wide, prompt=of_prompt(batch))
 
     LOW_TC_ROWS = 64           # from so many rows on the low-rank second products go to the tensor cores
     CHUNKED_FROM = 64          # tokens of the longest prompt of a step that is cut into chunks on the tensor cores
