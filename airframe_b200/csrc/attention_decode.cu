@@ -10,9 +10,9 @@
 //  * the even cut: every unit into about pages / share splits of equal size, one split a block.  No block
 //    meets the end of a unit; taken when the splits are no more than the blocks and none is more than two
 //    pages above the share (sequences of equal or of mixed lengths, one long one among short ones);
-//  * else the run cut: all units' pages end to end, each block an equal run of them.  A run may end one unit
-//    and begin the next: the block works them as segments, one after the other, and leaves a partial result
-//    for each (many short sequences; more units than blocks).
+//  * else the run cut: all units' pages end to end, each block an equal run of them, in which every unit counts
+//    DA_BREAK_PAGES more than its pages.  A run may end one unit and begin the next: the block works them as
+//    segments, one after the other, and leaves a partial result for each (many short sequences; more units than blocks).
 // Pass 1: a block of two groups of 4 warps
 // walks its pages, the groups taking alternate
 // pages (one warp per scheduler cannot hide the latency of its own chain of
@@ -158,30 +158,34 @@ __device__ __forceinline__ int da_even_splits(int P, int share, int room, int ho
 }
 
 // What a block loses at the end of a unit inside its run (merging, the next unit's queries, the first page's
-// wait), in pages: the even cut is taken if its largest split is no more than this above the share.
+// wait), in pages: the even cut is taken if its largest split is no more than this above the share, and in the run cut a unit
+// of P pages takes P + DA_BREAK_PAGES of a run, the break first.  (Runs of equal pages left the blocks that met
+// many short sequences behind.  64 sequences of 10 to 2,048 tokens, 256 units of which 88 have one page: a decode step of 26 layers
+// 2,412 -> 2,267 us.)
 constexpr int DA_BREAK_PAGES = 2;
 
 struct DaPlan {
-  int share;        // pages a block should get
+  int share;        // pages a block should get (the run cut: with the units' breaks)
   int n_blocks;     // blocks that work in the run cut
   int even;         // 0: the run cut; else the even cut, and how it rounds (da_even_splits)
-  int pages_before; // pages of the sequences before `b_query` (each counted once, not per unit)
+  int pages_before; // pages of the sequences before `b_query` (each counted once, not per unit; the run cut: with breaks)
 };
 
 // The plan, by one whole warp (every lane returns the same).  32-bit arithmetic all through: the launcher has
-// checked that batch x pages x units stays below 2^31.  If `pages_s` is given it gets the pages of the sequences
-// before b, and `splits_s` their splits in the even cut (b = 0 .. batch).
+// checked that batch x (pages + break) x units stays below 2^31.  If `pages_s` is given it gets the pages of the sequences
+// before b (the run cut: with a break for each that has any), and `splits_s` their splits in the even cut (b = 0 .. batch).
 __device__ __forceinline__ DaPlan da_plan(const int* slots, const int* lens, int batch, int window, int keep, int units_per_seq,
                                           int grid_blocks, int room, int b_query, int* pages_s, int* splits_s) {
   const int lane = threadIdx.x & 31;
-  int carry = 0, most = 0, before = 0, P_first = 0;
+  int carry = 0, most = 0, before = 0, P_first = 0, live = 0, live_before = 0;
   if (pages_s && lane == 0) pages_s[0] = 0;
   for (int base = 0; base < batch; base += 32) {
     const int i = base + lane;
     const int P = i < batch ? da_pages(slots, lens, i, window, keep) : 0;
     if (base == 0) P_first = P;
     most = max(most, P);
-    if (i < b_query) before += P;
+    if (i < b_query) before += P, live_before += P > 0 ? 1 : 0;
+    live += P > 0 ? 1 : 0;
     int v = P;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -219,6 +223,21 @@ __device__ __forceinline__ DaPlan da_plan(const int* slots, const int* lens, int
   if (fits1 && (!fits2 || worst1 <= worst2)) how = 1, worst = worst1;
   else if (fits2) how = 2, worst = worst2;
   pl.even = (how != 0 && worst <= pl.share + DA_BREAK_PAGES) ? how : 0;
+  if (!pl.even) {
+    live = __reduce_add_sync(0xffffffffu, live);
+    pl.pages_before += DA_BREAK_PAGES * __reduce_add_sync(0xffffffffu, live_before);
+    pl.share = max(1, ((carry + DA_BREAK_PAGES * live) * units_per_seq + pl.n_blocks - 1) / pl.n_blocks);
+    if (pages_s) {
+      int breaks = 0;
+      for (int base = 0; base < batch; base += 32) {
+        const int i = base + lane;
+        const int P = base == 0 ? P_first : (i < batch ? da_pages(slots, lens, i, window, keep) : 0);
+        const uint32_t with = __ballot_sync(0xffffffffu, P > 0);
+        if (i < batch) pages_s[i + 1] += DA_BREAK_PAGES * (breaks + __popc(with & (0xffffffffu >> (31 - lane))));
+        breaks += __popc(with);
+      }
+    }
+  }
   if (splits_s && pl.even) {
     int items = 0;
     if (lane == 0) splits_s[0] = 0;
@@ -248,17 +267,18 @@ __device__ __forceinline__ int da_find(const int* arr, int n, int scale, int x) 
   return lo;
 }
 
-// What block w begins with: pages [p_in, p_in + n_pages) of unit y of sequence b, the unit's split z; run_pages is
-// all the block works (in the run cut it goes on with the units that follow).  n_pages < 0: the block has no work.
+// What block w begins with: pages [p_in, p_in + n_pages) of unit y of sequence b, the unit's split z; run_left is what
+// its run holds behind that unit, pages and breaks (in the run cut it goes on with the units that follow).  n_pages < 0: the
+// block has no work.
 struct DaFirst {
-  int n_pages, b, y, z, p_in, run_pages;
+  int n_pages, b, y, z, p_in, run_left;
 };
 
 __device__ __forceinline__ DaFirst da_first_segment(const DaPlan& pl, const int* pages_s, const int* splits_s, int batch,
                                                     int units_per_seq, int w) {
   DaFirst fs;
   fs.n_pages = -1;
-  fs.b = fs.y = fs.z = fs.p_in = fs.run_pages = 0;
+  fs.b = fs.y = fs.z = fs.p_in = fs.run_left = 0;
   if (pl.even) {
     // split z of unit y of sequence b, one of da_even_splits(...) equal parts of its pages
     if (w >= splits_s[batch] * units_per_seq) return fs;
@@ -271,23 +291,29 @@ __device__ __forceinline__ DaFirst da_first_segment(const DaPlan& pl, const int*
     fs.z = r - fs.y * sp;
     fs.p_in = fs.z * per;
     fs.n_pages = max(0, min(per, P - fs.p_in));   // (0: the unit has fewer pages than splits; an empty partial result)
-    fs.run_pages = fs.n_pages;
     return fs;
   }
-  // the run cut: pages [gpos, gend) of all units' pages end to end
+  // the run cut: [gpos, gend) of all units end to end, a unit's break and then its pages
   const int total = pages_s[batch] * units_per_seq;
   const int gpos = w * pl.share, gend = min(total, gpos + pl.share);
   if (w >= pl.n_blocks || gpos >= gend) return fs;
   const int b = da_find(pages_s, batch, units_per_seq, gpos);
-  const int P = pages_s[b + 1] - pages_s[b];
-  const int seq0 = pages_s[b] * units_per_seq;
+  const int width = pages_s[b + 1] - pages_s[b];
+  const int y = (gpos - pages_s[b] * units_per_seq) / width;
+  const int unit0 = pages_s[b] * units_per_seq + y * width, page0 = unit0 + DA_BREAK_PAGES;
+  const int p_in = max(0, gpos - page0), n_pages = min(width - DA_BREAK_PAGES, gend - page0) - p_in;
+  if (n_pages <= 0) return fs;                // (the run lies in a break)
   fs.b = b;
-  fs.y = (gpos - seq0) / P;
-  fs.p_in = (gpos - seq0) - fs.y * P;
-  fs.run_pages = gend - gpos;
-  fs.n_pages = min(P - fs.p_in, fs.run_pages);
-  fs.z = w - (seq0 + fs.y * P) / pl.share;   // (the run may begin inside a unit: then it is not the unit's first split)
+  fs.y = y;
+  fs.p_in = p_in;
+  fs.n_pages = n_pages;
+  fs.run_left = max(0, gend - unit0 - width);
+  fs.z = w - page0 / pl.share;                // (the run may begin inside a unit: then it is not the unit's first split)
   return fs;
+}
+// The runs that hold pages of a unit whose break begins at unit0.
+__device__ __forceinline__ int da_run_splits(int unit0, int P, int share) {
+  return P > 0 ? (unit0 + DA_BREAK_PAGES + P - 1) / share - (unit0 + DA_BREAK_PAGES) / share + 1 : 0;
 }
 
 // ---------------------------------------------------------------- the plan of a step
@@ -298,7 +324,7 @@ __device__ __forceinline__ DaFirst da_first_segment(const DaPlan& pl, const int*
 // one after the other, before its first copy can start.  The plan, 32-bit integers:
 //   [0, 8)                    room (splits a unit may have), grid blocks, sequences, units a sequence, how cut
 //   [8, 8 + sequences*units)  the splits of every unit, for the merge
-//   then 16 a block           n_pages (< 0: no work), b, y, z, p_in, run_pages, position of the new token, slot,
+//   then 16 a block           n_pages (< 0: no work), b, y, z, p_in, run_left, position of the new token, slot,
 //                             the cache pages of the segment's first four pages
 constexpr int DA_PLAN_HEAD = 8;
 constexpr int DA_PLAN_REC = 16;
@@ -337,15 +363,9 @@ attn_decode_plan_kernel(int* __restrict__ plan, const int* __restrict__ slots, c
   }
   for (int u = threadIdx.x; u < batch * units_per_seq; u += blockDim.x) {
     const int b = u / units_per_seq, y = u - b * units_per_seq;
-    const int P = pages_s[b + 1] - pages_s[b];
-    int n = 0;
-    if (pl.even) {
-      n = da_even_splits(P, pl.share, room, pl.even);
-    } else if (P > 0) {
-      const int unit0 = pages_s[b] * units_per_seq + y * P;
-      n = (unit0 + P - 1) / pl.share - unit0 / pl.share + 1;
-    }
-    plan[DA_PLAN_HEAD + u] = n;
+    const int width = pages_s[b + 1] - pages_s[b];      // (the run cut: with a break)
+    plan[DA_PLAN_HEAD + u] = pl.even ? da_even_splits(width, pl.share, room, pl.even)
+                                     : da_run_splits(pages_s[b] * units_per_seq + y * width, width - DA_BREAK_PAGES, pl.share);
   }
   int* recs = plan + da_plan_records_at(batch, units_per_seq);
   for (int w = threadIdx.x; w < grid_blocks; w += blockDim.x) {
@@ -364,7 +384,7 @@ attn_decode_plan_kernel(int* __restrict__ plan, const int* __restrict__ slots, c
       }
     }
     reinterpret_cast<int4*>(r)[0] = make_int4(fs.n_pages, fs.b, fs.y, fs.z);
-    reinterpret_cast<int4*>(r)[1] = make_int4(fs.p_in, fs.run_pages, pos, slot);
+    reinterpret_cast<int4*>(r)[1] = make_int4(fs.p_in, fs.run_left, pos, slot);
     reinterpret_cast<int4*>(r)[2] = make_int4(ids[0], ids[1], ids[2], ids[3]);
     reinterpret_cast<int4*>(r)[3] = make_int4(0, 0, 0, 0);
   }
@@ -417,7 +437,7 @@ attn_decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     const int4 head = ld_keep_int4(reinterpret_cast<const int4*>(a.plan), keep);
     const int4 r0 = ld_keep_int4(rec, keep), r1 = ld_keep_int4(rec + 1, keep), r2 = ld_keep_int4(rec + 2, keep);
     fs.n_pages = r0.x, fs.b = r0.y, fs.y = r0.z, fs.z = r0.w;
-    fs.p_in = r1.x, fs.run_pages = r1.y, pos0 = r1.z, slot0 = r1.w;
+    fs.p_in = r1.x, fs.run_left = r1.y, pos0 = r1.z, slot0 = r1.w;
     ids0[0] = r2.x, ids0[1] = r2.y, ids0[2] = r2.z, ids0[3] = r2.w;
     if (head.x != a.n_splits || head.y != (int)gridDim.x || head.z != a.batch || head.w != units_per_seq) {
       // (a plan made for another launch: nothing is read or written by it)
@@ -439,7 +459,7 @@ attn_decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     }
   }
   if (fs.n_pages < 0) return;                          // (nothing of the block's is in flight yet)
-  int left = fs.run_pages;                             // pages the block has still to work
+  int left = fs.run_left;                              // what the block's run holds behind the segment's unit
   const float cs = a.cap > 0.f ? a.scale / a.cap : a.scale * LOG2E;
   const float cap2 = a.cap * LOG2E;
 
@@ -473,7 +493,8 @@ attn_decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     }
     const int P = da_pages(a.slots, a.lens, b, a.window, a.keep);
     nx.z = 0;
-    nx.n_pages = min(P, left);
+    nx.n_pages = min(P, left - DA_BREAK_PAGES);
+    left -= DA_BREAK_PAGES + P;
     of_unit(nx, b, y, 0, a.lens[b] - 1, a.slots[b]);
     return nx;
   };
@@ -679,8 +700,7 @@ attn_decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     // stage (up to 8 heads in the tile), the next segment's first pages go into the other stages before the
     // merge, so that the block's stream of pages does not stop at a unit's end.
     i_base += n_pages;
-    left -= n_pages;
-    const bool more = left > 0 && !gave_up;          // (the even cut: one segment)
+    const bool more = left > DA_BREAK_PAGES && !gave_up;          // (the even cut: one segment)
     Segment nx = sg;
     issued = 0;
     if (more) {
@@ -777,8 +797,7 @@ __global__ void attn_decode_merge_kernel(__nv_bfloat16* __restrict__ out, long l
       n_splits = da_even_splits(P, plan_s.share, max_splits, plan_s.even);
     } else {
       const int y = (h / group) * tiles + (h % group) / 16;
-      const int unit0 = plan_s.pages_before * units_per_seq + y * P;
-      n_splits = P > 0 ? (unit0 + P - 1) / plan_s.share - unit0 / plan_s.share + 1 : 0;
+      n_splits = da_run_splits(plan_s.pages_before * units_per_seq + y * (P + DA_BREAK_PAGES), P, plan_s.share);
     }
   }
   pdl_wait();
@@ -924,7 +943,7 @@ int launch_decode(DecodeArgs a, int batch, long long n_pages, cudaStream_t strea
   const int group = a.nq / a.nkv;
   const int units_per_seq = a.nkv * ((group + 15) / 16);
   // (a sequence attends to at most max_pages + 1 pages: a window's first and last page may be the same of the ring)
-  AF_REQUIRE(batch <= DA_MAX_BATCH && (long long)batch * (a.max_pages + 1) * units_per_seq < (1ll << 31),
+  AF_REQUIRE(batch <= DA_MAX_BATCH && (long long)batch * (a.max_pages + 1 + DA_BREAK_PAGES) * units_per_seq < (1ll << 31),
              "af_attn_decode: %d sequences of up to %d pages (takes %d sequences)", batch, a.max_pages, DA_MAX_BATCH);
   const int n_blocks = a.n_sms;   // one block an SM; the blocks work out among themselves which of them work
   af_launch(attn_decode_split_kernel<HD>, dim3(n_blocks), dim3(DA_THREADS), smem, stream, mk, mv, a);
@@ -1056,7 +1075,7 @@ AF_EXPORT int af_attn_decode_plan_kept(int* plan, long long plan_ints, const int
   AF_REQUIRE(keep >= 0 && (keep == 0 || window != 0), "af_attn_decode_plan: %d kept tokens with window %d", keep, window);
   AF_REQUIRE(n_splits >= 1 && ring_rows % AF_PAGE == 0, "af_attn_decode_plan: splits %d, ring rows %d", n_splits, ring_rows);
   const int units_per_seq = nkv * ((nq / nkv + 15) / 16);
-  AF_REQUIRE(batch <= DA_MAX_BATCH && (long long)batch * (max_pages + 1) * units_per_seq < (1ll << 31),
+  AF_REQUIRE(batch <= DA_MAX_BATCH && (long long)batch * (max_pages + 1 + DA_BREAK_PAGES) * units_per_seq < (1ll << 31),
              "af_attn_decode_plan: %d sequences of up to %d pages (takes %d sequences)", batch, max_pages, DA_MAX_BATCH);
   const int sms = af_sm_count();
   if (sms <= 0) return -1;
