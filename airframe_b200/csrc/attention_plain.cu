@@ -1351,17 +1351,26 @@ head_project_kernel(T* __restrict__ out, long long out_stride, const T* __restri
 // The same for the few rows of a decode step: a block takes 32 outputs of a head for eight tokens at once, so a
 // weight is read once for all of them; its 256 threads are 8 groups that each take a stretch of the inputs
 // (short chains side by side), joined in group order through shared memory.  Grid (head, 32 outputs, 8 tokens).
+// The first AF_HPF_AHEAD weights of a thread, which are cold, are asked for before the wait for the kernel in front: in
+// memory order behind it, a few at a time, they were most of the kernel's time (9 us at eight tokens, 18 heads).
+#define AF_HPF_AHEAD 32
 template <typename T>
 __global__ void __launch_bounds__(256)
 head_project_few_kernel(T* __restrict__ out, long long out_stride, const T* __restrict__ x, long long x_stride,
                         const T* __restrict__ w, int D, int N, int extra, int x_pitch, int n_tokens,
                         const float* __restrict__ gate, long long gate_stride) {
   pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ float xs[];                     // [8 tokens][D] inputs, then [8 groups][8 tokens][32] partial sums
   float* red = xs + 8 * D;
   const int h = blockIdx.x, n = blockIdx.y * 32 + (threadIdx.x & 31), t0 = blockIdx.z * 8;
   const int grp = threadIdx.x >> 5;
+  const int per = (D + 7) / 8, d0 = grp * per, d1 = min(D, d0 + per);
+  const T* wh = w + (size_t)h * D * N + (n < N ? n : 0);
+  T ahead[AF_HPF_AHEAD];
+#pragma unroll
+  for (int i = 0; i < AF_HPF_AHEAD; ++i) ahead[i] = d0 + i < d1 ? wh[(size_t)(d0 + i) * N] : from_f32<T>(0.f);
+  pdl_wait();
+  x = pdl_fresh(x);
   for (int i = threadIdx.x; i < 8 * D; i += blockDim.x) {
     const int u = i / D, d = i - u * D;
     xs[i] = t0 + u < n_tokens ? to_f32(x[(size_t)(t0 + u) * x_stride + (size_t)h * x_pitch + d]) : 0.f;
@@ -1373,12 +1382,17 @@ head_project_few_kernel(T* __restrict__ out, long long out_stride, const T* __re
         out[(size_t)(t0 + u) * out_stride + (size_t)h * (N + extra) + N + e] = x[(size_t)(t0 + u) * x_stride + (size_t)h * x_pitch + D + e];
     }
   __syncthreads();
-  const int per = (D + 7) / 8, d0 = grp * per, d1 = min(D, d0 + per);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < AF_HPF_AHEAD; ++i) {
+    if (d0 + i >= d1) break;
+    const float wv = to_f32(ahead[i]);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc[u] += xs[u * D + d0 + i] * wv;
+  }
   if (n < N) {
-    const T* wh = w + (size_t)h * D * N + n;
 #pragma unroll 4
-    for (int d = d0; d < d1; ++d) {
+    for (int d = d0 + AF_HPF_AHEAD; d < d1; ++d) {
       const float wv = to_f32(wh[(size_t)d * N]);
 #pragma unroll
       for (int u = 0; u < 8; ++u) acc[u] += xs[u * D + d] * wv;

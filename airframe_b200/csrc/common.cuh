@@ -203,22 +203,33 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// Sum over a block of up to 1024 threads; every thread gets the result.
-// `scratch` holds 33 floats of shared memory.
+// Sum over a block of up to 1024 threads; every thread gets the result.  `scratch` holds 32 floats of shared memory; every
+// warp adds the warps' sums up for itself (a second trip through shared memory and a third barrier cost 60 cycles).  FRESH:
+// nobody has read `scratch` before.
+template <bool FRESH = false>
 __device__ __forceinline__ float block_sum(float v, float* scratch) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarp = (blockDim.x + 31) >> 5;
   v = warp_sum(v);
-  __syncthreads();
+  if (!FRESH) __syncthreads();
   if (lane == 0) scratch[warp] = v;
   __syncthreads();
-  if (warp == 0) {
-    float t = lane < nwarp ? scratch[lane] : 0.f;
-    t = warp_sum(t);
-    if (lane == 0) scratch[32] = t;
+  return warp_sum(lane < nwarp ? scratch[lane] : 0.f);
+}
+
+// Four neighbours of n rows `stride` floats apart, added in index order: IN loads in flight.
+template <int IN>
+__device__ __forceinline__ float4 sum_parts4(const float* p, int n, size_t stride) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int p0 = 0; p0 < n; p0 += IN) {
+    float4 t[IN];
+#pragma unroll
+    for (int u = 0; u < IN; ++u)
+      t[u] = p0 + u < n ? *reinterpret_cast<const float4*>(p + (size_t)(p0 + u) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < IN; ++u) v.x += t[u].x, v.y += t[u].y, v.z += t[u].z, v.w += t[u].w;
   }
-  __syncthreads();
-  return scratch[32];
+  return v;
 }
 
 // cap * tanh(x / cap) for cap > 0, x otherwise (exact tanhf).

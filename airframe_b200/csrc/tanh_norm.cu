@@ -45,8 +45,8 @@ AF_EXPORT int af_tanh_norm(void* y, int y_dtype, const float* x, const float* w,
 }
 
 // x += tanh_norm_post(a); then, when y is given, y = tanh_norm_next(x).  `a` may come as `n_parts`
-// partial sums (float, [n_parts, rows, hidden]).  Four elements a thread where hidden % 4 == 0.
-template <typename TA, typename TY, int V>
+// partial sums (float, [n_parts, rows, hidden]).
+template <typename TA, typename TY>
 __global__ void __launch_bounds__(256)
 add_tanh_norm_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_parts, size_t part_stride,
                      const float* __restrict__ w_post, const float* __restrict__ b_post, float alpha_post,
@@ -54,24 +54,54 @@ add_tanh_norm_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_part
                      float alpha_next, int hidden, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
-  const size_t at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
+  const size_t at = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (at >= total) return;
   const int i = (int)(at % hidden);
-  float xv[V];
-  if (V == 4) {
-    const float4 t = *reinterpret_cast<const float4*>(x + at);
-    xv[0] = t.x, xv[1] = t.y, xv[2] = t.z, xv[3 % V] = t.w;
+  const float v = x[at] + tanh_norm_f32(summed(a, n_parts, part_stride, at), alpha_post, w_post[i], b_post[i]);
+  x[at] = v;
+  if (y != nullptr) y[at] = from_f32<TY>(tanh_norm_f32(v, alpha_next, w_next[i], b_next[i]));
+}
+
+// Four elements a thread (rows and weights of whole 16-byte pieces).  A decode step's few rows wait for latencies: the
+// weights are asked for before the wait, every load behind it at once, in narrow blocks on many SMs (with the products of heads below, a step of eight
+// sequences through ten runs of Banitar 880 -> 833 us).
+template <typename TA, typename TY>
+__global__ void __launch_bounds__(256)
+add_tanh_norm4_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_parts, size_t part_stride,
+                      const float* __restrict__ w_post, const float* __restrict__ b_post, float alpha_post,
+                      TY* __restrict__ y, const float* __restrict__ w_next, const float* __restrict__ b_next,
+                      float alpha_next, int hidden, size_t total) {
+  pdl_launch_dependents();
+  const size_t at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (at >= total) return;
+  const int i = (int)(at % hidden);
+  auto get4 = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
+  const float4 wp = get4(w_post + i), bp = get4(b_post + i);
+  float4 wn = wp, bn = bp;
+  if (y != nullptr) wn = get4(w_next + i), bn = get4(b_next + i);
+  pdl_wait();
+  x = pdl_fresh(x);
+  a = pdl_fresh(a);
+  float4 v = get4(x + at), t;
+  if constexpr (sizeof(TA) == 4) {
+    t = sum_parts4<16>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
   } else {
-    xv[0] = x[at];
+    const uint2 raw = *reinterpret_cast<const uint2*>(a + at);
+    t = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                    __uint_as_float(raw.y & 0xffff0000u));
   }
-#pragma unroll
-  for (int u = 0; u < V; ++u)
-    xv[u] += tanh_norm_f32(summed(a, n_parts, part_stride, at + u), alpha_post, w_post[i + u], b_post[i + u]);
-  if (V == 4) *reinterpret_cast<float4*>(x + at) = make_float4(xv[0], xv[1 % V], xv[2 % V], xv[3 % V]);
-  else x[at] = xv[0];
+  v.x += tanh_norm_f32(t.x, alpha_post, wp.x, bp.x), v.y += tanh_norm_f32(t.y, alpha_post, wp.y, bp.y);
+  v.z += tanh_norm_f32(t.z, alpha_post, wp.z, bp.z), v.w += tanh_norm_f32(t.w, alpha_post, wp.w, bp.w);
+  *reinterpret_cast<float4*>(x + at) = v;
   if (y == nullptr) return;
-#pragma unroll
-  for (int u = 0; u < V; ++u) y[at + u] = from_f32<TY>(tanh_norm_f32(xv[u], alpha_next, w_next[i + u], b_next[i + u]));
+  const float o[4] = {tanh_norm_f32(v.x, alpha_next, wn.x, bn.x), tanh_norm_f32(v.y, alpha_next, wn.y, bn.y),
+                      tanh_norm_f32(v.z, alpha_next, wn.z, bn.z), tanh_norm_f32(v.w, alpha_next, wn.w, bn.w)};
+  if constexpr (sizeof(TY) == 4) {
+    *reinterpret_cast<float4*>(y + at) = make_float4(o[0], o[1], o[2], o[3]);
+  } else {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+    *reinterpret_cast<uint2*>(y + at) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  }
 }
 
 AF_EXPORT int af_add_tanh_norm(float* x, const void* a, int a_dtype, int n_parts, long long part_stride,
@@ -83,14 +113,16 @@ AF_EXPORT int af_add_tanh_norm(float* x, const void* a, int a_dtype, int n_parts
   AF_REQUIRE(a_dtype == AF_F32 || n_parts == 1, "af_add_tanh_norm: partial sums are float");
   AF_REQUIRE(y == nullptr || (w_next != nullptr && b_next != nullptr), "af_add_tanh_norm: a norm needs its weights");
   const size_t total = (size_t)n_rows * hidden;
-  const bool vec = hidden % 4 == 0 && ((uintptr_t)x & 15) == 0;
+  const bool vec = hidden % 4 == 0 && part_stride % 4 == 0 &&
+                   (((uintptr_t)x | (uintptr_t)a | (uintptr_t)y | (uintptr_t)w_post | (uintptr_t)b_post | (uintptr_t)w_next | (uintptr_t)b_next) & 15) == 0;
   const size_t threads = vec ? total / 4 : total;
-  const size_t blocks = (threads + 255) / 256;
+  const unsigned block = threads <= 64 * 1024 ? 64 : 256;
+  const size_t blocks = (threads + block - 1) / block;
   AF_REQUIRE(blocks < (1ull << 31), "af_add_tanh_norm: too many rows");
-#define AF_ATN(TA, TY, V)                                                                                            \
-  af_launch(add_tanh_norm_kernel<TA, TY, V>, dim3((unsigned)blocks), dim3(256), 0, stream, x, (const TA*)a, n_parts, \
+#define AF_ATN(KERNEL, TA, TY)                                                                                \
+  af_launch(KERNEL<TA, TY>, dim3((unsigned)blocks), dim3(block), 0, stream, x, (const TA*)a, n_parts,         \
             (size_t)part_stride, w_post, b_post, alpha_post, (TY*)y, w_next, b_next, alpha_next, hidden, total)
-  AF_DISPATCH_DTYPE(a_dtype, TA, AF_DISPATCH_DTYPE(y_dtype, TY, if (vec) AF_ATN(TA, TY, 4); else AF_ATN(TA, TY, 1)));
+  AF_DISPATCH_DTYPE(a_dtype, TA, AF_DISPATCH_DTYPE(y_dtype, TY, if (vec) AF_ATN(add_tanh_norm4_kernel, TA, TY); else AF_ATN(add_tanh_norm_kernel, TA, TY)));
 #undef AF_ATN
   AF_CHECK_LAUNCH("af_add_tanh_norm");
 }
