@@ -247,7 +247,8 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const TA* __restrict__
 // The same for rows of up to 8192 elements with hidden % 4 == 0: a thread owns NV groups of four
 // elements (group v of thread t at element 4 (t + v * threads)), every load issued before the first
 // reduction.  Few rows (decode): NV = 1, many threads per row, what costs is the chain of memory
-// latencies; many rows (prefill): NV = 2, smaller blocks, more rows in flight on an SM.
+// latencies: the row of the stream is asked for with the first partial sums (all sixteen of a long product's at once would
+// take the registers that let the block stand by beside the product in front: 1,674 -> 1,695 us a step at batch 8); many rows (prefill): NV = 2, smaller blocks, more rows in flight on an SM.
 // MANY (the rows of a prompt): the kernel is bound by how many rows an SM holds at a time, so it keeps to 32
 // registers (seven blocks of a 2304-wide row per SM instead of four) and reads the norms' weights, which
 // every row shares and the L1 holds, where it uses them instead of keeping them from the start.
@@ -257,7 +258,7 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
                        const float* __restrict__ w_post, TY* __restrict__ y, const float* __restrict__ w_next,
                        int hidden, float eps_post, float eps_next, float offset) {
   pdl_launch_dependents();
-  __shared__ float scratch[33];
+  __shared__ float scratch[2][32];
   const int r = blockIdx.x;
   float av[NV][4], xv[NV][4], wp[NV][4], wn[NV][4];
   bool on[NV];
@@ -285,22 +286,11 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
     const int i = (threadIdx.x + v * blockDim.x) * 4;
     if (!on[v]) continue;
     const size_t at = (size_t)r * hidden + i;
+    const float4 xt = *reinterpret_cast<const float4*>(x + at);
+    xv[v][0] = xt.x, xv[v][1] = xt.y, xv[v][2] = xt.z, xv[v][3] = xt.w;
     if constexpr (sizeof(TA) == 4) {
-      const float* ap = reinterpret_cast<const float*>(a) + at;
-      for (int p0 = 0; p0 < n_parts; p0 += 8) {
-        float4 t[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          t[u] = p0 + u < n_parts ? *reinterpret_cast<const float4*>(ap + (size_t)(p0 + u) * part_stride)
-                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          av[v][0] += t[u].x;
-          av[v][1] += t[u].y;
-          av[v][2] += t[u].z;
-          av[v][3] += t[u].w;
-        }
-      }
+      const float4 t = sum_parts4<8>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
+      av[v][0] = t.x, av[v][1] = t.y, av[v][2] = t.z, av[v][3] = t.w;
     } else {
       const uint2 raw = *reinterpret_cast<const uint2*>(a + at);
       av[v][0] = __uint_as_float(raw.x << 16);
@@ -308,13 +298,11 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
       av[v][2] = __uint_as_float(raw.y << 16);
       av[v][3] = __uint_as_float(raw.y & 0xffff0000u);
     }
-    const float4 xt = *reinterpret_cast<const float4*>(x + at);
-    xv[v][0] = xt.x, xv[v][1] = xt.y, xv[v][2] = xt.z, xv[v][3] = xt.w;
   }
   float ss = 0.f;
 #pragma unroll
   for (int v = 0; v < NV; ++v) ss += av[v][0] * av[v][0] + av[v][1] * av[v][1] + av[v][2] * av[v][2] + av[v][3] * av[v][3];
-  ss = block_sum(ss, scratch);
+  ss = block_sum<true>(ss, scratch[0]);
   const float inv = rsqrtf(ss / (float)hidden + eps_post);
   float ss2 = 0.f;
 #pragma unroll
@@ -333,7 +321,7 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
           make_float4(xv[v][0], xv[v][1], xv[v][2], xv[v][3]);
   }
   if (y == nullptr) return;
-  ss2 = block_sum(ss2, scratch);
+  ss2 = block_sum<true>(ss2, scratch[1]);
   const float inv2 = rsqrtf(ss2 / (float)hidden + eps_next);
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
@@ -582,19 +570,8 @@ __device__ __forceinline__ void term_group(float* acc, float scale, const void* 
     acc[3] += scale * __uint_as_float(raw.y & 0xffff0000u);
     return;
   }
-  const float* f = static_cast<const float*>(p) + at;
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int p0 = 0; p0 < n_parts; p0 += 8) {
-    float4 t[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      t[u] = p0 + u < n_parts ? *reinterpret_cast<const float4*>(f + (size_t)(p0 + u) * part_stride)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v[0] += t[u].x, v[1] += t[u].y, v[2] += t[u].z, v[3] += t[u].w;
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) acc[u] += scale * v[u];
+  const float4 v = sum_parts4<8>(static_cast<const float*>(p) + at, n_parts, part_stride);
+  acc[0] += scale * v.x, acc[1] += scale * v.y, acc[2] += scale * v.z, acc[3] += scale * v.w;
 }
 
 template <typename TY, int NV>

@@ -44,6 +44,7 @@ __device__ __forceinline__ float ln_term1(const LnTerm& t, size_t at) {
   return s * t.scale;
 }
 
+template <int IN>
 __device__ __forceinline__ void ln_term4(const LnTerm& t, size_t at, float* v) {
   if (t.dtype == AF_BF16) {
     const uint2 raw = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(t.p) + at);
@@ -54,16 +55,7 @@ __device__ __forceinline__ void ln_term4(const LnTerm& t, size_t at, float* v) {
     return;
   }
   const float* p = reinterpret_cast<const float*>(t.p) + at;
-  float4 s = *reinterpret_cast<const float4*>(p);
-  for (int i0 = 1; i0 < t.parts; i0 += 4) {                 // (partial sums: four loads in flight, added in order)
-    float4 q[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      q[u] = i0 + u < t.parts ? *reinterpret_cast<const float4*>(p + (size_t)(i0 + u) * t.stride)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) s.x += q[u].x, s.y += q[u].y, s.z += q[u].z, s.w += q[u].w;
-  }
+  const float4 s = sum_parts4<IN>(p, t.parts, t.stride);
   v[0] = s.x * t.scale, v[1] = s.y * t.scale, v[2] = s.z * t.scale, v[3] = s.w * t.scale;
 }
 
@@ -190,11 +182,12 @@ norm_of_sum_kernel(LnSumArgs p) {
 // Rows of whole groups of four: a thread keeps NV groups in registers and every load of a group is in flight before
 // the first sum.  Few rows (a decode step): one group a thread, the weights and the state asked for before the wait for
 // the kernel in front; many rows (MANY): two groups a thread, the weights read where they are used (L1 holds them).
-template <typename TY, int NV, bool MANY, bool POST>
-__global__ void __launch_bounds__(MANY ? 512 : 1024, MANY ? 3 : 1)
+// IN: partial sums in flight at once (16 where the block leaves room for them: rows of up to 1,280).
+template <typename TY, int NV, bool MANY, bool POST, int IN = 4>
+__global__ void __launch_bounds__(MANY ? 512 : IN > 4 ? 320 : 1024, MANY ? 3 : 1)
 norm_of_sum_row_kernel(LnSumArgs p) {
   pdl_launch_dependents();
-  __shared__ float scratch[33];
+  __shared__ float scratch[2][32];
   const int r = blockIdx.x, hidden = p.hidden;
   const size_t base = (size_t)r * hidden;
   float v[NV][4], wv[NV][4], bv[NV][4], zb[NV][4], mu[NV][4], pv[NV][4], xs[POST ? NV : 1][4];
@@ -225,10 +218,10 @@ norm_of_sum_row_kernel(LnSumArgs p) {
     if (i >= hidden) continue;
     float xv[4], bt[4] = {0.f, 0.f, 0.f, 0.f}, zt[4];
     get4(p.x + base + i, xv);
-    ln_term4(p.a, base + i, v[n]);
-    if (p.b.p != nullptr) ln_term4(p.b, base + i, bt);
+    ln_term4<IN>(p.a, base + i, v[n]);
+    if (p.b.p != nullptr) ln_term4<IN>(p.b, base + i, bt);
     if (p.z.p != nullptr) {
-      ln_term4(p.z, base + i, zt);
+      ln_term4<IN>(p.z, base + i, zt);
       if (MANY) get4(p.z_bias + i, zb[n]);
     }
 #pragma unroll
@@ -240,7 +233,7 @@ norm_of_sum_row_kernel(LnSumArgs p) {
       s += v[n][u];
     }
   }
-  const float mean = block_sum(s, scratch) / (float)hidden;
+  const float mean = block_sum<true>(s, scratch[0]) / (float)hidden;
   float ss = 0.f;
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
@@ -251,7 +244,7 @@ norm_of_sum_row_kernel(LnSumArgs p) {
       ss += on ? v[n][u] * v[n][u] : 0.f;
     }
   }
-  const float inv = 1.f / sqrtf(block_sum(ss, scratch) / (float)hidden + p.eps);
+  const float inv = 1.f / sqrtf(block_sum<true>(ss, scratch[1]) / (float)hidden + p.eps);
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
     const int i = (threadIdx.x + n * blockDim.x) * 4;
@@ -412,10 +405,12 @@ AF_EXPORT int af_norm_of_sum(float* x, const void* a, int a_dtype, int a_parts, 
     const bool many = n_rows >= 256 && hidden >= 1024 && hidden <= 4096;
     const int nv = many || hidden > 4096 ? 2 : 1;
     const int threads = ((hidden / 4 + nv - 1) / nv + 31) / 32 * 32;
+    const int most = p.a.parts > p.b.parts ? p.a.parts : p.b.parts;
 #define LN_LAUNCH(TY, P)                                                                                              \
   do {                                                                                                                \
     if (many) af_launch(norm_of_sum_row_kernel<TY, 2, true, P>, dim3(n_rows), dim3(threads), 0, stream, p);           \
     else if (nv == 2) af_launch(norm_of_sum_row_kernel<TY, 2, false, P>, dim3(n_rows), dim3(threads), 0, stream, p);  \
+    else if (threads <= 320 && most > 4) af_launch(norm_of_sum_row_kernel<TY, 1, false, P, 16>, dim3(n_rows), dim3(threads), 0, stream, p); \
     else af_launch(norm_of_sum_row_kernel<TY, 1, false, P>, dim3(n_rows), dim3(threads), 0, stream, p);               \
   } while (0)
     if (post) AF_DISPATCH_DTYPE(y_dtype, TY, LN_LAUNCH(TY, true));
