@@ -18,7 +18,8 @@ struct AfHcTerm {
   float scale;
 };
 
-template <int VEC>
+// IN: partial sums in flight at once.
+template <int VEC, int IN>
 __device__ __forceinline__ void hc_term_add(float* acc, const AfHcTerm& t, size_t part_stride, size_t at) {
   if (t.p == nullptr) return;
   if (t.dtype == AF_BF16) {
@@ -37,7 +38,7 @@ __device__ __forceinline__ void hc_term_add(float* acc, const AfHcTerm& t, size_
   const float* f = static_cast<const float*>(t.p) + at;
   float v[VEC];
   if (VEC == 4) {
-    const float4 q = sum_parts4<8>(f, t.parts, part_stride);
+    const float4 q = sum_parts4<IN>(f, t.parts, part_stride);
     v[0] = q.x, v[1 % VEC] = q.y, v[2 % VEC] = q.z, v[3 % VEC] = q.w;
   } else {
     v[0] = 0.f;
@@ -150,8 +151,8 @@ hc_write_kernel(float* __restrict__ x, AfHcTerm a, AfHcTerm b, size_t part_strid
     float yv[VEC];
 #pragma unroll
     for (int e = 0; e < VEC; ++e) yv[e] = 0.f;
-    hc_term_add<VEC>(yv, a, part_stride, t * W + i);
-    hc_term_add<VEC>(yv, b, part_stride, t * W + i);
+    hc_term_add<VEC, SMAX <= 4 ? 2 : 8>(yv, a, part_stride, t * W + i);
+    hc_term_add<VEC, SMAX <= 4 ? 2 : 8>(yv, b, part_stride, t * W + i);
     if (ls != nullptr) {
       if (i != i0) hc_load<VEC>(l0, ls + i);
 #pragma unroll
