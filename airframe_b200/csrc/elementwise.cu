@@ -289,7 +289,7 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
     const float4 xt = *reinterpret_cast<const float4*>(x + at);
     xv[v][0] = xt.x, xv[v][1] = xt.y, xv[v][2] = xt.z, xv[v][3] = xt.w;
     if constexpr (sizeof(TA) == 4) {
-      const float4 t = sum_parts4<MANY ? 2 : 8>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
+      const float4 t = sum_parts4<MANY ? 1 : 8>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
       av[v][0] = t.x, av[v][1] = t.y, av[v][2] = t.z, av[v][3] = t.w;
     } else {
       const uint2 raw = *reinterpret_cast<const uint2*>(a + at);

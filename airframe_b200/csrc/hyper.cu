@@ -129,7 +129,7 @@ hc_write_kernel(float* __restrict__ x, AfHcTerm a, AfHcTerm b, size_t part_strid
   }
   // the first group's weights, for most widths the only one's, are on their way before the wait
   const int i0 = threadIdx.x * VEC;
-  const bool once = W <= (int)blockDim.x * VEC;
+  const bool once = SMAX > 4 && W <= (int)blockDim.x * VEC;      // (many tokens: no registers for it)
   float l0[VEC], w0[VEC], u0[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) l0[e] = w0[e] = u0[e] = 0.f;
@@ -151,8 +151,8 @@ hc_write_kernel(float* __restrict__ x, AfHcTerm a, AfHcTerm b, size_t part_strid
     float yv[VEC];
 #pragma unroll
     for (int e = 0; e < VEC; ++e) yv[e] = 0.f;
-    hc_term_add<VEC, SMAX <= 4 ? 2 : 8>(yv, a, part_stride, t * W + i);
-    hc_term_add<VEC, SMAX <= 4 ? 2 : 8>(yv, b, part_stride, t * W + i);
+    hc_term_add<VEC, SMAX <= 4 ? 1 : 8>(yv, a, part_stride, t * W + i);
+    hc_term_add<VEC, SMAX <= 4 ? 1 : 8>(yv, b, part_stride, t * W + i);
     if (ls != nullptr) {
       if (i != i0) hc_load<VEC>(l0, ls + i);
 #pragma unroll
