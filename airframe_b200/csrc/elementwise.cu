@@ -286,8 +286,11 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
     const int i = (threadIdx.x + v * blockDim.x) * 4;
     if (!on[v]) continue;
     const size_t at = (size_t)r * hidden + i;
-    const float4 xt = *reinterpret_cast<const float4*>(x + at);
-    xv[v][0] = xt.x, xv[v][1] = xt.y, xv[v][2] = xt.z, xv[v][3] = xt.w;
+    auto stream = [&] {
+      const float4 xt = *reinterpret_cast<const float4*>(x + at);
+      xv[v][0] = xt.x, xv[v][1] = xt.y, xv[v][2] = xt.z, xv[v][3] = xt.w;
+    };
+    if (!MANY) stream();
     if constexpr (sizeof(TA) == 4) {
       const float4 t = sum_parts4<MANY ? 1 : 8>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
       av[v][0] = t.x, av[v][1] = t.y, av[v][2] = t.z, av[v][3] = t.w;
@@ -298,6 +301,7 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
       av[v][2] = __uint_as_float(raw.y << 16);
       av[v][3] = __uint_as_float(raw.y & 0xffff0000u);
     }
+    if (MANY) stream();
   }
   float ss = 0.f;
 #pragma unroll
