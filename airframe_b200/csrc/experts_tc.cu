@@ -33,7 +33,10 @@ namespace {
 
 constexpr int EX_BM = 128;
 constexpr int EX_BK = 64;
-constexpr int EX_THREADS = 192;
+// Epilogue warps: four, or where the epilogue is long (the gates' exponentials and roots, 60 instructions an output) eight, which
+// take the chunks of a tile's rows in turn (four prompts of up to 1,023 tokens, 2,304 channels: 42 -> 29 us).
+__host__ __device__ constexpr int ex_epilogue_warps(int epi) { return epi == 2 ? 8 : 4; }
+__host__ __device__ constexpr int ex_threads(int epi) { return 64 + 32 * ex_epilogue_warps(epi); }
 
 __host__ __device__ constexpr int ex_stage_bytes(int bn, int nacc) { return nacc * EX_BM * EX_BK * 2 + bn * EX_BK * 2; }
 __host__ __device__ constexpr int ex_stages(int bn, int nacc) {
@@ -106,7 +109,7 @@ __device__ __forceinline__ void ex_tile(const ExArgs& a, int row_tile, int bn, i
 }
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(EX_THREADS, BN <= 64 ? 2 : 1)
+__global__ void __launch_bounds__(ex_threads(EPI), BN <= 64 ? 2 : 1)
 expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                       const __grid_constant__ CUtensorMap map_x, ExArgs a) {
   constexpr bool DUAL = ex_accs(EPI) == 2;
@@ -139,7 +142,7 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_c
       mbar_init(&empty[s], 1);
     }
     mbar_init(&acc_full, 1);
-    mbar_init(&acc_empty, 4);   // one arrival an epilogue warp
+    mbar_init(&acc_empty, ex_epilogue_warps(EPI));   // one arrival an epilogue warp
     give_up_s = 0;
     mbar_fence_init();
   }
@@ -226,18 +229,35 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_c
     }
   } else {
     const int quarter = warp & 3;          // this warp reads TMEM lanes [32 * quarter, + 32)
-    constexpr int CW = BN >= 32 ? 32 : 16;
+    constexpr int CW = BN >= 32 && !GATES ? 32 : 16;
+    constexpr int GROUPS = ex_epilogue_warps(EPI) / 4;
+    const int group = (warp - 2) >> 2;
+    static_assert(EX_GATES == 2, "ex_epilogue_warps");
     int round = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++round) {
       int expert, row0, rows;
       ex_tile(a, tile / a.tiles_w, BN, &expert, &row0, &rows);
       const int f = (tile % a.tiles_w) * EX_BM + quarter * 32 + lane;
+      const int n_chunks = (min(rows, BN) + CW - 1) / CW;
+      // (GATES: what a chunk reads besides the sums is asked for before the wait for them)
+      float uv[GATES ? CW : 1], ab = 0.f, ib = 0.f, rt = 0.f;
+      auto fetch = [&](int ch) {
+        if constexpr (GATES) {
+          const int n = f < a.N ? min(CW, rows - ch * CW) : 0;
+          const float* src = a.u + (size_t)(row0 + ch * CW) * a.ld_u + expert * a.N + f;
+#pragma unroll
+          for (int j = 0; j < CW; ++j) uv[j] = j < n ? __ldcg(src + (size_t)j * a.ld_u) : 0.f;
+        }
+      };
+      if constexpr (GATES) {
+        if (f < a.N) ab = __ldg(a.ba + expert * a.N + f), ib = __ldg(a.bi + expert * a.N + f), rt = __ldg(a.rate + expert * a.N + f);
+        fetch(group);
+      }
       if (!mbar_wait(&acc_full, round & 1, give_up)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
-      const int n_chunks = (min(rows, BN) + CW - 1) / CW;
 #pragma unroll 1
-      for (int ch = 0; ch < n_chunks; ++ch) {
+      for (int ch = group; ch < n_chunks; ch += GROUPS) {
         const int c0 = ch * CW;
         float g[CW], u[DUAL ? CW : 1];
         if constexpr (CW == 32) {
@@ -249,7 +269,7 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_c
         }
         if constexpr (GATES) {
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (ch == n_chunks - 1) {
+          if (ch + GROUPS >= n_chunks) {
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty);
@@ -257,11 +277,7 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_c
           if (f < a.N) {
             const int col = expert * a.N + f;
             const size_t ldu = (size_t)a.ld_u;
-            const float ab = __ldg(a.ba + col), ib = __ldg(a.bi + col), rt = __ldg(a.rate + col);
             const int n = min(CW, rows - c0);
-            float uv[CW];
-#pragma unroll
-            for (int j = 0; j < CW; ++j) uv[j] = j < n ? __ldcg(a.u + (size_t)(row0 + c0 + j) * ldu + col) : 0.f;
 #pragma unroll
             for (int j = 0; j < CW; ++j) {
               if (j >= n) continue;
@@ -273,6 +289,7 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_c
               a.out2[at] = sqrtf(d * (2.f - d)) * i * uv[j];          // 1 - a^2 = (1 - a)(1 + a)
             }
           }
+          if (ch + GROUPS < n_chunks) fetch(ch + GROUPS);
           continue;
         }
         // what the chunk's rows need besides the sums: lane l fetches it for row c0 + l
@@ -322,7 +339,7 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_c
           }
         }
       }
-      if (n_chunks == 0) {      // (a tile without rows: never planned, but the accumulators must be handed back)
+      if (group >= n_chunks) {  // (a tile with fewer chunks than there are groups: the accumulators must be handed back all the same)
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty);
@@ -353,7 +370,7 @@ int ex_launch(const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap& m
   if (sms <= 0) return -1;
   const long long tiles = (long long)a.max_row_tiles * a.tiles_w;
   const long long most = BN <= 64 ? tiles : (tiles < sms ? tiles : sms);   // few rows: a block per tile
-  af_launch(expert_rows_tc_kernel<BN, EPI>, dim3((unsigned)most), dim3(EX_THREADS), smem, stream, m0, m1, mx, a);
+  af_launch(expert_rows_tc_kernel<BN, EPI>, dim3((unsigned)most), dim3(ex_threads(EPI)), smem, stream, m0, m1, mx, a);
   AF_CHECK_LAUNCH("af_expert_rows_tc");
 }
 
