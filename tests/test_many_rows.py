@@ -16,6 +16,33 @@ def K():
     return kernels
 
 
+@pytest.mark.parametrize("nq, nkv, hd, dv", [(6, 2, 64, 64), (2, 1, 8, 8), (3, 3, 24, 24)])
+@pytest.mark.parametrize("T, table, bias", [(64, True, False), (130, False, True)])
+def test_whole_norm_of_a_prompt(K, nq, nkv, hd, dv, T, table, bias):
+    """Against the same rows in steps of up to 63 tokens, whose sums of squares meet in another order (2^-20 of the factor, so
+    that a result may round to the neighbouring bfloat16)."""
+    g = torch.Generator().manual_seed(T + hd)
+    n_q, n_k, n_v = nq * hd, nkv * hd, nkv * dv
+    proj = (torch.randn(T, n_q + n_k + n_v, generator=g) * 3).to(DEV)
+    wq, wk = torch.randn(n_q, generator=g).to(DEV), torch.randn(n_k, generator=g).to(DEV)
+    b = torch.randn(n_q + n_k + n_v, generator=g).to(DEV) if bias else None
+    inv = (10000.0 ** (-torch.arange(0, hd, 2) / hd)).float().to(DEV)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+
+    def run(lo, hi):
+        zeros = torch.zeros(hi - lo, dtype=torch.int32, device=DEV)
+        batch = SimpleNamespace(positions=pos[lo:hi], seq_of_token=zeros, slots=zeros[:1],
+                                len_after=torch.full((1,), T, dtype=torch.int32, device=DEV), aux={})
+        out = torch.empty(hi - lo, n_q + n_k + n_v, dtype=torch.bfloat16, device=DEV)
+        K.qk_norm_rope_store(out, proj[lo:hi], batch, nq, nkv, hd, inv, hd, "half", q_weight=wq, k_weight=wk, eps=1e-5, dv=dv,
+                             whole_norm=True, bias=b, table=K.rope_table(pos[lo:hi], inv) if table else None)
+        return out.double()
+
+    got, want = run(0, T), torch.cat([run(i, min(T, i + 50)) for i in range(0, T, 50)])
+    assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-4).all()
+    assert (got == want).double().mean() > 0.99
+
+
 @pytest.mark.parametrize("width, taps", [(64, 4), (516, 2), (60, 3)])
 def test_convolution_of_four_channels_a_thread(K, width, taps):
     """Sequences that begin inside a group of tokens, with and without a history, against rows that cannot be read in fours."""
