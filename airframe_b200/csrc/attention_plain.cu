@@ -435,7 +435,8 @@ __global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__
                                           int n_tokens, int nq, int nkv, int hd, int dv, float scale, float cap,
                                           int window, int mask_kind, int keep, const float* __restrict__ slopes,
                                           const float* __restrict__ sinks, const float* __restrict__ gate,
-                                          long long gate_stride) {
+                                          long long gate_stride, const int* __restrict__ seq_of_token,
+                                          const int* __restrict__ seq_starts, int below) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, split = FEW ? 0 : warp;
@@ -443,6 +444,10 @@ __global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__
   if (FEW && unit >= (long long)n_tokens * nq) return;
   const int t = n_tokens - 1 - (int)(unit / nq), h = (int)(unit % nq);      // (the last tokens, which see most, first)
   const int g = h / (nq / nkv);
+  if (below > 0) {                       // (longer sequences are another kernel's)
+    const int seq = seq_of_token[t];
+    if (seq_starts[seq + 1] - seq_starts[seq] >= below) return;
+  }
   const int pos = positions[t];          // position inside its sequence
   const int first_row = t - pos;         // row of the sequence's position 0
   using Attn = WarpAttn<NS>;
@@ -501,19 +506,20 @@ __global__ void __launch_bounds__(128) attn_prefill_plain_kernel(T* __restrict__
   attn_store(st, out + (size_t)t * out_stride + (size_t)h * dv, dv, lane, gate_factor(gate, gate_stride, t, h));
 }
 
-// `max_keys`: no token sees more.
+// `max_keys`: no token sees more.  `below` > 0: only sequences of fewer tokens, told by seq_of_token and seq_starts.
 AF_EXPORT int af_attn_prefill_plain(void* out, int out_stride, const void* q, int q_stride,
                                     const void* k, int k_stride, const void* v, int v_stride, int dtype,
                                     const int* positions, int n_tokens, int nq, int nkv, int hd, int dv,
                                     float scale, float cap, int window, int mask_kind, int keep, const float* slopes,
                                     const float* sinks, const float* gate, long long gate_stride, int max_keys,
-                                    cudaStream_t stream) {
+                                    const int* seq_of_token, const int* seq_starts, int below, cudaStream_t stream) {
   if (n_tokens == 0) return 0;
   AF_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "af_attn_prefill_plain: heads %d, groups %d", nq, nkv);
   AF_REQUIRE(hd > 0 && hd <= AF_MAX_HD && dv > 0 && dv <= AF_MAX_HD,
              "af_attn_prefill_plain: key size %d or value size %d beyond %d", hd, dv, AF_MAX_HD);
   AF_REQUIRE(mask_kind == AF_MASK_WINDOW || mask_kind == AF_MASK_CHUNK, "af_attn_prefill_plain: mask kind %d", mask_kind);
   AF_REQUIRE(keep >= 0, "af_attn_prefill_plain: %d kept tokens", keep);
+  AF_REQUIRE(below <= 0 || (seq_of_token != nullptr && seq_starts != nullptr), "af_attn_prefill_plain: the sequences' rows");
   const bool few = max_keys < AF_PLAIN_SPLIT;
   const long long units = (long long)n_tokens * nq, blocks = few ? (units + 3) / 4 : units;
   const int slices = (max(hd, dv) + 31) / 32;
@@ -525,7 +531,7 @@ AF_EXPORT int af_attn_prefill_plain(void* out, int out_stride, const void* q, in
                     af_launch(kernel, dim3((unsigned)blocks), dim3(128), 0, stream, 
                         (T*)out, out_stride, (const T*)q, q_stride, (const T*)k, k_stride, (const T*)v,
                         v_stride, positions, n_tokens, nq, nkv, hd, dv, scale, cap, window, mask_kind, keep, slopes,
-                        sinks, gate, gate_stride));
+                        sinks, gate, gate_stride, seq_of_token, seq_starts, below));
   AF_CHECK_LAUNCH("af_attn_prefill_plain");
 }
 

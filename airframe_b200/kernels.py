@@ -354,7 +354,7 @@ def _most_keys(max_len: int, window: int, keep: int) -> int:
 
 def attn_prefill_plain(out, q, k, v, positions, nq: int, nkv: int, hd: int, scale: float, cap: float,
                        window: int, slopes=None, dv=None, mask: str = "window", sinks=None, gate=None,
-                       keep: int = 0, max_len: int = 0) -> None:
+                       keep: int = 0, max_len: int = 0, seqs=None, below: int = 0) -> None:
     """Attention of prompts that start at position 0 over the step's own keys.
     q [T, nq*hd], k [T, nkv*hd], v [T, nkv*dv] are row views (any row stride; ``dv`` = hd by default).
     ``window`` > 0 with ``mask`` "window": a position sees the last ``window`` ones; "chunk": those of its
@@ -362,7 +362,8 @@ def attn_prefill_plain(out, q, k, v, positions, nq: int, nkv: int, hd: int, scal
     is added to head h's scores after scale and cap (a position encoding that biases scores).  ``sinks``
     (float32 [nq]): exp(sink[h]) joins head h's softmax denominator without a key or a value.  ``gate``
     (float32 [T, nq] logits): head h's output is multiplied by their sigmoid.  ``max_len``: no sequence is longer (0: unknown;
-    short prompts have kernels of their own, with the same bits)."""
+    short prompts have kernels of their own, with the same bits).  ``below`` > 0: only the sequences of fewer tokens, whose rows
+    ``seqs`` = (seq_of_token, seq_starts) tells."""
     if slopes is not None and slopes.numel() != nq:
         raise KernelError(f"attn_prefill_plain: {slopes.numel()} slopes for {nq} heads")
     if sinks is not None and sinks.numel() != nq:
@@ -377,7 +378,33 @@ def attn_prefill_plain(out, q, k, v, positions, nq: int, nkv: int, hd: int, scal
         c_int(T), c_int(nq), c_int(nkv), c_int(hd), c_int(dv or hd), c_float(scale), c_float(cap), c_int(window),
         c_int(MASKS[mask]), c_int(keep), _ptr(slopes, "slopes", torch.float32, allow_none=True),
         _ptr(sinks, "sinks", torch.float32, allow_none=True), gp, gs,
-        c_int(_most_keys(max_len or T, window, keep)), _stream()))
+        c_int(_most_keys(max_len or T, window, keep)), *(_ptr(t, "seqs", torch.int32, allow_none=True) for t in seqs or (None, None)),
+        c_int(below), _stream()))
+
+
+# From how many tokens on a sequence's 32-bit attention goes in tiles of 16 queries, where keys and values have up to
+# 256 elements: a sequence's own length decides, so that its bits do not depend on the sequences beside it.
+F32_TILES_FROM = 64
+
+
+def attn_prefill_f32(out, q, k, v, seq_starts, n_seqs: int, max_len: int, nq: int, nkv: int, hd: int, scale: float, cap: float,
+                     window: int, slopes=None, dv=None, mask: str = "window", sinks=None, gate=None, keep: int = 0,
+                     least: int = 1) -> None:
+    """Attention of the prompts of ``least`` tokens and more, float32, in tiles of 16 queries (``seq_starts`` int32
+    [n_seqs + 1], no sequence longer than ``max_len``; options as in :func:`attn_prefill_plain`)."""
+    if any(t.dtype != torch.float32 for t in (out, q, k, v)):
+        raise KernelError("attn_prefill_f32: float32 only")
+    if any(t is not None and t.numel() != nq for t in (slopes, sinks)):
+        raise KernelError(f"attn_prefill_f32: a slope and a sink for each of {nq} heads")
+    if mask not in MASKS:
+        raise KernelError(f"attn_prefill_f32: unknown mask '{mask}'")
+    gp, gs = _gate_args(gate, q.shape[0], nq, "attn_prefill_f32")
+    _check(_lib().af_attn_prefill_f32(
+        _ptr(out), c_longlong(_rows(out, "out")), _ptr(q), c_longlong(_rows(q, "q")), _ptr(k), c_longlong(_rows(k, "k")),
+        _ptr(v), c_longlong(_rows(v, "v")), _ptr(seq_starts, "seq_starts", torch.int32), c_int(n_seqs), c_int(max_len), c_int(least),
+        c_int(nq), c_int(nkv), c_int(hd), c_int(dv or hd), c_float(scale), c_float(cap), c_int(window), c_int(MASKS[mask]),
+        c_int(keep), _ptr(slopes, "slopes", torch.float32, allow_none=True), _ptr(sinks, "sinks", torch.float32, allow_none=True),
+        gp, gs, _stream()))
 
 
 def plain_decode_splits(batch: int, nq: int, most_keys: int) -> int:
@@ -785,6 +812,15 @@ def attn_prefill(out, q, k, v, batch, nq, nkv, hd, scale, cap, window, slopes=No
     use_tc = fast and aligned and bool(_lib().af_attn_prefill_tc_supported(c_int(hd)))
     use_mma = fast and not use_tc and bool(_lib().af_attn_prefill_supported(c_int(hd))) \
         and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v))
+    lens = getattr(batch, "seq_lens", None)
+    if q.dtype == torch.float32 and max(hd, dv or hd) <= 256 and lens and batch.n_seqs <= 65535 and max(lens) >= F32_TILES_FROM:
+        attn_prefill_f32(out, q, k, v, batch.seq_starts, batch.n_seqs, batch.max_len, nq, nkv, hd, scale, cap, window, slopes, dv,
+                         mask, sinks, gate, keep, least=F32_TILES_FROM)
+        if min(lens) < F32_TILES_FROM:
+            attn_prefill_plain(out, q, k, v, batch.positions, nq, nkv, hd, scale, cap, window, slopes, dv=dv, mask=mask, sinks=sinks,
+                               gate=gate, keep=keep, max_len=max(n for n in lens if n < F32_TILES_FROM),
+                               seqs=(batch.seq_of_token, batch.seq_starts), below=F32_TILES_FROM)
+        return
     if not (use_tc or use_mma):
         attn_prefill_plain(out, q, k, v, batch.positions, nq, nkv, hd, scale, cap, window, slopes, dv=dv, mask=mask,
                            sinks=sinks, gate=gate, keep=keep, max_len=getattr(batch, "max_len", 0))

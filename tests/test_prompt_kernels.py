@@ -33,3 +33,82 @@ def test_gemm_tensor_cores_token_tiles(K, N, Kd, out_dtype):
                 out = torch.full((M, N), float("nan"), device=DEV, dtype=out_dtype)
                 K.gemm_tc(out, x, w, n_acc=n_acc, token_tile=tile)
                 assert torch.equal(out, first), (M, n_acc, tile)
+
+
+def _attend(q, k, v, scale, cap, seen, slopes, sinks, gate):
+    """One sequence in 64 bits: q [n, H, d], k [n, G, d], v [n, G, dv]."""
+    n, H = q.shape[:2]
+    i, j = torch.arange(n)[:, None], torch.arange(n)[None, :]
+    out = []
+    for h in range(H):
+        g = h * k.shape[1] // H
+        s = (q[:, h].double() @ k[:, g].double().T) * scale
+        s = cap * torch.tanh(s / cap) if cap else s
+        s = (s + (slopes[h].double() * (j - i) if slopes is not None else 0.0)).masked_fill(~seen, -math.inf)
+        if sinks is not None:
+            s = torch.cat([s, sinks[h].double().expand(n, 1)], 1)
+        o = s.softmax(1)[:, :n] @ v[:, g].double()
+        out.append(o * torch.sigmoid(gate[:, h].double())[:, None] if gate is not None else o)
+    return torch.stack(out, 1)
+
+
+@pytest.mark.parametrize("hd, dv, nq, nkv", [(64, 64, 2, 1), (40, 24, 4, 2), (128, 128, 3, 3), (96, 256, 2, 1), (130, 30, 2, 2), (256, 256, 4, 2),
+                                             (255, 129, 2, 1)])
+@pytest.mark.parametrize("mask, window, keep, extras", [("window", 0, 0, False), ("window", 33, 5, True), ("window", 70, 0, True), ("chunk", 50, 70, True)])
+def test_attention_prefill_f32(K, hd, dv, nq, nkv, mask, window, keep, extras):
+    """Sequences around the tiles of 16 queries and 64 keys; sizes that fill no tile or no 16-byte piece; windows, chunks and first
+    tokens that stay visible; slopes, sinks, gates and a cap.  Bound: sums of up to 300 32-bit terms of size one."""
+    gen = torch.Generator().manual_seed(hd + dv + window)
+    lens, least = [64, 1, 65, 15, 129, 80, 300], 16
+    T = sum(lens)
+    q, k, v = (torch.randn(T, n, generator=gen) for n in (nq * hd, nkv * hd, nkv * dv))
+    slopes, sinks, gate = (torch.rand(nq, generator=gen), torch.randn(nq, generator=gen), torch.randn(T, nq, generator=gen)) if extras else (None,) * 3
+    cap = 20.0 if extras else 0.0
+    starts = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32)
+    out = torch.full((T, nq * dv), 7.0, device=DEV)
+    to = [None if t is None else t.to(DEV) for t in (slopes, sinks, gate)]
+    K.attn_prefill_f32(out, q.to(DEV), k.to(DEV), v.to(DEV), starts.to(DEV), len(lens), max(lens), nq, nkv, hd, hd ** -0.5, cap, window, to[0], dv,
+                       mask, to[1], to[2], keep, least=least)
+    at = 0
+    for n in lens:
+        s, i, j = slice(at, at + n), torch.arange(n)[:, None], torch.arange(n)[None, :]
+        at += n
+        if n < least:                       # (another kernel's: nothing is written)
+            assert bool((out[s] == 7.0).all())
+            continue
+        seen = j <= i
+        if window:
+            seen = seen & (((i // window == j // window) if mask == "chunk" else (i - j < window)) | (j < keep))
+        want = _attend(q[s].view(n, nq, hd), k[s].view(n, nkv, hd), v[s].view(n, nkv, dv), hd ** -0.5, cap, seen, slopes, sinks,
+                       gate[s] if extras else None)
+        err = (out[s].double().cpu().view(n, nq, dv) - want).abs().max()
+        assert err < 4e-6, (n, float(err))
+
+
+def test_attention_prefill_f32_of_a_step(K):
+    """A step's long and short sequences by two kernels: each sequence has the bits that it has alone, and what is not finite
+    reaches only the tokens that see it."""
+    gen = torch.Generator().manual_seed(5)
+    lens, nq, nkv, hd = [63, 200, 3, 64, 90], 4, 2, 64
+    T = sum(lens)
+    q, k, v = (torch.randn(T, n * hd, generator=gen).to(DEV) for n in (nq, nkv, nkv))
+
+    def run(q, k, v, lens):
+        starts = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+        batch = SimpleNamespace(seq_lens=lens, n_seqs=len(lens), max_len=max(lens), seq_starts=starts,
+                                positions=torch.cat([torch.arange(n) for n in lens]).to(DEV, torch.int32),
+                                seq_of_token=torch.cat([torch.full((n,), i) for i, n in enumerate(lens)]).to(DEV, torch.int32))
+        out = torch.full((sum(lens), nq * hd), 7.0, device=DEV)
+        K.attn_prefill(out, q, k, v, batch, nq, nkv, hd, hd ** -0.5, 0.0, 0)
+        return out
+
+    together, at = run(q, k, v, lens), 0
+    for n in lens:
+        assert torch.equal(together[at:at + n], run(q[at:at + n], k[at:at + n], v[at:at + n], [n]))
+        at += n
+    for bad, t in ((float("nan"), k), (float("inf"), v), (float("nan"), v)):
+        u = t.clone()
+        u[63 + 70] = bad                                   # (token 70 of the second sequence)
+        out = run(q, u if t is k else k, u if t is v else v, lens)
+        assert torch.equal(out[:63 + 70], together[:63 + 70]) and torch.equal(out[263:], together[263:])
+        assert not out[63 + 70:263].isfinite().any()
