@@ -263,7 +263,7 @@ def kv_keep(kv) -> int:
     return int(getattr(kv, "keep_first", 0))
 
 
-ROPE_TABLE_ROWS = 64     # from this many rows on, the rotary kernel for bfloat16 rows takes the step's table
+ROPE_TABLE_ROWS = 64     # from this many rows on, the rotary kernels for whole rows take the step's table
 
 
 def rope_cache_write(qkv, positions, inv_freq, nq: int, nkv: int, hd: int, rot_dim: int, pairing: str,

@@ -136,7 +136,7 @@ class Rope(PositionEncoding):
             raise ConfigError(f"rope: rotary_dim {self.rotary_dim} exceeds head_dim {hd}")
         # many rows (a prompt): the cosines and sines come from the step's table, made once for all layers
         table = None
-        if (qkv.shape[0] >= kernels.ROPE_TABLE_ROWS and parts is None and qkv.dtype == torch.bfloat16
+        if (qkv.shape[0] >= kernels.ROPE_TABLE_ROWS and parts is None
                 and self.rotates_half_pairs(hd)):
             table = self.rotary_table(batch, hd)
         kernels.rope_cache_write(qkv, batch.positions, self.inv_freq, nq, nkv, hd, self.rotary_dim,

@@ -16,6 +16,60 @@ def K():
     return kernels
 
 
+def rope_step(K, qkv, pos, nq, nkv, hd, table):
+    """Rows turned in place and stored: (rows, key pages, value pages) of one sequence at positions 0 ..."""
+    T, pages = qkv.shape[0], (int(pos.max()) + 64) // 64
+    inv = (10000.0 ** (-torch.arange(0, hd, 2) / hd)).float().to(DEV)
+    zeros = torch.zeros(T, dtype=torch.int32, device=DEV)
+    slots, after = zeros[:1], torch.full((1,), int(pos.max()) + 1, dtype=torch.int32, device=DEV)
+    kc, vc = (torch.full((pages, nkv, K.PAGE, hd), 7.0, dtype=qkv.dtype, device=DEV) for _ in range(2))
+    table = K.rope_table(pos, inv) if table else None
+    K.rope_cache_write(qkv, pos, inv, nq, nkv, hd, hd, "half", seq_of_token=zeros, slots=slots, len_after=after, kcache=kc, vcache=vc,
+                       page_table=torch.arange(pages, dtype=torch.int32, device=DEV)[None], ring_rows=pages * 64, table=table)
+    return qkv, kc, vc
+
+
+@pytest.mark.parametrize("dtype, T, piece", [(torch.bfloat16, 1001, 500), (torch.float32, 130, 1), (torch.float32, 7, 7)])
+@pytest.mark.parametrize("nq, nkv, hd", [(4, 2, 64), (3, 1, 8), (8, 4, 256)])
+def test_rotated_rows(K, dtype, T, piece, nq, nkv, hd):
+    """Bits do not depend on how many rows a step has nor on where the angles come from; 64 bits beside them."""
+    g = torch.Generator().manual_seed(T + hd)
+    rows = torch.randn(T, (nq + 2 * nkv) * hd, generator=g).to(dtype)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    first = rope_step(K, rows.to(DEV), pos, nq, nkv, hd, True)
+    for a, b in zip(first, rope_step(K, rows.to(DEV), pos, nq, nkv, hd, False)):
+        assert torch.equal(a, b)
+    parts = [rope_step(K, rows[i:i + piece].to(DEV), pos[i:i + piece], nq, nkv, hd, True)[0] for i in range(0, T, piece)]
+    assert torch.equal(first[0], torch.cat(parts))
+    x = rows[:, :(nq + nkv) * hd].double().view(T, nq + nkv, hd)
+    a = torch.arange(T).double()[:, None, None] * (10000.0 ** (-torch.arange(0, hd, 2) / hd)).float().double()
+    lo, hi = x[..., :hd // 2], x[..., hd // 2:]
+    want = torch.cat([lo * a.cos() - hi * a.sin(), hi * a.cos() + lo * a.sin()], -1)
+    got = first[0].double().cpu()
+    # (an angle of up to T, rounded to 32 bits; a result of up to 6 rounded to its type)
+    tol = 6 * (T * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22))
+    assert (got[:, :(nq + nkv) * hd].view(T, nq + nkv, hd) - want).abs().max() < tol
+    assert torch.equal(got[:, (nq + nkv) * hd:], rows[:, (nq + nkv) * hd:].double())
+    k, v = got[:, nq * hd:(nq + nkv) * hd].view(T, nkv, hd), got[:, (nq + nkv) * hd:].view(T, nkv, hd)
+    for cache, rows_of in ((first[1], k), (first[2], v)):
+        stored = cache.transpose(1, 2).reshape(-1, nkv, hd).double().cpu()
+        assert torch.equal(stored[:T], rows_of) and bool((stored[T:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M, inter", [(1, 4), (3, 1024), (5, 1028), (2, 4100)])
+def test_gated_activation_of_32_bit_rows(K, M, inter):
+    """Four values a thread at the edges of a block's 1,024; the same bits as a row that cannot be read in fours."""
+    gu = torch.randn(M, 2 * inter, generator=torch.Generator().manual_seed(inter)) * 2
+    out = torch.empty(M, inter, device=DEV)
+    off = torch.empty(M * inter + 1, device=DEV)[1:].view(M, inter)     # (one value off the 16-byte pieces)
+    for act, f in (("gelu_tanh", lambda g: torch.nn.functional.gelu(g, approximate="tanh")), ("silu", torch.nn.functional.silu)):
+        K.gated_act(out, gu.to(DEV), act)
+        K.gated_act(off, gu.to(DEV), act)
+        assert torch.equal(out, off)
+        want = f(gu[:, :inter].double()) * gu[:, inter:].double()
+        assert (out.double().cpu() - want).abs().max() < 2e-6 * want.abs().max()
+
+
 @pytest.mark.parametrize("nq, nkv, hd, dv", [(6, 2, 64, 64), (2, 1, 8, 8), (3, 3, 24, 24)])
 @pytest.mark.parametrize("T, table, bias", [(64, True, False), (130, False, True)])
 def test_whole_norm_of_a_prompt(K, nq, nkv, hd, dv, T, table, bias):
