@@ -104,94 +104,99 @@ __global__ void rope_cache_kernel(T* __restrict__ qkv, int row_stride, const flo
   }
 }
 
-// The same for bfloat16 rows without partial sums, half-split pairs over the
-// whole head and head_dim % 16 == 0: one block per token, 16-byte loads and
-// stores, eight pairs a thread.
-__global__ void __launch_bounds__(256)
+// The same for bfloat16 rows without partial sums and half-split pairs over the whole head (head_dim % 8 == 0): a block
+// takes TOK tokens, a thread four pairs of the same place in every head it turns, so that the pairs' angles serve all of them and the
+// loads of all its tokens are under way together.  What bounds a long prompt are latencies, those of the chain slot - page - row in
+// front of a token among them: few blocks of several tokens, all on the chip at once (2,048 tokens, 8 + 4 heads of 256: 15.9 -> 10.0 us).
+template <int TOK>
+__global__ void __launch_bounds__(256, TOK == 1 ? 6 : 4)
 rope_cache_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride, const int* __restrict__ positions,
                       const int* __restrict__ seq_of_token, const int* __restrict__ slots,
                       const int* __restrict__ len_after, const float* __restrict__ inv_freq,
-                      const float2* __restrict__ table, int nq, int nkv, int hd,
+                      const float2* __restrict__ table, int nq, int nkv, int hd, int n_tokens,
                       __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache,
                       const int* __restrict__ page_table, int max_pages, int ring_rows, int keep) {
   pdl_launch_dependents();
-  // (positions, slots, lengths, page table and frequencies are inputs of the step: the row's place in
+  // (positions, slots, lengths, page table and frequencies are inputs of the step: the rows' places in
   // the cache and the sines and cosines are worked out before the wait for the kernel in front)
-  const int t = blockIdx.x;
-  const int pos = positions[t];
-  __nv_bfloat16* row = qkv + (size_t)t * row_stride;
-  const int half = hd / 2;
-  const int per_head = half / 8;                 // 16-byte pieces of a half head
-  const int n_heads = nq + 2 * nkv;
-  // where this token's k and v rows go in the cache
-  size_t dst_row = 0;
-  bool store = false;
-  if (kcache != nullptr) {
-    const int seq = seq_of_token[t];
-    const int slot = slots[seq];
-    if (slot >= 0 && af_cache_stores(pos, len_after[seq], ring_rows, keep)) {
-      const int r = af_cache_row(pos, ring_rows, keep);
-      if (AF_INDEX_OK(pos >= 0 && r / AF_PAGE < max_pages, r)) {
+  const int t0 = blockIdx.x * TOK, half = hd / 2, per_head = half / 4, n_heads = nq + 2 * nkv;
+  const int c = threadIdx.x % per_head * 4, head0 = threadIdx.x / per_head, step = blockDim.x / per_head;
+  int pos[TOK], dst[TOK];                          // (the row of kv head 0 in the cache; -1: not stored)
+#pragma unroll
+  for (int u = 0; u < TOK; ++u) pos[u] = t0 + u < n_tokens ? positions[t0 + u] : 0;
+#pragma unroll
+  for (int u = 0; u < TOK; ++u) {
+    dst[u] = -1;
+    if (kcache == nullptr || t0 + u >= n_tokens) continue;
+    const int seq = seq_of_token[t0 + u], slot = slots[seq];
+    if (slot >= 0 && af_cache_stores(pos[u], len_after[seq], ring_rows, keep)) {
+      const int r = af_cache_row(pos[u], ring_rows, keep);
+      if (AF_INDEX_OK(pos[u] >= 0 && r / AF_PAGE < max_pages, r)) {
         const int page = page_table[(size_t)slot * max_pages + r / AF_PAGE];
-        dst_row = ((size_t)page * nkv) * AF_PAGE + r % AF_PAGE;   // + h * AF_PAGE rows for kv head h
-        store = AF_INDEX_OK(page >= 0, page);
+        if (AF_INDEX_OK(page >= 0, page)) dst[u] = page * nkv * AF_PAGE + r % AF_PAGE;
       }
     }
   }
-  // a thread's pieces all have the same place in their heads when the block's size is a multiple of
-  // the pieces of a head (it is for head sizes up to 512 that divide so): its 8 pairs' angles are fixed
-  const bool fixed_c = blockDim.x % per_head == 0;
-  float sn0[8], cs0[8];
-  if (fixed_c && table == nullptr) {
-    const int c = threadIdx.x % per_head;
+  float cs[TOK][4], sn[TOK][4];
+  if (table == nullptr) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) sincosf((float)pos * inv_freq[c * 8 + e], &sn0[e], &cs0[e]);
+    for (int u = 0; u < TOK; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sincosf((float)pos[u] * inv_freq[c + e], &sn[u][e], &cs[u][e]);
   }
   pdl_wait();
-  row = pdl_fresh(row);
-  if (fixed_c && table != nullptr) {
+  qkv = pdl_fresh(qkv);
+  if (table != nullptr) {
     // the step's table of (cos, sin), made once for all layers by the same arithmetic (a kernel of this step
     // wrote it: read after the wait)
-    const float4* tp = reinterpret_cast<const float4*>(pdl_fresh(table) + (size_t)t * half + (threadIdx.x % per_head) * 8);
+    table = pdl_fresh(table);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float4 v = tp[e];
-      cs0[2 * e] = v.x, sn0[2 * e] = v.y, cs0[2 * e + 1] = v.z, sn0[2 * e + 1] = v.w;
+    for (int u = 0; u < TOK; ++u) {
+      const float4* tp = reinterpret_cast<const float4*>(table + (size_t)min(t0 + u, n_tokens - 1) * half + c);
+      const float4 x = tp[0], y = tp[1];
+      cs[u][0] = x.x, sn[u][0] = x.y, cs[u][1] = x.z, sn[u][1] = x.w, cs[u][2] = y.x, sn[u][2] = y.y, cs[u][3] = y.z, sn[u][3] = y.w;
     }
   }
-  for (int i = threadIdx.x; i < n_heads * per_head; i += blockDim.x) {
-    const int head = i / per_head, c = i - head * per_head;
-    __nv_bfloat16* x = row + (size_t)head * hd + c * 8;
-    uint4 lo = *reinterpret_cast<const uint4*>(x);
-    uint4 hi = *reinterpret_cast<const uint4*>(x + half);
-    if (head < nq + nkv) {
-      uint32_t* lw = reinterpret_cast<uint32_t*>(&lo);
-      uint32_t* hw = reinterpret_cast<uint32_t*>(&hi);
+  for (int head = head0; head < n_heads; head += step) {
+    uint2 lo[TOK], hi[TOK];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float a[2] = {__uint_as_float(lw[j] << 16), __uint_as_float(lw[j] & 0xffff0000u)};
-        float b[2] = {__uint_as_float(hw[j] << 16), __uint_as_float(hw[j] & 0xffff0000u)};
-        float ra[2], rb[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float sn = sn0[2 * j + e], cs = cs0[2 * j + e];
-          if (!fixed_c) sincosf((float)pos * inv_freq[c * 8 + 2 * j + e], &sn, &cs);
-          ra[e] = a[e] * cs - b[e] * sn;
-          rb[e] = b[e] * cs + a[e] * sn;
-        }
-        __nv_bfloat162 pa = __floats2bfloat162_rn(ra[0], ra[1]), pb = __floats2bfloat162_rn(rb[0], rb[1]);
-        lw[j] = *reinterpret_cast<uint32_t*>(&pa);
-        hw[j] = *reinterpret_cast<uint32_t*>(&pb);
-      }
-      *reinterpret_cast<uint4*>(x) = lo;
-      *reinterpret_cast<uint4*>(x + half) = hi;
+    for (int u = 0; u < TOK; ++u) {
+      if (t0 + u >= n_tokens) continue;
+      const __nv_bfloat16* x = qkv + (size_t)(t0 + u) * row_stride + (size_t)head * hd + c;
+      lo[u] = *reinterpret_cast<const uint2*>(x);
+      hi[u] = *reinterpret_cast<const uint2*>(x + half);
     }
-    if (store && head >= nq) {
-      const bool is_v = head >= nq + nkv;
-      const int h = head - nq - (is_v ? nkv : 0);
-      __nv_bfloat16* d = (is_v ? vcache : kcache) + (dst_row + (size_t)h * AF_PAGE) * hd + c * 8;
-      *reinterpret_cast<uint4*>(d) = lo;
-      *reinterpret_cast<uint4*>(d + half) = hi;
+#pragma unroll
+    for (int u = 0; u < TOK; ++u) {
+      if (t0 + u >= n_tokens) continue;
+      if (head < nq + nkv) {
+        uint32_t lw[2] = {lo[u].x, lo[u].y}, hw[2] = {hi[u].x, hi[u].y};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float a[2] = {__uint_as_float(lw[j] << 16), __uint_as_float(lw[j] & 0xffff0000u)};
+          const float b[2] = {__uint_as_float(hw[j] << 16), __uint_as_float(hw[j] & 0xffff0000u)};
+          float ra[2], rb[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float s = sn[u][2 * j + e], co = cs[u][2 * j + e];
+            ra[e] = a[e] * co - b[e] * s;
+            rb[e] = b[e] * co + a[e] * s;
+          }
+          const __nv_bfloat162 pa = __floats2bfloat162_rn(ra[0], ra[1]), pb = __floats2bfloat162_rn(rb[0], rb[1]);
+          lw[j] = *reinterpret_cast<const uint32_t*>(&pa);
+          hw[j] = *reinterpret_cast<const uint32_t*>(&pb);
+        }
+        lo[u] = make_uint2(lw[0], lw[1]), hi[u] = make_uint2(hw[0], hw[1]);
+        __nv_bfloat16* x = qkv + (size_t)(t0 + u) * row_stride + (size_t)head * hd + c;
+        *reinterpret_cast<uint2*>(x) = lo[u];
+        *reinterpret_cast<uint2*>(x + half) = hi[u];
+      }
+      if (dst[u] >= 0 && head >= nq) {
+        const bool is_v = head >= nq + nkv;
+        __nv_bfloat16* d = (is_v ? vcache : kcache) + ((size_t)dst[u] + (size_t)(head - nq - (is_v ? nkv : 0)) * AF_PAGE) * hd + c;
+        *reinterpret_cast<uint2*>(d) = lo[u];
+        *reinterpret_cast<uint2*>(d + half) = hi[u];
+      }
     }
   }
 }
@@ -269,13 +274,20 @@ AF_EXPORT int af_rope_cache_write(void* qkv, int dtype, int row_stride, const fl
   AF_REQUIRE(pairing == AF_PAIR_HALF || pairing == AF_PAIR_ADJACENT, "af_rope_cache_write: pairing");
   AF_REQUIRE(ring_rows % AF_PAGE == 0, "af_rope_cache_write: ring rows %d not whole pages", ring_rows);
   AF_REQUIRE((kcache == nullptr) == (vcache == nullptr), "af_rope_cache_write: k and v cache");
-  if (dtype == AF_BF16 && parts == nullptr && pairing == AF_PAIR_HALF && rot_dim == hd && hd % 16 == 0 &&
+  if (dtype == AF_BF16 && parts == nullptr && pairing == AF_PAIR_HALF && rot_dim == hd && hd % 16 == 0 && hd <= 2048 &&
       row_stride % 8 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)kcache & 15) == 0 &&
       ((uintptr_t)vcache & 15) == 0 && n_tokens >= 64) {
-    af_launch(rope_cache_vec_kernel, dim3(n_tokens), dim3(256), 0, stream, (__nv_bfloat16*)qkv, (long long)row_stride,
-              positions, seq_of_token, slots, len_after, inv_freq,
-              ((uintptr_t)table & 15) == 0 ? reinterpret_cast<const float2*>(table) : nullptr, nq, nkv, hd, (__nv_bfloat16*)kcache,
-              (__nv_bfloat16*)vcache, page_table, max_pages, ring_rows, keep);
+    const int per_head = hd / 8, block = 256 / per_head * per_head;
+    const float2* tab = ((uintptr_t)table & 15) == 0 ? reinterpret_cast<const float2*>(table) : nullptr;
+    // (several tokens a block as soon as a token a block would take more than one round of the SMs)
+    if (n_tokens > 6 * af_sm_count())
+      af_launch(rope_cache_vec_kernel<4>, dim3((n_tokens + 3) / 4), dim3(block), 0, stream, (__nv_bfloat16*)qkv, (long long)row_stride,
+                positions, seq_of_token, slots, len_after, inv_freq, tab, nq, nkv, hd, n_tokens, (__nv_bfloat16*)kcache,
+                (__nv_bfloat16*)vcache, page_table, max_pages, ring_rows, keep);
+    else
+      af_launch(rope_cache_vec_kernel<1>, dim3(n_tokens), dim3(block), 0, stream, (__nv_bfloat16*)qkv, (long long)row_stride,
+                positions, seq_of_token, slots, len_after, inv_freq, tab, nq, nkv, hd, n_tokens, (__nv_bfloat16*)kcache,
+                (__nv_bfloat16*)vcache, page_table, max_pages, ring_rows, keep);
     AF_CHECK_LAUNCH("af_rope_cache_write");
   }
   if (dtype == AF_F32 && parts == nullptr && pairing == AF_PAIR_HALF && rot_dim == hd && hd % 8 == 0 && hd <= 2048 && row_stride % 4 == 0 &&
