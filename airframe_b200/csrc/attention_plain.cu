@@ -1366,9 +1366,14 @@ latent_prep_kernel(LatentPrepArgs<T> p) {
   pdl_launch_dependents();
   __shared__ float scratch[33];
   const int t = blockIdx.x, rot = p.rot, rank = p.rank, dim = p.dim;
+  // (few tokens: the first of a token's blocks takes the latent row and what goes beside it, the others the heads'
+  // queries: 8 tokens 5.8 -> 3.0 us)
+  const bool rows = blockIdx.y == 0, queries = gridDim.y == 1 || blockIdx.y > 0;
+  const int u0 = gridDim.y == 1 ? 0 : ((int)blockIdx.y - 1) * p.heads / ((int)gridDim.y - 1);
+  const int heads = gridDim.y == 1 ? p.heads : (int)blockIdx.y * p.heads / ((int)gridDim.y - 1) - u0;
   const int pos = p.positions[t];
   T* kdst = nullptr;
-  if (p.kcache != nullptr && p.kv_src != nullptr) {
+  if (rows && p.kcache != nullptr && p.kv_src != nullptr) {
     const int seq = p.seq_of_token[t];
     const int slot = p.slots[seq];
     if (slot >= 0 && !(p.ring_rows > 0 && pos + p.ring_rows < p.len_after[seq])) {
@@ -1391,7 +1396,7 @@ latent_prep_kernel(LatentPrepArgs<T> p) {
   };
   auto first_of = [&](int i) { return p.adjacent ? 2 * i : i; };
   auto second_of = [&](int i) { return p.adjacent ? 2 * i + 1 : i + half; };
-  if (p.kv_src != nullptr) {
+  if (rows && p.kv_src != nullptr) {
     const float* lat = p.kv_src + (size_t)t * p.kv_ld;
     T* kvr = p.kv + (size_t)t * p.kv_stride;
     float ss = 0.f;
@@ -1412,7 +1417,7 @@ latent_prep_kernel(LatentPrepArgs<T> p) {
       if (kdst != nullptr) kdst[rank + e0] = ra, kdst[rank + e1] = rb;
     }
   }
-  if (p.side_src != nullptr) {
+  if (rows && p.side_src != nullptr) {
     const float* src = p.side_src + (size_t)t * p.side_ld;
     T* dst = p.side + (size_t)t * p.side_stride;
     float ss = 0.f;
@@ -1421,29 +1426,30 @@ latent_prep_kernel(LatentPrepArgs<T> p) {
     const float inv = rsqrtf(ss / (float)p.side_n + p.eps);
     for (int i = threadIdx.x; i < p.side_n; i += blockDim.x) dst[i] = from_f32<T>(src[i] * inv * p.side_w[i]);
   }
-  if (p.q_src == nullptr) return;
+  if (!queries || p.q_src == nullptr) return;
   const float* x = p.q_src + (size_t)t * p.q_ld;
   auto q_at = [&](int i) {
     float s = x[i];
+#pragma unroll 8
     for (int u = 1; u < p.q_parts; ++u) s += x[(size_t)u * p.q_part_stride + i];
     return s;
   };
   T* qr = p.q + (size_t)t * p.q_stride;
-  for (int i = threadIdx.x; i < p.heads * half; i += blockDim.x) {
-    const int u = i / half, e = i - u * half;
+  for (int i = threadIdx.x; i < heads * half; i += blockDim.x) {
+    const int u = u0 + i / half, e = i % half;
     const float2 cs = turn(e);
     const int e0 = first_of(e), e1 = second_of(e);
     const float a = q_at(u * (dim + rot) + dim + e0), b = q_at(u * (dim + rot) + dim + e1);
     T* d = qr + (size_t)u * p.pitch + dim;
     d[e0] = from_f32<T>(a * cs.x - b * cs.y), d[e1] = from_f32<T>(b * cs.x + a * cs.y);
   }
-  for (int i = threadIdx.x; i < p.heads * dim; i += blockDim.x) {
-    const int u = i / dim, e = i - u * dim;
+  for (int i = threadIdx.x; i < heads * dim; i += blockDim.x) {
+    const int u = u0 + i / dim, e = i % dim;
     qr[(size_t)u * p.pitch + e] = from_f32<T>(q_at(u * (dim + rot) + e));
   }
   const int pad = p.pitch - dim - rot;
-  for (int i = threadIdx.x; i < p.heads * pad; i += blockDim.x) {
-    const int u = i / pad, e = i - u * pad;
+  for (int i = threadIdx.x; i < heads * pad; i += blockDim.x) {
+    const int u = u0 + i / pad, e = i % pad;
     qr[(size_t)u * p.pitch + dim + rot + e] = from_f32<T>(0.f);
   }
 }
@@ -1464,6 +1470,7 @@ AF_EXPORT int af_latent_prep(void* q, long long q_stride, const float* q_src, lo
   AF_REQUIRE(side_src == nullptr || (side != nullptr && side_n > 0 && side_w != nullptr),
              "af_latent_prep: bad sizes of the second latent");
   AF_REQUIRE(ring_rows % AF_PAGE == 0, "af_latent_prep: ring rows %d not whole pages", ring_rows);
+  const int blocks = q_src != nullptr && n_tokens <= 64 ? 1 + (heads < 4 ? heads : 4) : 1;       // (a prompt's tokens fill the chip)
 #define LATENT_PREP(T)                                                                                                  \
   do {                                                                                                                  \
     LatentPrepArgs<T> p;                                                                                                \
@@ -1475,7 +1482,7 @@ AF_EXPORT int af_latent_prep(void* q, long long q_stride, const float* q_src, lo
     p.table = (const float2*)table, p.positions = positions, p.seq_of_token = seq_of_token, p.slots = slots;            \
     p.len_after = len_after, p.kcache = (T*)kcache, p.page_table = page_table, p.max_pages = max_pages;                 \
     p.ring_rows = ring_rows;                                                                                            \
-    af_launch(latent_prep_kernel<T>, dim3(n_tokens), dim3(256), 0, stream, p);                                          \
+    af_launch(latent_prep_kernel<T>, dim3(n_tokens, blocks), dim3(256), 0, stream, p);                                          \
   } while (0)
   AF_DISPATCH_DTYPE(dtype, T, LATENT_PREP(T));
 #undef LATENT_PREP
