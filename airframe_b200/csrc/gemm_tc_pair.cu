@@ -1,6 +1,6 @@
 // The prefill matrix product on pairs of SMs:  out[M, N] = x[M, K] * w[N, K]^T  (bfloat16, 32-bit sums).
 //
-// Two blocks (a cluster of two, on neighbouring SMs) work on one tile of 256 weight rows by 256 tokens
+// Two blocks (a cluster of two, on neighbouring SMs) work on one tile of 256 weight rows by up to 256 tokens
 // with tcgen05.mma.cta_group::2: each block loads its own 128 weight rows (the "A" operand, the TMEM
 // lanes of its own accumulator) and its own 128 of the 256 tokens (half of the "B" operand); the tensor
 // cores of both SMs read both halves.  Against one block that does 256 x 256 alone this halves the
@@ -30,10 +30,9 @@ constexpr int TP_BN = 256;        // tokens per pair
 constexpr int TP_BK = 64;
 constexpr int TP_THREADS = 192;
 constexpr int TP_A_BYTES = TP_BM * TP_BK * 2;
-constexpr int TP_B_BYTES = (TP_BN / 2) * TP_BK * 2;
-constexpr int TP_STAGE_BYTES = TP_A_BYTES + TP_B_BYTES;
-constexpr int TP_STAGES = 6;
-constexpr int TP_SMEM = TP_STAGES * TP_STAGE_BYTES + 1024;
+constexpr int TP_BUDGET = 192 * 1024;
+constexpr int TP_MOST_STAGES = 8, TP_STAGES = 6;
+__host__ __device__ constexpr int tp_stage_bytes(int bn) { return TP_A_BYTES + bn / 2 * TP_BK * 2; }
 
 struct TpArgs {
   void* out;
@@ -43,6 +42,7 @@ struct TpArgs {
   float cap;
   int* err;
   int group;              // the order in which the pairs walk the tiles (af_tile_of)
+  int bn, stages;         // tokens of a tile (a multiple of 32 up to 256), stages of the ring
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -104,14 +104,15 @@ __device__ __forceinline__ float tp_act(float g, int act) {
   return 0.5f * g * (1.f + t);
 }
 
-template <int ACT, typename TO>
+template <int ACT, typename TO, bool ANY>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, TpArgs a) {
   constexpr bool GATED = ACT >= 0;
-  constexpr uint32_t IDESC = umma_idesc_pair(TP_BN);
+  const int bn = ANY ? a.bn : TP_BN, stages = ANY ? a.stages : TP_STAGES, stage_bytes = tp_stage_bytes(bn);
+  const uint32_t idesc = umma_idesc_pair(bn);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full[TP_STAGES], empty[TP_STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint64_t full[TP_MOST_STAGES], empty[TP_MOST_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int give_up_s;
   volatile int* give_up = &give_up_s;
@@ -125,7 +126,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const int n_tiles = a.tiles_w * a.tiles_m;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < TP_STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -156,15 +157,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       // is in its walk is counted on, not divided out stage by stage (this thread has a stage's copies to send
       // in the time its products take).
       struct Walk {
-        int kb, tile, wt, mt;
+        int kb, tile, wt, mt, s;
       };
       auto begin = [&](Walk& w) {
-        w.kb = 0;
+        w.kb = w.s = 0;
         w.tile = pair;
         w.wt = w.mt = 0;
         if (w.tile < n_tiles) af_tile_of(w.tile, a.tiles_w, a.tiles_m, a.group, &w.wt, &w.mt);
       };
       auto step = [&](Walk& w) {
+        if (++w.s == stages) w.s = 0;
         if (++w.kb == kb_count) {
           w.kb = 0;
           w.tile += n_pairs;
@@ -174,41 +176,42 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       Walk ww, wx;
       begin(ww);
       begin(wx);
-      auto load_w = [&](int it) {
+      auto load_w = [&]() {
         const int n0 = ww.wt * (2 * TP_BM) + (int)rank * TP_BM;
-        tma_load_2d_pair(tiles + (size_t)(it % TP_STAGES) * TP_STAGE_BYTES, &map_w, ww.kb * TP_BK, n0,
-                         map_to_rank(smem_u32(&full[it % TP_STAGES]), 0));
+        tma_load_2d_pair(tiles + (size_t)ww.s * stage_bytes, &map_w, ww.kb * TP_BK, n0, map_to_rank(smem_u32(&full[ww.s]), 0));
         step(ww);
       };
-      auto load_x = [&](int it) {
-        const int m0 = wx.mt * TP_BN + (int)rank * (TP_BN / 2);
-        tma_load_2d_pair(tiles + (size_t)(it % TP_STAGES) * TP_STAGE_BYTES + TP_A_BYTES, &map_x, wx.kb * TP_BK,
-                         m0, map_to_rank(smem_u32(&full[it % TP_STAGES]), 0));
+      auto load_x = [&]() {
+        const int m0 = wx.mt * bn + (int)rank * (bn / 2);
+        tma_load_2d_pair(tiles + (size_t)wx.s * stage_bytes + TP_A_BYTES, &map_x, wx.kb * TP_BK, m0,
+                         map_to_rank(smem_u32(&full[wx.s]), 0));
         step(wx);
       };
       // The weights do not depend on the kernel in front: the first stages' weight tiles go out before the
       // wait for it, the activations after it.
-      const int early = total < TP_STAGES ? total : TP_STAGES;
+      const int early = total < stages ? total : stages;
       for (int it = 0; it < early; ++it) {
-        if (leader) mbar_expect_tx(&full[it], 2 * TP_STAGE_BYTES);
-        load_w(it);
+        if (leader) mbar_expect_tx(&full[it], 2 * stage_bytes);
+        load_w();
       }
       pdl_wait();
-      for (int it = 0; it < early; ++it) load_x(it);
-      for (int it = early; it < total; ++it) {
-        const int s = it % TP_STAGES;
-        const uint32_t ph = (it / TP_STAGES) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1, give_up)) break;
-        if (leader) mbar_expect_tx(&full[s], 2 * TP_STAGE_BYTES);
-        load_w(it);
-        load_x(it);
+      for (int it = 0; it < early; ++it) load_x();
+      uint32_t ph = 0;
+      for (int it = early; it < total; ++it) {     // (more than `stages` of them: the ring stands at its first stage again)
+        const int s = wx.s;
+        if (!mbar_wait(&empty[s], ph, give_up)) break;
+        if (s == stages - 1) ph ^= 1;
+        if (leader) mbar_expect_tx(&full[s], 2 * stage_bytes);
+        load_w();
+        load_x();
       }
       if (*give_up) grace_period();
     }
   } else if (warp == 1) {
     if (lane == 0 && leader) {
       bool ok = true;
-      int it = 0, round = 0;
+      int s = 0, round = 0;
+      uint32_t ph = 0;
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++round) {
         const int buf = round & 1;
         // the accumulator is free once the epilogue warps of both blocks have read the tile two rounds back
@@ -217,20 +220,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           break;
         }
         tc_fence_after();
-        for (int kb = 0; kb < kb_count; ++kb, ++it) {
-          const int s = it % TP_STAGES;
-          const uint32_t ph = (it / TP_STAGES) & 1;
+        for (int kb = 0; kb < kb_count; ++kb) {
           if (!mbar_wait(&full[s], ph, give_up)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t st = smem_u32(tiles + (size_t)s * TP_STAGE_BYTES);
+          const uint32_t st = smem_u32(tiles + (size_t)s * stage_bytes);
           const uint64_t da = umma_desc(st), db = umma_desc(st + TP_A_BYTES);
 #pragma unroll
           for (int k = 0; k < TP_BK / 16; ++k)
-            umma_f16_pair(tmem_base + buf * TP_BN, da + 2 * k, db + 2 * k, IDESC, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_f16_pair(tmem_base + buf * TP_BN, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           umma_commit_pair(&empty[s]);
+          if (++s == stages) s = 0, ph ^= 1;
         }
         if (ok) umma_commit_pair(&acc_full[buf]);
       }
@@ -245,7 +247,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       int wt2, mt;
       af_tile_of(tile, a.tiles_w, a.tiles_m, a.group, &wt2, &mt);
       const int wt = wt2 * 2 + (int)rank;                      // this block's tile of 128 weight rows
-      const int m0 = mt * TP_BN;
+      const int m0 = mt * bn, m_end = min(a.M, m0 + bn);
       if (!mbar_wait(&acc_full[buf], (round >> 1) & 1, give_up)) break;
       tc_fence_after();
       TO* out = reinterpret_cast<TO*>(a.out);
@@ -253,12 +255,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       const int f = GATED ? wt * 64 + quarter * 16 + (lane & 15) : wt * TP_BM + quarter * 32 + lane;
       constexpr int CW = 64;
 #pragma unroll 1
-      for (int c0 = 0; c0 < TP_BN; c0 += CW) {
+      for (int c0 = 0; c0 < bn; c0 += CW) {        // (columns that a round reads beyond bn are never stored)
         float v[CW];
         tmem_ld32(lane_base + c0, v);
         tmem_ld32(lane_base + c0 + 32, v + 32);
         tmem_wait_ld();
-        if (c0 + CW >= TP_BN) {
+        if (c0 + CW >= bn) {
           // all of this tile is in registers: its accumulator may be written again
           tc_fence_before();
           __syncwarp();
@@ -279,7 +281,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             TO* o = out + (size_t)tok0 * a.ldo + f;
 #pragma unroll
             for (int j = 0; j < CW / 2; ++j)
-              if (tok0 + j < a.M) o[(size_t)j * a.ldo] = from_f32<TO>(v[j]);
+              if (tok0 + j < m_end) o[(size_t)j * a.ldo] = from_f32<TO>(v[j]);
           }
         } else {
           if (a.cap > 0.f) {
@@ -288,13 +290,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           }
           if (f < a.N) {
             TO* o = out + (size_t)(m0 + c0) * a.ldo + f;
-            if (m0 + c0 + CW <= a.M) {
+            if (m0 + c0 + CW <= m_end) {
 #pragma unroll
               for (int j = 0; j < CW; ++j) o[(size_t)j * a.ldo] = from_f32<TO>(v[j]);
             } else {
 #pragma unroll
               for (int j = 0; j < CW; ++j)
-                if (m0 + c0 + j < a.M) o[(size_t)j * a.ldo] = from_f32<TO>(v[j]);
+                if (m0 + c0 + j < m_end) o[(size_t)j * a.ldo] = from_f32<TO>(v[j]);
             }
           }
         }
@@ -310,25 +312,35 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   if (threadIdx.x == 0 && give_up_s && a.err) atomicExch(a.err, 1);
 }
 
-template <int ACT, typename TO>
-int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, TpArgs a, long long n_w_rows, cudaStream_t stream) {
+template <int ACT, typename TO, bool ANY>
+int launch_pair_tile(const CUtensorMap& mw, const CUtensorMap& mx, TpArgs a, long long n_w_rows, cudaStream_t stream) {
   static bool configured[AF_MAX_DEVICES] = {};
   const int dev = af_current_device();
   if (dev < 0) return -1;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<ACT, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<ACT, TO, ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         TP_BUDGET + 1024);
     if (e != cudaSuccess) return af_fail((int)e, "af_gemm_tc_pair: %s", cudaGetErrorString(e));
     configured[dev] = true;
   }
   a.tiles_w = (int)((n_w_rows + 2 * TP_BM - 1) / (2 * TP_BM));
-  a.tiles_m = (a.M + TP_BN - 1) / TP_BN;
+  a.tiles_m = (a.M + a.bn - 1) / a.bn;
+  a.stages = TP_BUDGET / tp_stage_bytes(a.bn);
+  if (a.stages > TP_MOST_STAGES) a.stages = TP_MOST_STAGES;
   const long long tiles = (long long)a.tiles_w * a.tiles_m;
   const int sms = af_sm_count();
   if (sms <= 0) return -1;
   const long long pairs = tiles < sms / 2 ? tiles : sms / 2;
   a.group = af_tile_group(a.tiles_m, sms / 2);
-  af_launch(gemm_tc_pair_kernel<ACT, TO>, dim3((unsigned)(2 * pairs)), dim3(TP_THREADS), TP_SMEM, stream, mw, mx, a);
+  af_launch(gemm_tc_pair_kernel<ACT, TO, ANY>, dim3((unsigned)(2 * pairs)), dim3(TP_THREADS), a.stages * tp_stage_bytes(a.bn) + 1024, stream, mw, mx, a);
   AF_CHECK_LAUNCH("af_gemm_tc_pair");
+}
+
+// (tiles of 256 tokens keep their constants, as in gemm_tc.cu)
+template <int ACT, typename TO>
+int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const TpArgs& a, long long n_w_rows, cudaStream_t stream) {
+  return a.bn == TP_BN ? launch_pair_tile<ACT, TO, false>(mw, mx, a, n_w_rows, stream)
+                       : launch_pair_tile<ACT, TO, true>(mw, mx, a, n_w_rows, stream);
 }
 
 }  // namespace
@@ -336,10 +348,10 @@ int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, TpArgs a, long lon
 // out = x w^T on pairs of SMs (see the top of the file); meant for many tokens (prompts).  x [M, K] and
 // w [n_w_rows, K] bfloat16 with dense rows (strides multiples of 8, bases 16-byte aligned).  gated != 0: w holds
 // groups of 16 gate rows + 16 up rows, N = n_w_rows / 2, out = act(x . gate) * (x . up).  out: bfloat16 or float
-// [M, N], rows ldo apart.  err: device word set to 1 when a wait inside the kernel ran out of time.
+// [M, N], rows ldo apart.  token_tile: tokens of a pair's tile, a multiple of 32 up to 256 (0: 256).  err: device word set to 1 when a wait inside the kernel ran out of time.
 AF_EXPORT int af_gemm_tc_pair(void* out, int out_dtype, long long ldo, const void* x, long long ldx, const void* w,
                               long long ldw, long long n_w_rows, int M, int K, int gated, int act, float cap,
-                              int* err, cudaStream_t stream) {
+                              int token_tile, int* err, cudaStream_t stream) {
   if (M == 0 || n_w_rows == 0) return 0;
   AF_REQUIRE(M > 0 && n_w_rows > 0 && K > 0, "af_gemm_tc_pair: bad sizes %d %lld %d", M, n_w_rows, K);
   AF_REQUIRE(K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0, "af_gemm_tc_pair: K %d and row strides must be multiples of 8", K);
@@ -347,13 +359,16 @@ AF_EXPORT int af_gemm_tc_pair(void* out, int out_dtype, long long ldo, const voi
   AF_REQUIRE(!gated || n_w_rows % 32 == 0, "af_gemm_tc_pair: a gated weight holds whole groups of 16 + 16 rows");
   AF_REQUIRE(!gated || act == AF_ACT_GELU_TANH || act == AF_ACT_SILU, "af_gemm_tc_pair: unknown activation %d", act);
   AF_REQUIRE(!(gated && cap > 0.f), "af_gemm_tc_pair: the gated variant takes no cap");
+  const int bn = token_tile > 0 ? token_tile : TP_BN;
+  AF_REQUIRE(bn % 32 == 0 && bn <= TP_BN, "af_gemm_tc_pair: token tile %d", bn);
   CUtensorMap mw, mx;
   int rc = af_make_map_bf16(&mw, w, n_w_rows, K, ldw, TP_BM);
   if (rc) return rc;
-  rc = af_make_map_bf16(&mx, x, M, K, ldx, TP_BN / 2);
+  rc = af_make_map_bf16(&mx, x, M, K, ldx, bn / 2);
   if (rc) return rc;
   const int N = gated ? (int)(n_w_rows / 2) : (int)n_w_rows;
   TpArgs a{out, ldo, M, N, K, 0, 0, cap, err};
+  a.bn = bn;
   const bool bf = out_dtype == AF_BF16;
   AF_REQUIRE(bf || out_dtype == AF_F32, "af_gemm_tc_pair: out dtype %d", out_dtype);
   if (gated && act == AF_ACT_GELU_TANH)

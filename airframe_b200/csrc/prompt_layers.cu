@@ -7,9 +7,7 @@
 extern "C" {
 int af_gemm_tc(void* out, int out_dtype, long long ldo, long long part_stride, const void* x, long long ldx, const void* w,
                long long ldw, long long n_w_rows, int M, int K, int gated, int act, int n_acc, float cap, int splits, int per_sm,
-               int* err, cudaStream_t stream);
-int af_gemm_tc_pair(void* out, int out_dtype, long long ldo, const void* x, long long ldx, const void* w, long long ldw,
-                    long long n_w_rows, int M, int K, int gated, int act, float cap, int* err, cudaStream_t stream);
+               int token_tile, int* err, cudaStream_t stream);
 int af_rope_cache_write(void* qkv, int dtype, int row_stride, const float* parts, int n_parts, long long part_stride,
                         const int* positions, const int* seq_of_token, const int* slots, const int* len_after,
                         const float* inv_freq, const float* table, int n_tokens, int nq, int nkv, int hd, int rot_dim,
@@ -45,20 +43,18 @@ struct PromptStep {
   const int *positions, *seq_of_token, *slots, *len_after, *seq_starts;
   int* err;
   long long T, H, nq, nkv, hd, rot_dim, pairing, inter, act, n_seqs, max_len;
-  long long splits[3], accs[4];     // of the products q k v, o, down; and of gate and up
+  long long splits[3];              // of the products q k v, o, down
   double offset;
 };
 
 // One product into `out`, or into partial sums.
-int prompt_product(const PromptStep& s, void* out, const void* x, const void* w, long long rows, int K, int splits, int accs,
-                   bool gated, cudaStream_t stream) {
+int prompt_product(const PromptStep& s, void* out, const void* x, const void* w, long long rows, int K, int splits, bool gated,
+                   cudaStream_t stream) {
   const int M = (int)s.T, per_sm = 0;
   const long long N = gated ? rows / 2 : rows;
   if (splits > 1)
-    return af_gemm_tc(s.parts, AF_F32, N, (long long)M * N, x, K, w, K, rows, M, K, 0, 0, accs, 0.f, splits, per_sm, s.err, stream);
-  if (accs == 4)
-    return af_gemm_tc_pair(out, AF_BF16, N, x, K, w, K, rows, M, K, gated ? 1 : 0, (int)s.act, 0.f, s.err, stream);
-  return af_gemm_tc(out, AF_BF16, N, 0, x, K, w, K, rows, M, K, gated ? 1 : 0, (int)s.act, accs, 0.f, 1, per_sm, s.err, stream);
+    return af_gemm_tc(s.parts, AF_F32, N, (long long)M * N, x, K, w, K, rows, M, K, 0, 0, 0, 0.f, splits, per_sm, 0, s.err, stream);
+  return af_gemm_tc(out, AF_BF16, N, 0, x, K, w, K, rows, M, K, gated ? 1 : 0, (int)s.act, 0, 0.f, 1, per_sm, 0, s.err, stream);
 }
 
 }  // namespace
@@ -74,7 +70,7 @@ AF_EXPORT int af_prompt_layers(const void* step, const void* runs, int n_runs, c
   const float offset = (float)s.offset;
   for (int i = 0; i < n_runs; ++i) {
     const PromptRun& r = all[i];
-    int e = prompt_product(s, s.qkv, s.h, r.w_qkv, W, H, (int)s.splits[0], (int)s.accs[0], false, stream);
+    int e = prompt_product(s, s.qkv, s.h, r.w_qkv, W, H, (int)s.splits[0], false, stream);
     if (e) return e;
     const bool joined = s.splits[0] > 1;
     e = af_rope_cache_write(s.qkv, AF_BF16, W, joined ? s.parts : nullptr, joined ? (int)s.splits[0] : 0,
@@ -86,7 +82,7 @@ AF_EXPORT int af_prompt_layers(const void* step, const void* runs, int n_runs, c
                            (int)s.n_seqs, T, (int)s.max_len, nq, nkv, hd, (float)r.scale, (float)r.cap, (int)r.window,
                            r.window ? (int)r.keep : 0, nullptr, nullptr, 0, s.err, stream);
     if (e) return e;
-    e = prompt_product(s, s.a, s.ctx, r.w_o, H, nq * hd, (int)s.splits[1], (int)s.accs[1], false, stream);
+    e = prompt_product(s, s.a, s.ctx, r.w_o, H, nq * hd, (int)s.splits[1], false, stream);
     if (e) return e;
     auto add = [&](long long splits, const float* post, double eps_post, const float* next, double eps_next) {
       const bool sums = splits > 1;
@@ -96,9 +92,9 @@ AF_EXPORT int af_prompt_layers(const void* step, const void* runs, int n_runs, c
     };
     e = add(s.splits[1], r.n_post_mixer, r.eps_post_mixer, r.n_pre_ff, r.eps_pre_ff);
     if (e) return e;
-    e = prompt_product(s, s.mid, s.h, r.w_gu, 2ll * inter, H, 1, (int)s.accs[3], true, stream);
+    e = prompt_product(s, s.mid, s.h, r.w_gu, 2ll * inter, H, 1, true, stream);
     if (e) return e;
-    e = prompt_product(s, s.a, s.mid, r.w_down, H, inter, (int)s.splits[2], (int)s.accs[2], false, stream);
+    e = prompt_product(s, s.a, s.mid, r.w_down, H, inter, (int)s.splits[2], false, stream);
     if (e) return e;
     e = add(s.splits[2], r.n_post_ff, r.eps_post_ff, r.n_next, r.eps_next);
     if (e) return e;

@@ -536,29 +536,12 @@ def gemm_tc_splits(M: int, N: int, K: int) -> int:
     return (kb + per - 1) // per
 
 
-def gemm_tc_accumulators(M: int, rows: int, K: int, splits: int) -> int:
-    """Weight tiles a block of the product works at once: 1, 2, or 4 for the kernel on pairs of SMs.
-
-    Many tokens: two weight tiles per block halve the bytes a block stages per flop; worth it once the
-    tiles of 256 x 256 fill the GPU.  With fewer tiles and a long K a tile runs on a pair of SMs (the same
-    bytes per flop, 128 rows a block); with a short K the pair's set-up costs what it saves.  Measured at
-    2,048 tokens on a B200: 18432 x 2304 gated 122 us / 124 us / 132 us (two tiles / pair / one tile),
-    2304 x 9216 90 / 59 / 63, 2304 x 2048 25 / 17 / 15, 4096 x 2304 31 / 31 / 31."""
-    if M > 128 and splits == 1:
-        blocks2 = ((rows + 255) // 256) * ((M + 255) // 256)
-        if blocks2 >= 120:
-            return 2
-        if blocks2 >= 60 and K >= 4096:
-            return 4
-    return 1
-
-
 # Blocks per SM of the weight-bound product (up to 64 tokens): 0 lets the library choose.
 GEMM_TC_PER_SM = 0
 
 
 def gemm_tc(out, x, w, cap: float = 0.0, splits: int = 1, gated: bool = False, activation: str = "gelu_tanh",
-            n_acc: int = 0, checked: bool = False, per_sm: int = -1) -> None:
+            n_acc: int = 0, checked: bool = False, per_sm: int = -1, token_tile: int = 0) -> None:
     """out = x @ w^T on the tcgen05 tensor cores (bfloat16 operands, 32-bit
     accumulation in TMEM).  splits > 1: out is float32 [splits, M, N] partial
     sums.  gated: w holds, per group of 32 rows, 16 gate rows then the 16 up
@@ -566,7 +549,8 @@ def gemm_tc(out, x, w, cap: float = 0.0, splits: int = 1, gated: bool = False, a
     act(x . gate_f) * (x . up_f), N = rows / 2.  n_acc: weight tiles per block
     (1 or 2), or 4: the kernel that runs a tile on a pair of SMs
     (``tcgen05.mma.cta_group::2``, two accumulators in turn: for prompts);
-    0: chosen from the sizes.  ``checked``: the caller has asked
+    0: chosen from the sizes, with the tokens of a tile unless ``token_tile`` says them
+    (a multiple of 16 up to 256, on pairs of 32).  ``checked``: the caller has asked
     :func:`gemm_tc_supported` already."""
     M, K = x.shape
     rows = w.shape[0]
@@ -581,21 +565,19 @@ def gemm_tc(out, x, w, cap: float = 0.0, splits: int = 1, gated: bool = False, a
         if tuple(out.shape) != (M, N):
             raise KernelError(f"gemm_tc: output shape {tuple(out.shape)}, expected {(M, N)}")
         ldo, part = out.stride(0), 0
-    if n_acc == 0:
-        n_acc = gemm_tc_accumulators(M, rows, K, splits)
     if n_acc == 4:
         if splits > 1:
             raise KernelError("gemm_tc: the kernel on pairs of SMs does not split K")
         _check(_lib().af_gemm_tc_pair(_ptr(out), c_int(dtype_code(out.dtype)), c_longlong(ldo), _ptr(x),
                                       c_longlong(x.stride(0)), _ptr(w), c_longlong(w.stride(0)), c_longlong(rows),
                                       c_int(M), c_int(K), c_int(1 if gated else 0), c_int(ACTIVATIONS[activation]),
-                                      c_float(cap), _ptr(error_word(x.device), "err", torch.int32), _stream()))
+                                      c_float(cap), c_int(token_tile), _ptr(error_word(x.device), "err", torch.int32), _stream()))
         return
     _check(_lib().af_gemm_tc(_ptr(out), c_int(dtype_code(out.dtype)), c_longlong(ldo), c_longlong(part), _ptr(x),
                              c_longlong(x.stride(0)), _ptr(w), c_longlong(w.stride(0)), c_longlong(rows),
                              c_int(M), c_int(K), c_int(1 if gated else 0), c_int(ACTIVATIONS[activation]),
                              c_int(n_acc), c_float(cap), c_int(splits), c_int(GEMM_TC_PER_SM if per_sm < 0 else per_sm),
-                             _ptr(error_word(x.device), "err", torch.int32), _stream()))
+                             c_int(token_tile), _ptr(error_word(x.device), "err", torch.int32), _stream()))
 
 
 def rope_table(positions, inv_freq) -> torch.Tensor:

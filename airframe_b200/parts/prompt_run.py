@@ -20,7 +20,7 @@ from .norm import RmsNorm
 from .rope import Rope
 
 _RUN = struct.Struct("<13Q4q6d")
-_STEP = struct.Struct("<13Q18qd")
+_STEP = struct.Struct("<13Q14qd")
 
 
 def _matrix(w, rows: int, cols: int) -> bool:
@@ -73,8 +73,6 @@ def run(model, x, batch, cache) -> bool:
     T, H, W, N = x.shape[0], m.hidden, m.w_qkv.shape[0], m.nq * m.hd
     products = ((W, H), (H, N), (H, f.inter))
     splits = [kernels.gemm_tc_splits(T, rows, K) for rows, K in products]
-    accs = [kernels.gemm_tc_accumulators(T, rows, K, s) for (rows, K), s in zip(products, splits)]
-    accs.append(kernels.gemm_tc_accumulators(T, 2 * f.inter, H, 1))
     h = first.norms["pre_mixer"].forward(x, torch.bfloat16)
     qkv, ctx, mid, a = (torch.empty(T, n, dtype=torch.bfloat16, device=x.device) for n in (W, N, f.inter, H))
     room = max((s * T * rows for (rows, _), s in zip(products, splits) if s > 1), default=0)
@@ -99,6 +97,6 @@ def run(model, x, batch, cache) -> bool:
         *(t.data_ptr() for t in (batch.positions, batch.seq_of_token, batch.slots, batch.len_after, batch.seq_starts)),
         kernels.error_word(x.device).data_ptr(), T, H, m.nq, m.nkv, m.hd, m.position.rotary_dim,
         kernels.PAIRINGS[m.position.pairing], f.inter, kernels.ACTIVATIONS[f.activation], batch.n_seqs, batch.max_len,
-        *splits, *accs, first.norms["pre_mixer"].offset)
+        *splits, first.norms["pre_mixer"].offset)
     kernels.prompt_layers(step, bytes(runs), len(blocks))
     return True
