@@ -220,9 +220,10 @@ class SequenceCache:
         slot = self.slots.take()
         self.lens[slot] = 0
         self.room[slot] = 0
-        for st in self.states.values():
-            if st is not None:
-                st[slot].zero_()
+        # (one launch for all layers' rows: 32 of them cost a step of prompts 39 us of the device and some 0.2 ms of the host)
+        held = [st[slot] for st in self.states.values() if st is not None]
+        if held:
+            torch._foreach_zero_(held)
         return slot
 
     def free_slot(self, slot: int) -> None:
