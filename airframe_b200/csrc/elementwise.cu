@@ -247,8 +247,9 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const TA* __restrict__
 // The same for rows of up to 8192 elements with hidden % 4 == 0: a thread owns NV groups of four
 // elements (group v of thread t at element 4 (t + v * threads)), every load issued before the first
 // reduction.  Few rows (decode): NV = 1, many threads per row, what costs is the chain of memory
-// latencies: the row of the stream is asked for with the first partial sums (all sixteen of a long product's at once would
-// take the registers that let the block stand by beside the product in front: 1,674 -> 1,695 us a step at batch 8); many rows (prefill): NV = 2, smaller blocks, more rows in flight on an SM.
+// latencies (all sixteen partial sums of a long product asked for at once would take the registers that let the block stand by
+// beside the product in front: 1,674 -> 1,695 us a step at batch 8; the stream's row before the sums 1,672 -> 1,680); many rows
+// (prefill): NV = 2, smaller blocks, more rows in flight on an SM.
 // MANY (the rows of a prompt): the kernel is bound by how many rows an SM holds at a time, so it keeps to 32
 // registers (seven blocks of a 2304-wide row per SM instead of four) and reads the norms' weights, which
 // every row shares and the L1 holds, where it uses them instead of keeping them from the start.
@@ -286,11 +287,6 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
     const int i = (threadIdx.x + v * blockDim.x) * 4;
     if (!on[v]) continue;
     const size_t at = (size_t)r * hidden + i;
-    auto stream = [&] {
-      const float4 xt = *reinterpret_cast<const float4*>(x + at);
-      xv[v][0] = xt.x, xv[v][1] = xt.y, xv[v][2] = xt.z, xv[v][3] = xt.w;
-    };
-    if (!MANY) stream();
     if constexpr (sizeof(TA) == 4) {
       const float4 t = sum_parts4<MANY ? 1 : 8>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
       av[v][0] = t.x, av[v][1] = t.y, av[v][2] = t.z, av[v][3] = t.w;
@@ -301,7 +297,8 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
       av[v][2] = __uint_as_float(raw.y << 16);
       av[v][3] = __uint_as_float(raw.y & 0xffff0000u);
     }
-    if (MANY) stream();
+    const float4 xt = *reinterpret_cast<const float4*>(x + at);
+    xv[v][0] = xt.x, xv[v][1] = xt.y, xv[v][2] = xt.z, xv[v][3] = xt.w;
   }
   float ss = 0.f;
 #pragma unroll

@@ -18,8 +18,7 @@ struct AfHcTerm {
   float scale;
 };
 
-// IN: partial sums in flight at once.
-template <int VEC, int IN>
+template <int VEC>
 __device__ __forceinline__ void hc_term_add(float* acc, const AfHcTerm& t, size_t part_stride, size_t at) {
   if (t.p == nullptr) return;
   if (t.dtype == AF_BF16) {
@@ -37,12 +36,15 @@ __device__ __forceinline__ void hc_term_add(float* acc, const AfHcTerm& t, size_
   }
   const float* f = static_cast<const float*>(t.p) + at;
   float v[VEC];
-  if (VEC == 4) {
-    const float4 q = sum_parts4<IN>(f, t.parts, part_stride);
-    v[0] = q.x, v[1 % VEC] = q.y, v[2 % VEC] = q.z, v[3 % VEC] = q.w;
-  } else {
-    v[0] = 0.f;
-    for (int s = 0; s < t.parts; ++s) v[0] += f[(size_t)s * part_stride];
+#pragma unroll
+  for (int u = 0; u < VEC; ++u) v[u] = 0.f;
+  for (int s = 0; s < t.parts; ++s) {
+    if (VEC == 4) {
+      const float4 q = *reinterpret_cast<const float4*>(f + (size_t)s * part_stride);
+      v[0] += q.x, v[1 % VEC] += q.y, v[2 % VEC] += q.z, v[3 % VEC] += q.w;
+    } else {
+      v[0] += f[(size_t)s * part_stride];
+    }
   }
 #pragma unroll
   for (int u = 0; u < VEC; ++u) acc[u] += t.scale * v[u];
@@ -62,15 +64,6 @@ template <int VEC>
 __device__ __forceinline__ void hc_store(float* p, const float* v) {
   if (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1 % VEC], v[2 % VEC], v[3 % VEC]);
   else p[0] = v[0];
-}
-template <int VEC>
-__device__ __forceinline__ void hc_store(__nv_bfloat16* p, const float* v) {
-  if (VEC == 4) {
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1 % VEC]), hi = __floats2bfloat162_rn(v[2 % VEC], v[3 % VEC]);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-  } else {
-    p[0] = __float2bfloat16_rn(v[0]);
-  }
 }
 
 // y[t] = norm(sum_s in[s] x[t][s]) (offset + w)
@@ -120,21 +113,13 @@ hc_write_kernel(float* __restrict__ x, AfHcTerm a, AfHcTerm b, size_t part_strid
                 const float* __restrict__ w_next, float eps, float offset, TY* __restrict__ y, int S, int W) {
   pdl_launch_dependents();
   extern __shared__ float row[];
-  __shared__ float scratch[32];
+  __shared__ float scratch[33];
   __shared__ float cmix[AF_HC_MAX * AF_HC_MAX], cout[AF_HC_MAX], cin[AF_HC_MAX];
   for (int i = threadIdx.x; i < S * S; i += blockDim.x) cmix[i] = mix[i];      // (a block may have fewer threads than S * S)
   if (threadIdx.x < S) {
     cout[threadIdx.x] = out_w[threadIdx.x];
     cin[threadIdx.x] = in_next != nullptr ? in_next[threadIdx.x] : 0.f;
   }
-  // the first group's weights, for most widths the only one's, are on their way before the wait
-  const int i0 = threadIdx.x * VEC;
-  const bool once = SMAX > 4 && W <= (int)blockDim.x * VEC;      // (many tokens: no registers for it)
-  float l0[VEC], w0[VEC], u0[VEC];
-#pragma unroll
-  for (int e = 0; e < VEC; ++e) l0[e] = w0[e] = u0[e] = 0.f;
-  if (i0 < W && ls != nullptr) hc_load<VEC>(l0, ls + i0);
-  if (i0 < W && y != nullptr && once) hc_load<VEC>(w0, w_next + i0);
   pdl_wait();
   x = pdl_fresh(x);
   a.p = pdl_fresh(a.p);
@@ -144,20 +129,21 @@ hc_write_kernel(float* __restrict__ x, AfHcTerm a, AfHcTerm b, size_t part_strid
   float* xt = x + t * S * W;
   float ss = 0.f;
   for (int i = threadIdx.x * VEC; i < W; i += blockDim.x * VEC) {
+    float yv[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) yv[e] = 0.f;
+    hc_term_add<VEC>(yv, a, part_stride, t * W + i);
+    hc_term_add<VEC>(yv, b, part_stride, t * W + i);
+    if (ls != nullptr) {
+      float l[VEC];
+      hc_load<VEC>(l, ls + i);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) yv[e] *= l[e];
+    }
     float xs[SMAX][VEC];
 #pragma unroll
     for (int s = 0; s < SMAX; ++s)
       if (s < S) hc_load<VEC>(xs[s], xt + (size_t)s * W + i);
-    float yv[VEC];
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) yv[e] = 0.f;
-    hc_term_add<VEC, SMAX <= 4 ? 1 : 8>(yv, a, part_stride, t * W + i);
-    hc_term_add<VEC, SMAX <= 4 ? 1 : 8>(yv, b, part_stride, t * W + i);
-    if (ls != nullptr) {
-      if (i != i0) hc_load<VEC>(l0, ls + i);
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) yv[e] *= l0[e];
-    }
     float u[VEC];
 #pragma unroll
     for (int e = 0; e < VEC; ++e) u[e] = 0.f;
@@ -184,24 +170,14 @@ hc_write_kernel(float* __restrict__ x, AfHcTerm a, AfHcTerm b, size_t part_strid
     if (y != nullptr) {
 #pragma unroll
       for (int e = 0; e < VEC; ++e) {
-        if (once) u0[e] = u[e];
-        else row[i + e] = u[e];
+        row[i + e] = u[e];
         ss += u[e] * u[e];
       }
     }
   }
   if (y == nullptr) return;
-  ss = block_sum<true>(ss, scratch);
+  ss = block_sum(ss, scratch);
   const float inv = rsqrtf(ss / (float)W + eps);
-  if (once) {
-    if (i0 < W) {
-      float o[VEC];
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) o[e] = u0[e] * inv * (offset + w0[e]);
-      hc_store<VEC>(y + t * W + i0, o);
-    }
-    return;
-  }
   for (int i = threadIdx.x; i < W; i += blockDim.x) y[t * W + i] = from_f32<TY>(row[i] * inv * (offset + w_next[i]));
 }
 
@@ -270,7 +246,7 @@ AF_EXPORT int af_hc_write(float* x, const void* a, int a_dtype, int a_parts, flo
   AF_REQUIRE((size_t)W * sizeof(float) <= 48 * 1024, "af_hc_write: rows of up to 12288 values");
   const AfHcTerm ta{a, a_dtype, a_parts, scale_a}, tb{b, b_dtype, b_parts, scale_b};
   const size_t part_stride = (size_t)n_tokens * W;
-  const bool vec = W % 4 == 0 && (((uintptr_t)x | (uintptr_t)a | (uintptr_t)b | (uintptr_t)ls | (uintptr_t)w_next | (uintptr_t)y) & 15) == 0;
+  const bool vec = W % 4 == 0 && (((uintptr_t)x | (uintptr_t)a | (uintptr_t)b | (uintptr_t)ls) & 15) == 0;
   const size_t smem = y != nullptr ? (size_t)W * sizeof(float) : 0;
 #define AF_HC_LAUNCH(VEC_, SMAX_)                                                                                      \
   AF_DISPATCH_DTYPE(y_dtype, TY,                                                                                       \
