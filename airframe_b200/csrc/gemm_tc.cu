@@ -219,6 +219,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           first = false;
         }
         for (; kb < kb_count; ++kb, ++it) {
+          if constexpr (!WIDE) s = it % MOST, ph = (it / MOST) & 1;
           if (it >= STAGES && !mbar_wait(&empty[s], ph ^ 1, give_up)) break;
           unsigned char* st = tiles + (size_t)s * STAGE_BYTES;
           mbar_expect_tx(&full[s], STAGE_BYTES);
@@ -229,7 +230,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             else tma_load_2d(st + acc * A_BYTES, &map_w, k, n0 + acc * TC_BM, &full[s]);
           }
           tma_load_2d(st + NACC * A_BYTES, &map_x, k, m0, &full[s]);
-          if (++s == STAGES) s = 0, ph ^= 1;
+          if (WIDE && ++s == STAGES) s = 0, ph ^= 1;
         }
       }
       if (first) pdl_wait();
@@ -238,7 +239,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   } else if (warp == 1) {
     if (lane == 0) {
       bool ok = true;
-      int s = 0, round = 0;
+      int it = 0, s = 0, round = 0;
       uint32_t ph = 0;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++round) {
         // an accumulator is free once the epilogue warps have read the tile before out of it
@@ -248,7 +249,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = 0; kb < kb_count; ++kb) {
+        for (int kb = 0; kb < kb_count; ++kb, ++it) {
+          if constexpr (!WIDE) s = it % MOST, ph = (it / MOST) & 1;
           if (!mbar_wait(&full[s], ph, give_up)) {
             ok = false;
             break;
@@ -264,7 +266,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
               umma_f16(tmem_base + (turn * NACC + acc) * BN, umma_desc(st + acc * A_BYTES) + 2 * k, db + 2 * k, IDESC, accum);
           }
           umma_commit(&empty[s]);
-          if (++s == STAGES) s = 0, ph ^= 1;
+          if (WIDE && ++s == STAGES) s = 0, ph ^= 1;
         }
         if (ok) umma_commit(&acc_full[turn]);
       }
@@ -277,7 +279,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++round) {
       int tile_w, mt;
       af_tile_of(tile, a.tiles_w, a.tiles_m, a.group, &tile_w, &mt);
-      const int m0 = mt * bn, m_end = min(a.M, m0 + bn);
+      const int m0 = mt * bn, m_end = WIDE ? min(a.M, m0 + bn) : a.M;
       const int turn = round % TURNS;
       if (!mbar_wait(&acc_full[turn], (round / TURNS) & 1, give_up)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
