@@ -69,6 +69,8 @@ attn_decode_latent_kernel(const __nv_bfloat16* __restrict__ q, long long q_strid
     hi = min(pos, lo + per - 1);
   }
   pdl_wait();
+  q = pdl_fresh(q);
+  kcache = pdl_fresh(kcache);
   // ---- the queries of the tile's heads (rows of heads that are not there: zeros)
   const int pieces = dk / 8;
   for (int i = tid; i < 16 * pieces; i += blockDim.x) {

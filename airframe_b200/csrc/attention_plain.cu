@@ -1030,6 +1030,8 @@ qk_norm_rope_store_kernel(T* __restrict__ qkv, long long out_stride, const float
     qk_cache_rows(kcache, vcache, seq_of_token, slots, len_after, page_table, max_pages, ring_rows, keep, nkv, t, pos,
                   head - nq, pk, pv, &kdst, &vdst);
   pdl_wait();
+  proj = pdl_fresh(proj);
+  table = pdl_fresh(table);
   qk_pack_head(qkv, out_stride, proj, ld, bias, head >= nq ? k_weight : q_weight, false, 1.f, eps, norm_after, magnitude,
                v_from_k, inv_freq, table, nq, nkv, hd, dv, rot_dim, pairing, pk, pv, t, head, pos, lane, kdst, vdst);
 }
@@ -1054,6 +1056,8 @@ qk_whole_norm_rope_store_kernel(T* __restrict__ qkv, long long out_stride, const
   const int pos = positions[t];
   const int pk = pitch > 0 ? pitch : hd, pv = pitch > 0 ? pitch : dv;
   pdl_wait();
+  proj = pdl_fresh(proj);
+  table = pdl_fresh(table);
   const float* row = proj + (size_t)t * ld;
   const int n_q = nq * hd, n_k = nkv * hd;
   float sq = 0.f, sk = 0.f;
@@ -1104,6 +1108,8 @@ qk_whole_norm_rope_row_kernel(T* __restrict__ qkv, long long out_stride, const f
     cache_rows[0] = k0, cache_rows[1] = v0;
   }
   pdl_wait();
+  proj = pdl_fresh(proj);
+  table = pdl_fresh(table);
   const float* row = proj + (size_t)t * ld;
   const int n_q = nq * hd, n_k = nkv * hd, n_all = n_q + n_k + nkv * dv;
   float sq = 0.f, sk = 0.f;
@@ -1191,6 +1197,8 @@ qk_whole_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long out_str
     qk_cache_rows(kcache, vcache, seq_of_token, slots, len_after, page_table, max_pages, ring_rows, keep, nkv, t, pos, 0, hd, dv,
                   &cache_rows[0], &cache_rows[1]);
   pdl_wait();
+  proj = pdl_fresh(proj);
+  table = pdl_fresh(table);
   auto get4 = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
   auto put4 = [](__nv_bfloat16* p, float4 v) {
     const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
@@ -1561,6 +1569,7 @@ head_project_few_kernel(T* __restrict__ out, long long out_stride, const T* __re
   for (int i = 0; i < AF_HPF_AHEAD; ++i) ahead[i] = d0 + i < d1 ? wh[(size_t)(d0 + i) * N] : from_f32<T>(0.f);
   pdl_wait();
   x = pdl_fresh(x);
+  gate = pdl_fresh(gate);
   for (int i = threadIdx.x; i < 8 * D; i += blockDim.x) {
     const int u = i / D, d = i - u * D;
     xs[i] = t0 + u < n_tokens ? to_f32(x[(size_t)(t0 + u) * x_stride + (size_t)h * x_pitch + d]) : 0.f;

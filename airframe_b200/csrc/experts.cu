@@ -524,6 +524,8 @@ expert_rows_kernel(void* __restrict__ out_, const T* __restrict__ a, const T* __
   plan = pdl_fresh(plan);
   perm = pdl_fresh(perm);
   a = pdl_fresh(a);
+  pair_weight = pdl_fresh(pair_weight);
+  scale_out = pdl_fresh(scale_out);
   int expert = 0, row0 = blockIdx.x * AF_EX_TM, rows = min(AF_EX_TM, n_rows - row0);
   if (plan != nullptr) {
     if ((int)blockIdx.x >= plan[0]) return;

@@ -299,6 +299,7 @@ token_shift_kernel(TY* __restrict__ hs, TY* __restrict__ y, const float* __restr
   pdl_wait();
   if (c >= hidden) return;
   x = pdl_fresh(x);
+  prev = pdl_fresh(prev);
   float v[V], b[V], m[V];
 #pragma unroll
   for (int u = 0; u < V; ++u) v[u] = x[(size_t)t * hidden + c + u], m[u] = mu[c + u], b[u] = 0.f;

@@ -37,6 +37,7 @@ delta_prep_kernel(float* __restrict__ out, const float* __restrict__ proj, long 
     bias_w[e] = c < dk ? w0[h * dk + c] : 0.f;
   }
   pdl_wait();
+  proj = pdl_fresh(proj);
   const float* row = proj + (size_t)t * ld;
   for (int l = threadIdx.x; l < rank; l += blockDim.x) low[l] = tanhf(row[off_w1 + l]);
   float kv[4], av[4], ss = 0.f;
@@ -803,6 +804,8 @@ gated_scan_kernel(TY* __restrict__ y, const float* __restrict__ proj, long long 
   const int slot = slots[b];
   const float zb = on ? bz[c] : 0.f, xb = on ? bx[c] : 0.f;
   pdl_wait();
+  proj = pdl_fresh(proj);
+  state = pdl_fresh(state);
   if (last - first < from || last - first > to) return;        // (of another launch)
   if (slot < 0) {
     if (on)
@@ -1069,6 +1072,7 @@ chunk_cumulate_kernel(float* __restrict__ A, const float* __restrict__ w, long l
   const int first = chunk_starts[blockIdx.y], last = chunk_starts[blockIdx.y + 1];
   pdl_wait();
   if (c >= n) return;
+  w = pdl_fresh(w);
   float p = 1.f;
 #pragma unroll 8
   for (int t = first; t < last; ++t) {
@@ -1091,6 +1095,9 @@ chunk_carry_kernel(float* __restrict__ local, float* __restrict__ state, const f
   const int c0 = seq_first_chunk[b], c1 = seq_first_chunk[b + 1];
   pdl_wait();
   if (e >= per || slot < 0) return;
+  local = pdl_fresh(local);
+  state = pdl_fresh(state);
+  A = pdl_fresh(A);
   const int ch = (int)(e % dk);
   const int h = (int)(e / ((size_t)dv * dk));
   const int n = heads * dk;
@@ -1117,9 +1124,11 @@ chunk_correct_kernel(float* __restrict__ out, long long out_ts, const float* __r
   const int j0 = blockIdx.x * 32, h = blockIdx.y;
   const int row0 = tiles[3 * blockIdx.z], rows = tiles[3 * blockIdx.z + 1], chunk = tiles[3 * blockIdx.z + 2];
   const int n = heads * dk;
-  const float* S = s_in + (((size_t)chunk * heads + h) * dv) * dk;
   pdl_wait();
   q = pdl_fresh(q);
+  A = pdl_fresh(A);
+  out = pdl_fresh(out);
+  const float* S = pdl_fresh(s_in) + (((size_t)chunk * heads + h) * dv) * dk;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   for (int c0 = 0; c0 < dk; c0 += 64) {
     for (int i = threadIdx.x; i < 32 * 64; i += 256) {

@@ -393,7 +393,7 @@ retention_carry_kernel(RtArgs a, float* __restrict__ state, const int* __restric
   const size_t at16 = (size_t)(e / a.dk) * a.dkp + e % a.dk;
   pdl_wait();
   if (e >= per_head || slot < 0) return;
-  float* st = state + ((size_t)slot * a.heads + h) * per_head + e;
+  float* st = pdl_fresh(state) + ((size_t)slot * a.heads + h) * per_head + e;
   const size_t step = (size_t)a.heads * per_head, step16 = (size_t)a.heads * a.dv * a.dkp;
   const float* p = pdl_fresh(a.local) + (size_t)ch0 * step + (size_t)h * per_head + e;
   size_t o = (size_t)ch0 * step16 + (size_t)h * a.dv * a.dkp + at16;

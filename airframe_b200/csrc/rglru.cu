@@ -387,6 +387,7 @@ decay_scan_kernel(TY* __restrict__ out, const float* __restrict__ decay, const f
   decay = pdl_fresh(decay);
   input = pdl_fresh(input);
   proj = pdl_fresh(proj);
+  state = pdl_fresh(state);
   if (slot < 0) {
     if (on)
       for (int t = first + w; t < last; t += nw) out[(size_t)t * width + c] = from_f32<TY>(0.f);
