@@ -1189,7 +1189,7 @@ qk_whole_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long out_str
                               const int* __restrict__ page_table, int max_pages, int ring_rows, int keep) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) float srow[];          // q | k | v of the token, biases added
-  __shared__ float red[2][4];
+  __shared__ float red[2][8];
   __shared__ __nv_bfloat16* cache_rows[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x, pos = positions[t];
@@ -1206,7 +1206,7 @@ qk_whole_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long out_str
   };
   const float* row = proj + (size_t)t * ld;
   const int n_q = nq * hd, n_k = nkv * hd, n_v = nkv * dv, n_all = n_q + n_k + n_v;
-  float sq = 0.f, sk = 0.f;
+  float sq, sk;
 #pragma unroll 8
   for (int i = threadIdx.x * 4; i < n_all; i += 512) {
     float4 v = get4(row + i);
@@ -1215,15 +1215,25 @@ qk_whole_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long out_str
       v.x += b.x, v.y += b.y, v.z += b.z, v.w += b.w;
     }
     *reinterpret_cast<float4*>(srow + i) = v;
-    const float s = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-    if (i < n_q) sq += s; else if (i < n_q + n_k) sk += s;
   }
-  sq = warp_sum(sq), sk = warp_sum(sk);
-  if (lane == 0) red[0][warp] = sq, red[1][warp] = sk;
+  __syncthreads();
+  // (the squares meet in the order of the kernel above, whose 256 threads take every 256th value: a row has the same bits in a
+  // step of any number of tokens)
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    sq = sk = 0.f;
+#pragma unroll 4
+    for (int i = threadIdx.x + 128 * u; i < n_q + n_k; i += 256) {
+      const float v = srow[i];
+      if (i < n_q) sq += v * v; else sk += v * v;
+    }
+    sq = warp_sum(sq), sk = warp_sum(sk);
+    if (lane == 0) red[0][warp + 4 * u] = sq, red[1][warp + 4 * u] = sk;
+  }
   __syncthreads();
   sq = sk = 0.f;
 #pragma unroll
-  for (int w = 0; w < 4; ++w) sq += red[0][w], sk += red[1][w];
+  for (int w = 0; w < 8; ++w) sq += red[0][w], sk += red[1][w];
   const float inv_q = rsqrtf(sq / (float)n_q + eps), inv_k = rsqrtf(sk / (float)n_k + eps);
   __nv_bfloat16 *orow = qkv + (size_t)t * out_stride, *kd0 = cache_rows[0], *vd0 = cache_rows[1];
   const int half = hd / 2, groups = half / 4;
@@ -1246,7 +1256,7 @@ qk_whole_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long out_str
     auto turn = [&](float x, float wx, float y, float wy, float c, float s, float& l, float& h) {
       const float u = x * inv * wx, v = y * inv * wy;
       s *= magnitude, c *= magnitude;
-      l = u * c - v * s, h = v * c + u * s;
+      l = fmaf(u, c, -(v * s)), h = fmaf(u, s, v * c);      // (as the compiler joins them in the kernel above: the same bits)
     };
     turn(a.x, wa.x, b.x, wb.x, cs0.x, cs0.y, lo.x, hi.x), turn(a.y, wa.y, b.y, wb.y, cs0.z, cs0.w, lo.y, hi.y);
     turn(a.z, wa.z, b.z, wb.z, cs1.x, cs1.y, lo.z, hi.z), turn(a.w, wa.w, b.w, wb.w, cs1.z, cs1.w, lo.w, hi.w);

@@ -70,11 +70,10 @@ def test_gated_activation_of_32_bit_rows(K, M, inter):
         assert (out.double().cpu() - want).abs().max() < 2e-6 * want.abs().max()
 
 
-@pytest.mark.parametrize("nq, nkv, hd, dv", [(6, 2, 64, 64), (2, 1, 8, 8), (3, 3, 24, 24)])
+@pytest.mark.parametrize("nq, nkv, hd, dv", [(6, 2, 64, 64), (2, 1, 8, 8), (3, 3, 24, 24), (4, 2, 16, 12), (18, 6, 128, 128)])
 @pytest.mark.parametrize("T, table, bias", [(64, True, False), (130, False, True)])
 def test_whole_norm_of_a_prompt(K, nq, nkv, hd, dv, T, table, bias):
-    """Against the same rows in steps of up to 63 tokens, whose sums of squares meet in another order (2^-20 of the factor, so
-    that a result may round to the neighbouring bfloat16)."""
+    """The same bits, packed and in the cache, as the rows have in steps of up to 63 tokens."""
     g = torch.Generator().manual_seed(T + hd)
     n_q, n_k, n_v = nq * hd, nkv * hd, nkv * dv
     proj = (torch.randn(T, n_q + n_k + n_v, generator=g) * 3).to(DEV)
@@ -82,19 +81,28 @@ def test_whole_norm_of_a_prompt(K, nq, nkv, hd, dv, T, table, bias):
     b = torch.randn(n_q + n_k + n_v, generator=g).to(DEV) if bias else None
     inv = (10000.0 ** (-torch.arange(0, hd, 2) / hd)).float().to(DEV)
     pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    pages = (T + 63) // 64 + 1
 
-    def run(lo, hi):
-        zeros = torch.zeros(hi - lo, dtype=torch.int32, device=DEV)
-        batch = SimpleNamespace(positions=pos[lo:hi], seq_of_token=zeros, slots=zeros[:1],
-                                len_after=torch.full((1,), T, dtype=torch.int32, device=DEV), aux={})
-        out = torch.empty(hi - lo, n_q + n_k + n_v, dtype=torch.bfloat16, device=DEV)
-        K.qk_norm_rope_store(out, proj[lo:hi], batch, nq, nkv, hd, inv, hd, "half", q_weight=wq, k_weight=wk, eps=1e-5, dv=dv,
-                             whole_norm=True, bias=b, table=K.rope_table(pos[lo:hi], inv) if table else None)
-        return out.double()
+    def run(cuts):
+        kv = SimpleNamespace(k=torch.full((pages, nkv, K.PAGE, hd), 7.0, dtype=torch.bfloat16, device=DEV),
+                             v=torch.full((pages, nkv, K.PAGE, dv), 7.0, dtype=torch.bfloat16, device=DEV),
+                             page_table=torch.arange(pages, dtype=torch.int32, device=DEV).flip(0)[None].contiguous(), ring_rows=pages * 64)
+        rows = []
+        for lo, hi in cuts:
+            zeros = torch.zeros(hi - lo, dtype=torch.int32, device=DEV)
+            batch = SimpleNamespace(positions=pos[lo:hi], seq_of_token=zeros, slots=zeros[:1],
+                                    len_after=torch.full((1,), T, dtype=torch.int32, device=DEV), aux={})
+            rows.append(torch.empty(hi - lo, n_q + n_k + n_v, dtype=torch.bfloat16, device=DEV))
+            K.qk_norm_rope_store(rows[-1], proj[lo:hi], batch, nq, nkv, hd, inv, hd, "half", q_weight=wq, k_weight=wk, eps=1e-5, dv=dv,
+                                 whole_norm=True, bias=b, table=K.rope_table(pos[lo:hi], inv) if table else None, kv=kv)
+        return torch.cat(rows), kv.k, kv.v
 
-    got, want = run(0, T), torch.cat([run(i, min(T, i + 50)) for i in range(0, T, 50)])
-    assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-4).all()
-    assert (got == want).double().mean() > 0.99
+    got, want = run([(0, T)]), run([(i, min(T, i + 50)) for i in range(0, T, 50)])
+    for x, y in zip(got, want):
+        assert torch.equal(x, y)
+    for cache, rows in ((got[1], got[0][:, n_q:n_q + n_k].view(T, nkv, hd)), (got[2], got[0][:, n_q + n_k:].view(T, nkv, dv))):
+        stored = cache.flip(0).transpose(1, 2).reshape(pages * 64, nkv, -1)
+        assert torch.equal(stored[:T], rows) and bool((stored[T:] == 7.0).all())
 
 
 @pytest.mark.parametrize("width, taps", [(64, 4), (516, 2), (60, 3)])
