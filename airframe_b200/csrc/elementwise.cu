@@ -187,7 +187,7 @@ AF_EXPORT int af_rmsnorm(void* y, int y_dtype, const float* x, const float* w, c
   AF_REQUIRE(n_rows > 0 && hidden > 0, "af_rmsnorm: bad sizes");
   if (hidden % 4 == 0 && hidden <= 8192 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
     const int nv = hidden > 4096 ? 2 : 1;
-    const int threads = ((hidden / (4 * nv) + 31) / 32) * 32;
+    const int threads = ((hidden / 4 + nv - 1) / nv + 31) / 32 * 32;
     if (nv == 2) {
       AF_DISPATCH_DTYPE(y_dtype, TY,
                         af_launch(rmsnorm_row_kernel<TY, 2>, dim3(n_rows), dim3(threads), 0, stream, (TY*)y, x, w,
@@ -355,7 +355,7 @@ AF_EXPORT int af_add_rmsnorm(float* x, const void* a, int a_dtype, int n_parts, 
                        (part_stride % 4 == 0);
   if (hidden % 4 == 0 && hidden <= 8192 && aligned && ((uintptr_t)y & 7) == 0) {
     const int nv = (n_rows >= 256 && hidden >= 1024) || hidden > 4096 ? 2 : 1;
-    const int threads = ((hidden / (4 * nv) + 31) / 32) * 32;
+    const int threads = ((hidden / 4 + nv - 1) / nv + 31) / 32 * 32;
 #define LAUNCH_ROW(TA, TY)                                                                                  \
   do {                                                                                                      \
     if (nv == 2 && n_rows >= 256 && threads <= 512)                                                         \
@@ -659,7 +659,7 @@ AF_EXPORT int af_add_scaled_rmsnorm(float* x, const void* a, int a_dtype, int a_
   if (hidden % 4 == 0 && hidden <= 8192 &&
       (((uintptr_t)x | (uintptr_t)a | (uintptr_t)b | (uintptr_t)w_next | (uintptr_t)y) & 15) == 0) {
     const int nv = hidden > 4096 ? 2 : 1;
-    const int threads = ((hidden / (4 * nv) + 31) / 32) * 32;
+    const int threads = ((hidden / 4 + nv - 1) / nv + 31) / 32 * 32;
     if (nv == 2) {
       AF_DISPATCH_DTYPE(y_dtype, TY,
                         af_launch(add_scaled_rmsnorm_row_kernel<TY, 2>, dim3(n_rows), dim3(threads), 0, stream, x, a, a_dtype,
@@ -833,7 +833,7 @@ AF_EXPORT int af_add_normed_terms(float* x, const void* a, int a_dtype, int a_pa
       (((uintptr_t)x | (uintptr_t)a | (uintptr_t)b | (uintptr_t)w_post | (uintptr_t)w_next | (uintptr_t)y) & 15) == 0) {
     // (many rows: two groups a thread, so that more rows share an SM and their phases overlap)
     const int nv = (n_rows >= 256 && hidden >= 1024) || hidden > 4096 ? 2 : 1;
-    const int row_threads = ((hidden / (4 * nv) + 31) / 32) * 32;
+    const int row_threads = ((hidden / 4 + nv - 1) / nv + 31) / 32 * 32;
     if (nv == 2 && n_rows >= 256 && row_threads <= 512) {
       AF_DISPATCH_DTYPE(y_dtype, TY,
                         af_launch(add_normed_terms_row_kernel<TY, 2, true>, dim3(n_rows), dim3(row_threads), 0, stream, x, a,

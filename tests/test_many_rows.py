@@ -105,6 +105,40 @@ def test_whole_norm_of_a_prompt(K, nq, nkv, hd, dv, T, table, bias):
         assert torch.equal(stored[:T], rows) and bool((stored[T:] == 7.0).all())
 
 
+@pytest.mark.parametrize("M, H", [(300, 1028), (300, 2308), (5, 4100), (300, 4100), (3, 8188)])
+def test_norms_of_widths_one_group_over_a_blocks(K, M, H):
+    """Two groups of four values a thread and an odd number of groups: the last one belongs to a row as the others do."""
+    g = torch.Generator().manual_seed(M + H)
+    x, a, b = (torch.randn(M, H, generator=g) for _ in range(3))
+    w1, w2 = torch.randn(H, generator=g), torch.randn(H, generator=g)
+    x[:, -4:] *= 40.0
+    a[:, -4:] *= 40.0
+    norm = lambda t, w: t / (t.square().mean(1, keepdim=True) + 1e-5).sqrt() * w.double()
+    x64, a64, b64 = x.double(), a.double(), b.double()
+
+    def check(y, xd, want_x, want_y):
+        # (a sum of H squares in 32 bits, a few roundings)
+        assert (y.double().cpu() - want_y).abs().max() < 1e-5 * want_y.abs().max()
+        assert xd is None or (xd.double().cpu() - want_x).abs().max() < 1e-5 * want_x.abs().max()
+
+    dev = lambda t: t.to(DEV)
+    y = torch.full((M, H), float("nan"), device=DEV)
+    K.rmsnorm(y, dev(x), dev(w1), 1e-5, 0.0)
+    check(y, None, None, norm(x64, w1))
+    y, xd = torch.full((M, H), float("nan"), device=DEV), dev(x)
+    K.add_rmsnorm(xd, dev(a), dev(w1), 1e-5, 0.0, y=y, w_next=dev(w2), eps_next=1e-5)
+    want = x64 + norm(a64, w1)
+    check(y, xd, want, norm(want, w2))
+    y, xd = torch.full((M, H), float("nan"), device=DEV), dev(x)
+    K.add_scaled_rmsnorm(xd, [(dev(a), 0.5), (dev(b), 2.0)], y=y, w_next=dev(w2), eps=1e-5)
+    want = x64 + 0.5 * a64 + 2.0 * b64
+    check(y, xd, want, norm(want, w2))
+    y, xd = torch.full((M, H), float("nan"), device=DEV), dev(x)
+    K.add_normed_terms(xd, [(dev(a), 0.5), (dev(b), 2.0)], dev(w1), 1e-5, y=y, w_next=dev(w2), eps_next=1e-5)
+    want = x64 + norm(0.5 * a64 + 2.0 * b64, w1)
+    check(y, xd, want, norm(want, w2))
+
+
 @pytest.mark.parametrize("width, taps", [(64, 4), (516, 2), (60, 3)])
 def test_convolution_of_four_channels_a_thread(K, width, taps):
     """Sequences that begin inside a group of tokens, with and without a history, against rows that cannot be read in fours."""
