@@ -1080,7 +1080,7 @@ qk_whole_norm_rope_store_kernel(T* __restrict__ qkv, long long out_stride, const
   }
 }
 
-// The same with the token's projection row in shared memory (rows of up to 12,288 values, the norm in front of the
+// The same with the token's projection row in shared memory (rows of up to 12,256 values, the norm in front of the
 // rotation, values of their own): the row is read once, both mean squares leave one reduction, the cache row is
 // looked up once a token, and the pairs of all heads are one flat loop whose loads do not wait for one another.
 template <typename T>
@@ -1298,8 +1298,10 @@ AF_EXPORT int af_qk_norm_rope_store(void* qkv, int dtype, long long out_stride, 
   AF_REQUIRE(ring_rows % AF_PAGE == 0, "af_qk_norm_rope_store: ring rows %d not whole pages", ring_rows);
   AF_REQUIRE((kcache == nullptr) == (vcache == nullptr), "af_qk_norm_rope_store: k and v cache");
   AF_REQUIRE((q_weight == nullptr) == (k_weight == nullptr), "af_qk_norm_rope_store: both norm weights or none");
+  // (a row's values in a block's shared memory, beside the few static bytes of the kernels that keep them there: 48 KB in all)
   const size_t row_bytes = ((size_t)(nq + nkv) * hd + (size_t)nkv * dv) * sizeof(float);
-  if (whole_norm && !norm_after && !v_from_k && row_bytes <= 48 * 1024 && dtype == AF_BF16 && n_tokens >= 64 && pairing == AF_PAIR_HALF &&
+  const bool row_fits = row_bytes <= 48 * 1024 - 128;
+  if (whole_norm && !norm_after && !v_from_k && row_fits && dtype == AF_BF16 && n_tokens >= 64 && pairing == AF_PAIR_HALF &&
       rot_dim == hd && hd % 8 == 0 && dv % 4 == 0 && (pitch == 0 || (pitch == hd && pitch == dv)) && ld % 4 == 0 && out_stride % 4 == 0 &&
       (((uintptr_t)qkv | (uintptr_t)proj | (uintptr_t)bias | (uintptr_t)q_weight | (uintptr_t)k_weight | (uintptr_t)table |
         (uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0) {
@@ -1308,7 +1310,7 @@ AF_EXPORT int af_qk_norm_rope_store(void* qkv, int dtype, long long out_stride, 
               (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, page_table, max_pages, ring_rows, keep);
     AF_CHECK_LAUNCH("af_qk_norm_rope_store");
   }
-  if (whole_norm && !norm_after && !v_from_k && row_bytes <= 48 * 1024) {
+  if (whole_norm && !norm_after && !v_from_k && row_fits) {
     AF_DISPATCH_DTYPE(dtype, T,
                       af_launch(qk_whole_norm_rope_row_kernel<T>, dim3((unsigned)n_tokens), dim3(256), row_bytes, stream,
                                 (T*)qkv, out_stride, proj, ld, bias, q_weight, k_weight, eps, magnitude, positions,

@@ -105,6 +105,25 @@ def test_whole_norm_of_a_prompt(K, nq, nkv, hd, dv, T, table, bias):
         assert torch.equal(stored[:T], rows) and bool((stored[T:] == 7.0).all())
 
 
+@pytest.mark.parametrize("T", [3, 70])
+@pytest.mark.parametrize("nq, nkv, hd", [(32, 8, 256), (48, 24, 128), (7, 1, 1360)])
+def test_whole_norm_of_the_widest_rows(K, nq, nkv, hd, T):
+    """Rows of 48 KB and a little less, which a block's shared memory holds or does not, against 64 bits."""
+    g = torch.Generator().manual_seed(nq)
+    n = (nq + 2 * nkv) * hd
+    proj, wq, wk = torch.randn(T, n, generator=g), torch.randn(nq * hd, generator=g), torch.randn(nkv * hd, generator=g)
+    pos = torch.zeros(T, dtype=torch.int32, device=DEV)                   # (position 0: the rotation leaves its rows alone)
+    batch = SimpleNamespace(positions=pos, seq_of_token=pos, slots=pos[:1], len_after=pos[:1] + 1, aux={})
+    out = torch.empty(T, n, dtype=torch.bfloat16, device=DEV)
+    inv = torch.ones(hd // 2, device=DEV)
+    K.qk_norm_rope_store(out, proj.to(DEV), batch, nq, nkv, hd, inv, hd, "half", q_weight=wq.to(DEV), k_weight=wk.to(DEV), eps=1e-5, whole_norm=True)
+    q, k, v = proj.double().split([nq * hd, nkv * hd, nkv * hd], 1)
+    norm = lambda x, w: x / (x.square().mean(1, keepdim=True) + 1e-5).sqrt() * w.double()
+    want = torch.cat([norm(q, wq), norm(k, wk), v], 1)
+    # (half a unit of a bfloat16 and the sum's roundings)
+    assert ((out.double().cpu() - want).abs() <= (2.0 ** -8 + 2.0 ** -18) * want.abs() + 1e-30).all()
+
+
 @pytest.mark.parametrize("M, H", [(300, 1028), (300, 2308), (5, 4100), (300, 4100), (3, 8188)])
 def test_norms_of_widths_one_group_over_a_blocks(K, M, H):
     """Two groups of four values a thread and an odd number of groups: the last one belongs to a row as the others do."""
