@@ -121,19 +121,20 @@ rope_cache_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride, con
   // the cache and the sines and cosines are worked out before the wait for the kernel in front)
   const int t0 = blockIdx.x * TOK, half = hd / 2, per_head = half / 4, n_heads = nq + 2 * nkv;
   const int c = threadIdx.x % per_head * 4, head0 = threadIdx.x / per_head, step = blockDim.x / per_head;
-  int pos[TOK], dst[TOK];                          // (the row of kv head 0 in the cache; -1: not stored)
+  int pos[TOK];
+  uint32_t dst[TOK];                               // (page * AF_PAGE + the row in it; all ones: not stored)
 #pragma unroll
   for (int u = 0; u < TOK; ++u) pos[u] = t0 + u < n_tokens ? positions[t0 + u] : 0;
 #pragma unroll
   for (int u = 0; u < TOK; ++u) {
-    dst[u] = -1;
+    dst[u] = 0xffffffffu;
     if (kcache == nullptr || t0 + u >= n_tokens) continue;
     const int seq = seq_of_token[t0 + u], slot = slots[seq];
     if (slot >= 0 && af_cache_stores(pos[u], len_after[seq], ring_rows, keep)) {
       const int r = af_cache_row(pos[u], ring_rows, keep);
       if (AF_INDEX_OK(pos[u] >= 0 && r / AF_PAGE < max_pages, r)) {
         const int page = page_table[(size_t)slot * max_pages + r / AF_PAGE];
-        if (AF_INDEX_OK(page >= 0, page)) dst[u] = page * nkv * AF_PAGE + r % AF_PAGE;
+        if (AF_INDEX_OK(page >= 0, page)) dst[u] = (uint32_t)page * AF_PAGE + r % AF_PAGE;
       }
     }
   }
@@ -191,9 +192,10 @@ rope_cache_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride, con
         *reinterpret_cast<uint2*>(x) = lo[u];
         *reinterpret_cast<uint2*>(x + half) = hi[u];
       }
-      if (dst[u] >= 0 && head >= nq) {
+      if (dst[u] != 0xffffffffu && head >= nq) {
         const bool is_v = head >= nq + nkv;
-        __nv_bfloat16* d = (is_v ? vcache : kcache) + ((size_t)dst[u] + (size_t)(head - nq - (is_v ? nkv : 0)) * AF_PAGE) * hd + c;
+        const size_t at = ((size_t)(dst[u] / AF_PAGE) * nkv + (head - nq - (is_v ? nkv : 0))) * AF_PAGE + dst[u] % AF_PAGE;
+        __nv_bfloat16* d = (is_v ? vcache : kcache) + at * hd + c;
         *reinterpret_cast<uint2*>(d) = lo[u];
         *reinterpret_cast<uint2*>(d + half) = hi[u];
       }

@@ -197,3 +197,22 @@ def test_split_sums_joined_four_at_a_time(K, M, N, Kd, cap):
     want = x.double() @ w.double().T
     want = cap * torch.tanh(want / cap) if cap else want
     assert (out.double() - want).abs().max() < 2e-5 * Kd ** 0.5
+
+
+def test_rotated_rows_behind_two_to_the_31st_cache_row(K):
+    """A cache of more rows than 32 bits with a sign count: heads of 16 elements, the last pages of 64 GB.  (Keys and values share the
+    memory, a page apart; nothing but the rows' own places is touched.)"""
+    rows, nkv, hd, T = 2 ** 31 + 4 * 64, 1, 16, 64
+    if torch.cuda.mem_get_info()[0] < 80 << 30:
+        pytest.skip("80 GB of free device memory")
+    memory = torch.empty(rows // 64 + 1, nkv, 64, hd, dtype=torch.bfloat16, device=DEV)
+    last = rows // 64 - 2
+    memory[last - 1:] = 7.0
+    qkv = torch.randn(T, 4 * hd).to(torch.bfloat16).to(DEV)                # 2 query heads, 1 of keys, 1 of values
+    pos, zeros = torch.arange(T, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+    K.rope_cache_write(qkv, pos, torch.ones(hd // 2, device=DEV), 2, nkv, hd, hd, "half", seq_of_token=zeros, slots=zeros[:1],
+                       len_after=zeros[:1] + T, kcache=memory[:-1], vcache=memory[1:], ring_rows=0,
+                       page_table=torch.tensor([[last]], dtype=torch.int32, device=DEV))
+    assert last * 64 >= 2 ** 31
+    assert torch.equal(memory[last, 0], qkv[:, 2 * hd:3 * hd]) and torch.equal(memory[last + 1, 0], qkv[:, 3 * hd:])
+    assert bool((memory[last - 1] == 7.0).all()) and bool((memory[last + 2:] == 7.0).all())
