@@ -394,6 +394,8 @@ def attn_prefill_f32(out, q, k, v, seq_starts, n_seqs: int, max_len: int, nq: in
     [n_seqs + 1], no sequence longer than ``max_len``; options as in :func:`attn_prefill_plain`)."""
     if any(t.dtype != torch.float32 for t in (out, q, k, v)):
         raise KernelError("attn_prefill_f32: float32 only")
+    if k.shape[0] != q.shape[0] or v.shape[0] != q.shape[0] or out.shape[0] != q.shape[0]:
+        raise KernelError("attn_prefill_f32: q, k, v and out hold the same rows")
     if any(t is not None and t.numel() != nq for t in (slopes, sinks)):
         raise KernelError(f"attn_prefill_f32: a slope and a sink for each of {nq} heads")
     if mask not in MASKS:

@@ -28,3 +28,14 @@ def test_which_steps_go_in_chunks():
         assert chunks_pay(lens), lens
     for lens in ([1], [127], [64] * 16, [33] * 16, [128] + [1] * 63, [128] + [1] * 255, [128] + [8] * 60, [130] + [17] * 63, [2048] + [1] * 400):
         assert not chunks_pay(lens), lens
+
+
+def test_attention_of_prompts_in_32_bits_takes_rows_of_one_number():
+    """Keys or values of fewer rows than the queries are refused before anything is launched: the kernel would read behind them."""
+    import pytest
+    import torch
+    from airframe_b200 import kernels
+    q, short, starts = torch.zeros(80, 64), torch.zeros(79, 64), torch.tensor([0, 80], dtype=torch.int32)
+    for k, v in ((short, q), (q, short)):
+        with pytest.raises(kernels.KernelError, match="the same rows"):
+            kernels.attn_prefill_f32(torch.zeros(80, 64), q, k, v, starts, 1, 80, 1, 1, 64, 1.0, 0.0, 0)
