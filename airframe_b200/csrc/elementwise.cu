@@ -411,7 +411,7 @@ __global__ void gated_act_kernel(T* __restrict__ out, const T* __restrict__ gu, 
 }
 
 // Four neighbours a thread (32-bit rows of whole 16-byte pieces).  Bound by its bytes: a value a thread left most of the memory's
-// rate unused (301 x 9,216: 13.5 -> 5.8 us).
+// rate unused (301 x 9,216: 11.8 -> 4.0 us).
 __global__ void __launch_bounds__(256)
 gated_act4_kernel(float* __restrict__ out, const float* __restrict__ gu, int inter, int act) {
   pdl_launch_dependents();
@@ -430,7 +430,9 @@ AF_EXPORT int af_gated_act(void* out, const void* gu, int dtype, int n_rows, int
   if (n_rows == 0) return 0;
   AF_REQUIRE(n_rows > 0 && inter > 0, "af_gated_act: bad sizes");
   AF_REQUIRE(act == AF_ACT_GELU_TANH || act == AF_ACT_SILU, "af_gated_act: unknown activation %d", act);
-  if (dtype == AF_F32 && inter % 4 == 0 && inter <= 65535 * 1024 && (((uintptr_t)out | (uintptr_t)gu) & 15) == 0) {
+  // (fewer values: four times the threads, each with a shorter chain of exponentials, are done sooner: 8 x 9,216 1.03 against 1.12 us,
+  // 32 1.57 and 1.59, 63 2.5 and 1.8; x 4,096 8 rows 0.9 and 1.1, 100 2.07 and 2.06, 128 2.5 and 1.8)
+  if (dtype == AF_F32 && (long long)n_rows * inter >= 1 << 19 && inter % 4 == 0 && inter <= 65535 * 1024 && (((uintptr_t)out | (uintptr_t)gu) & 15) == 0) {
     af_launch(gated_act4_kernel, dim3(n_rows, (inter + 1023) / 1024), dim3(256), 0, stream, (float*)out, (const float*)gu, inter, act);
     AF_CHECK_LAUNCH("af_gated_act");
   }

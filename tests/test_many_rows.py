@@ -29,7 +29,7 @@ def rope_step(K, qkv, pos, nq, nkv, hd, table):
     return qkv, kc, vc
 
 
-@pytest.mark.parametrize("dtype, T, piece", [(torch.bfloat16, 1001, 500), (torch.float32, 130, 1), (torch.float32, 7, 7)])
+@pytest.mark.parametrize("dtype, T, piece", [(torch.bfloat16, 1001, 500), (torch.float32, 400, 1), (torch.float32, 400, 95), (torch.float32, 7, 3)])
 @pytest.mark.parametrize("nq, nkv, hd", [(4, 2, 64), (3, 1, 8), (8, 4, 256)])
 def test_rotated_rows(K, dtype, T, piece, nq, nkv, hd):
     """Bits do not depend on how many rows a step has nor on where the angles come from; 64 bits beside them."""
@@ -56,7 +56,7 @@ def test_rotated_rows(K, dtype, T, piece, nq, nkv, hd):
         assert torch.equal(stored[:T], rows_of) and bool((stored[T:] == 7.0).all())
 
 
-@pytest.mark.parametrize("M, inter", [(1, 4), (3, 1024), (5, 1028), (2, 4100)])
+@pytest.mark.parametrize("M, inter", [(1, 4), (3, 1024), (2, 4100), (2 ** 17, 4), (512, 1024), (510, 1028), (128, 4100)])
 def test_gated_activation_of_32_bit_rows(K, M, inter):
     """Four values a thread at the edges of a block's 1,024; the same bits as a row that cannot be read in fours."""
     gu = torch.randn(M, 2 * inter, generator=torch.Generator().manual_seed(inter)) * 2
