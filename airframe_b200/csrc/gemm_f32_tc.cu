@@ -270,30 +270,6 @@ f32_join_kernel(float* __restrict__ out, long long ldo, const float* __restrict_
   out[(size_t)m * ldo + n] = softcap_f32(v, cap);
 }
 
-// The same, four neighbouring sums a thread and all splits' on their way at once: one after the other their latencies were most
-// of the kernel (301 tokens, 4,096 and 2,304 columns: 4.9 -> 4.0 us).
-constexpr int FT_MOST_SPLITS = 8;
-__global__ void __launch_bounds__(256)
-f32_join4_kernel(float* __restrict__ out, long long ldo, const float* __restrict__ parts, int splits, int M, int N, float cap) {
-  pdl_launch_dependents();
-  const int row4 = N / 4;
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (i >= (long long)M * row4) return;
-  const int m = (int)(i / row4), n = (int)(i - (long long)m * row4) * 4;
-  pdl_wait();
-  parts = pdl_fresh(parts);
-  float4 p[FT_MOST_SPLITS];
-#pragma unroll
-  for (int s = 0; s < FT_MOST_SPLITS; ++s)
-    if (s < splits) p[s] = *reinterpret_cast<const float4*>(parts + ((size_t)s * M + m) * N + n);
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int s = 0; s < FT_MOST_SPLITS; ++s)
-    if (s < splits) v.x += p[s].x, v.y += p[s].y, v.z += p[s].z, v.w += p[s].w;
-  *reinterpret_cast<float4*>(out + (size_t)m * ldo + n) =
-      make_float4(softcap_f32(v.x, cap), softcap_f32(v.y, cap), softcap_f32(v.z, cap), softcap_f32(v.w, cap));
-}
-
 template <int NT>
 int ft_launch(const CUtensorMap& map, const FtArgs& a, int splits, cudaStream_t stream) {
   static bool sized[AF_MAX_DEVICES];
@@ -351,11 +327,6 @@ AF_EXPORT int af_gemm_f32_tc(float* out, long long ldo, const float* x, long lon
     default: e = ft_launch<160>(map, a, splits, stream); break;
   }
   if (e || splits == 1) return e;
-  if (N % 4 == 0 && ldo % 4 == 0 && (((uintptr_t)out | (uintptr_t)sums) & 15) == 0 && splits <= FT_MOST_SPLITS) {
-    const long long blocks = ((long long)M * (N / 4) + 255) / 256;
-    af_launch(f32_join4_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, out, ldo, sums, splits, M, N, cap);
-    AF_CHECK_LAUNCH("af_gemm_f32_tc (join)");
-  }
   af_launch(f32_join_kernel, dim3((N + 255) / 256, M), dim3(256), 0, stream, out, ldo, sums, splits, M, N, cap);
   AF_CHECK_LAUNCH("af_gemm_f32_tc (join)");
 }

@@ -185,20 +185,6 @@ def test_convolution_of_four_channels_a_thread(K, width, taps):
         assert (u[starts[b]:starts[b] + n].double().cpu() - want).abs().max() < 1e-5
 
 
-@pytest.mark.parametrize("M, N, Kd, cap", [(33, 260, 2048, 0.0), (70, 2304, 4096, 30.0), (1, 4, 1100, 0.0)])
-def test_split_sums_joined_four_at_a_time(K, M, N, Kd, cap):
-    """The same bits as into rows that cannot be written in fours, whose sums are joined one by one."""
-    g = torch.Generator().manual_seed(N)
-    x, w = torch.randn(M, Kd, generator=g).to(DEV), torch.randn(N, Kd, generator=g).to(DEV)
-    out, odd = torch.empty(M, N, device=DEV), torch.empty(M, N + 1, device=DEV)[:, :N]
-    K.gemm_f32_tc(out, x, w, cap=cap)
-    K.gemm_f32_tc(odd, x, w, cap=cap)
-    assert torch.equal(out, odd)
-    want = x.double() @ w.double().T
-    want = cap * torch.tanh(want / cap) if cap else want
-    assert (out.double() - want).abs().max() < 2e-5 * Kd ** 0.5
-
-
 def test_rotated_rows_behind_two_to_the_31st_cache_row(K):
     """A cache of more rows than 32 bits with a sign count: heads of 16 elements, the last pages of 64 GB.  (Keys and values share the
     memory, a page apart; nothing but the rows' own places is touched.)"""
