@@ -28,7 +28,7 @@ struct PtArgs {
   const float *q, *k, *v;
   long long out_stride, q_stride, k_stride, v_stride;
   const int* seq_starts;
-  int least;                          // shorter sequences are another kernel's
+  int n_seqs, least;                  // (shorter sequences are another kernel's)
   int nq, nkv, hd, dv;
   float scale, cap;
   int window, mask_kind, keep;
@@ -87,10 +87,30 @@ attn_prefill_f32_kernel(PtArgs a) {
   const int h = blockIdx.y, g = h / (a.nq / a.nkv);
   pdl_wait();
   a.q = pdl_fresh(a.q), a.k = pdl_fresh(a.k), a.v = pdl_fresh(a.v);
-  const int first = a.seq_starts[blockIdx.z], len = a.seq_starts[blockIdx.z + 1] - first;
-  const int tiles = (len + PT_Q - 1) / PT_Q;
-  if (len < a.least || (int)blockIdx.x >= tiles) return;
-  const int p0 = (tiles - 1 - (int)blockIdx.x) * PT_Q, n_q = min(PT_Q, len - p0), last = p0 + n_q - 1;
+  // the block's sequence: tile blockIdx.x of those of all sequences of `least` tokens and more, one after the other.  (A block a tile of the
+  // longest for every sequence left most of them without work, and each holds an SM: a sequence of 300 tokens among 100 of 3, 18 heads, a window of 64:
+  // 100 us.)
+  int first = 0, len = 0, tile = (int)blockIdx.x;
+  for (int base = 0; base < a.n_seqs && len == 0; base += 32) {
+    const int i = min(base + lane, a.n_seqs - 1), from = a.seq_starts[i], n = base + lane < a.n_seqs ? a.seq_starts[i + 1] - from : 0;
+    const int mine = n >= a.least ? (n + PT_Q - 1) / PT_Q : 0;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += up;
+    }
+    const unsigned behind = __ballot_sync(0xffffffffu, upto > tile);
+    if (behind != 0) {
+      const int of = __ffs(behind) - 1;
+      first = __shfl_sync(0xffffffffu, from, of), len = __shfl_sync(0xffffffffu, n, of);
+      tile -= __shfl_sync(0xffffffffu, upto - mine, of);
+    } else {
+      tile -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+  }
+  if (len == 0) return;
+  const int p0 = ((len + PT_Q - 1) / PT_Q - 1 - tile) * PT_Q, n_q = min(PT_Q, len - p0), last = p0 + n_q - 1;
   const int lo0 = pt_first_visible(p0, a.window, a.mask_kind);
   const float* kb = a.k + (size_t)first * a.k_stride + (size_t)g * a.hd;
   const float* vb = a.v + (size_t)first * a.v_stride + (size_t)g * a.dv;
@@ -309,23 +329,27 @@ int pt_launch(dim3 grid, const PtArgs& a, cudaStream_t stream) {
 
 }  // namespace
 
-// Attention of the sequences of `least` tokens and more among n_seqs (rows seq_starts[i] .. seq_starts[i + 1]; the longest has
+// Attention of the sequences of `least` tokens and more among n_seqs (rows seq_starts[i] .. seq_starts[i + 1] of n_rows; the longest has
 // max_len) over the step's own keys and values, all float32; options as in af_attn_prefill_plain.  Keys and values of up to 256.
 AF_EXPORT int af_attn_prefill_f32(float* out, long long out_stride, const float* q, long long q_stride, const float* k,
                                   long long k_stride, const float* v, long long v_stride, const int* seq_starts, int n_seqs,
-                                  int max_len, int least, int nq, int nkv, int hd, int dv, float scale, float cap, int window,
+                                  int n_rows, int max_len, int least, int nq, int nkv, int hd, int dv, float scale, float cap, int window,
                                   int mask_kind, int keep, const float* slopes, const float* sinks, const float* gate,
                                   long long gate_stride, cudaStream_t stream) {
   if (n_seqs == 0 || max_len < least) return 0;
-  AF_REQUIRE(n_seqs > 0 && n_seqs <= 65535 && max_len > 0 && nq > 0 && nq <= 65535 && nkv > 0 && nq % nkv == 0,
-             "af_attn_prefill_f32: %d sequences, heads %d, groups %d", n_seqs, nq, nkv);
+  AF_REQUIRE(n_seqs > 0 && n_rows > 0 && max_len > 0 && least > 0 && nq > 0 && nq <= 65535 && nkv > 0 && nq % nkv == 0,
+             "af_attn_prefill_f32: %d sequences of %d rows, heads %d, groups %d", n_seqs, n_rows, nq, nkv);
   AF_REQUIRE(hd > 0 && hd <= 256 && dv > 0 && dv <= 256, "af_attn_prefill_f32: key size %d or value size %d beyond 256", hd, dv);
   AF_REQUIRE(mask_kind == AF_MASK_WINDOW || mask_kind == AF_MASK_CHUNK, "af_attn_prefill_f32: mask kind %d", mask_kind);
   AF_REQUIRE(keep >= 0, "af_attn_prefill_f32: %d kept tokens", keep);
   const bool vec = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0 && ((q_stride | k_stride | v_stride | hd | dv) & 3) == 0;
-  const PtArgs a{out, q, k, v, out_stride, q_stride, k_stride, v_stride, seq_starts, least, nq, nkv, hd, dv, scale, cap, window,
+  const PtArgs a{out, q, k, v, out_stride, q_stride, k_stride, v_stride, seq_starts, n_seqs, least, nq, nkv, hd, dv, scale, cap, window,
                  mask_kind, window > 0 ? keep : 0, slopes, sinks, gate, gate_stride, vec ? 1 : 0};
-  const dim3 grid((max_len + PT_Q - 1) / PT_Q, nq, n_seqs);
+  // (no more tiles than these: a sequence's last may be short; those of max_len tokens each; a sequence of `least` tokens and more is one of n_rows / least)
+  const long long longest = (max_len + PT_Q - 1) / PT_Q, seqs = n_seqs < n_rows / least ? n_seqs : n_rows / least;
+  const long long most = n_rows / PT_Q + seqs < longest * seqs ? n_rows / PT_Q + seqs : longest * seqs;
+  if (most == 0) return 0;
+  const dim3 grid((unsigned)most, nq);
   const int HD = hd <= 64 ? 64 : hd <= 128 ? 128 : 256, DV = dv <= 64 ? 64 : dv <= 128 ? 128 : 256;
   if (DV == 256) return HD == 256 ? pt_launch<256, 256>(grid, a, stream) : pt_launch<128, 256>(grid, a, stream);
   if (HD == 256) return pt_launch<256, 128>(grid, a, stream);

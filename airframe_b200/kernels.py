@@ -352,6 +352,9 @@ def _most_keys(max_len: int, window: int, keep: int) -> int:
     return min(max_len, window + keep) if window else max_len
 
 
+_NO_SEQS = (c_void_p(0), c_void_p(0))
+
+
 def attn_prefill_plain(out, q, k, v, positions, nq: int, nkv: int, hd: int, scale: float, cap: float,
                        window: int, slopes=None, dv=None, mask: str = "window", sinks=None, gate=None,
                        keep: int = 0, max_len: int = 0, seqs=None, below: int = 0) -> None:
@@ -378,7 +381,7 @@ def attn_prefill_plain(out, q, k, v, positions, nq: int, nkv: int, hd: int, scal
         c_int(T), c_int(nq), c_int(nkv), c_int(hd), c_int(dv or hd), c_float(scale), c_float(cap), c_int(window),
         c_int(MASKS[mask]), c_int(keep), _ptr(slopes, "slopes", torch.float32, allow_none=True),
         _ptr(sinks, "sinks", torch.float32, allow_none=True), gp, gs,
-        c_int(_most_keys(max_len or T, window, keep)), *(_ptr(t, "seqs", torch.int32, allow_none=True) for t in seqs or (None, None)),
+        c_int(_most_keys(max_len or T, window, keep)), *(_NO_SEQS if seqs is None else (_ptr(t, "seqs", torch.int32) for t in seqs)),
         c_int(below), _stream()))
 
 
@@ -403,7 +406,7 @@ def attn_prefill_f32(out, q, k, v, seq_starts, n_seqs: int, max_len: int, nq: in
     gp, gs = _gate_args(gate, q.shape[0], nq, "attn_prefill_f32")
     _check(_lib().af_attn_prefill_f32(
         _ptr(out), c_longlong(_rows(out, "out")), _ptr(q), c_longlong(_rows(q, "q")), _ptr(k), c_longlong(_rows(k, "k")),
-        _ptr(v), c_longlong(_rows(v, "v")), _ptr(seq_starts, "seq_starts", torch.int32), c_int(n_seqs), c_int(max_len), c_int(least),
+        _ptr(v), c_longlong(_rows(v, "v")), _ptr(seq_starts, "seq_starts", torch.int32), c_int(n_seqs), c_int(q.shape[0]), c_int(max_len), c_int(least),
         c_int(nq), c_int(nkv), c_int(hd), c_int(dv or hd), c_float(scale), c_float(cap), c_int(window), c_int(MASKS[mask]),
         c_int(keep), _ptr(slopes, "slopes", torch.float32, allow_none=True), _ptr(sinks, "sinks", torch.float32, allow_none=True),
         gp, gs, _stream()))
@@ -796,8 +799,9 @@ def attn_prefill(out, q, k, v, batch, nq, nkv, hd, scale, cap, window, slopes=No
     use_tc = fast and aligned and bool(_lib().af_attn_prefill_tc_supported(c_int(hd)))
     use_mma = fast and not use_tc and bool(_lib().af_attn_prefill_supported(c_int(hd))) \
         and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v))
-    lens = getattr(batch, "seq_lens", None)
-    if q.dtype == torch.float32 and max(hd, dv or hd) <= 256 and lens and batch.n_seqs <= 65535 and max(lens) >= F32_TILES_FROM:
+    if (q.dtype == torch.float32 and hd <= 256 and (dv or hd) <= 256 and getattr(batch, "max_len", 0) >= F32_TILES_FROM
+            and getattr(batch, "seq_lens", None)):
+        lens = batch.seq_lens
         attn_prefill_f32(out, q, k, v, batch.seq_starts, batch.n_seqs, batch.max_len, nq, nkv, hd, scale, cap, window, slopes, dv,
                          mask, sinks, gate, keep, least=F32_TILES_FROM)
         if min(lens) < F32_TILES_FROM:

@@ -112,3 +112,26 @@ def test_attention_prefill_f32_of_a_step(K):
         out = run(q, u if t is k else k, u if t is v else v, lens)
         assert torch.equal(out[:63 + 70], together[:63 + 70]) and torch.equal(out[263:], together[263:])
         assert not out[63 + 70:263].isfinite().any()
+
+
+def test_attention_prefill_f32_of_many_sequences(K):
+    """More sequences than a warp's lanes, long ones between ones that another kernel takes: a block finds its own, and each long
+    sequence has the bits that it has alone."""
+    gen = torch.Generator().manual_seed(6)
+    lens, nq, nkv, hd, least = [3] * 31 + [200] + [63] * 40 + [64, 1, 300] + [80] * 20 + [5], 3, 1, 64, 64
+    starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    T = starts[-1]
+    q, k, v = (torch.randn(T, n * hd, generator=gen).to(DEV) for n in (nq, nkv, nkv))
+
+    def run(lo, hi, own):
+        out = torch.full((hi - lo, nq * hd), 7.0, device=DEV)
+        at = torch.tensor([sum(own[:i]) for i in range(len(own) + 1)], dtype=torch.int32, device=DEV)
+        K.attn_prefill_f32(out, q[lo:hi], k[lo:hi], v[lo:hi], at, len(own), max(own), nq, nkv, hd, hd ** -0.5, 0.0, 0, least=least)
+        return out
+
+    out = run(0, T, lens)
+    for lo, n in zip(starts, lens):
+        if n < least:
+            assert bool((out[lo:lo + n] == 7.0).all())
+        else:
+            assert torch.equal(out[lo:lo + n], run(lo, lo + n, [n]))
