@@ -63,9 +63,10 @@ add_tanh_norm_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_part
 }
 
 // Four elements a thread (rows and weights of whole 16-byte pieces).  A decode step's few rows wait for latencies: the
-// weights are asked for before the wait, every load behind it at once, in narrow blocks on many SMs (with the products of heads below, a step of eight
-// sequences through ten runs of Banitar 880 -> 833 us).
-template <typename TA, typename TY>
+// weights are asked for before the wait, every load behind it at once, in narrow blocks on many SMs (with the products of heads, a step of eight
+// sequences through ten runs of Banitar 880 -> 833 us).  The rows of a prompt keep the loads of one partial sum in flight (IN): sixteen
+// took the registers of half the warps (2,048 rows of 4,096 35.5 -> 23.9 us).
+template <typename TA, typename TY, int IN>
 __global__ void __launch_bounds__(256)
 add_tanh_norm4_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_parts, size_t part_stride,
                       const float* __restrict__ w_post, const float* __restrict__ b_post, float alpha_post,
@@ -84,7 +85,7 @@ add_tanh_norm4_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_par
   a = pdl_fresh(a);
   float4 v = get4(x + at), t;
   if constexpr (sizeof(TA) == 4) {
-    t = sum_parts4<16>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
+    t = sum_parts4<IN>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
   } else {
     const uint2 raw = *reinterpret_cast<const uint2*>(a + at);
     t = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
@@ -116,13 +117,20 @@ AF_EXPORT int af_add_tanh_norm(float* x, const void* a, int a_dtype, int n_parts
   const bool vec = hidden % 4 == 0 && part_stride % 4 == 0 &&
                    (((uintptr_t)x | (uintptr_t)a | (uintptr_t)y | (uintptr_t)w_post | (uintptr_t)b_post | (uintptr_t)w_next | (uintptr_t)b_next) & 15) == 0;
   const size_t threads = vec ? total / 4 : total;
-  const unsigned block = threads <= 64 * 1024 ? 64 : 256;
+  // (narrow blocks where the tensor cores' product follows; in front of the CUDA cores' product of 32-bit rows, whose blocks find less room beside
+  // many of them, they cost a decode step of eight sequences 70 of 1,100 us)
+  const bool few = threads <= 64 * 1024;
+  const unsigned block = few && y_dtype == AF_BF16 ? 64 : 256;
   const size_t blocks = (threads + block - 1) / block;
   AF_REQUIRE(blocks < (1ull << 31), "af_add_tanh_norm: too many rows");
-#define AF_ATN(KERNEL, TA, TY)                                                                                \
-  af_launch(KERNEL<TA, TY>, dim3((unsigned)blocks), dim3(block), 0, stream, x, (const TA*)a, n_parts,         \
-            (size_t)part_stride, w_post, b_post, alpha_post, (TY*)y, w_next, b_next, alpha_next, hidden, total)
-  AF_DISPATCH_DTYPE(a_dtype, TA, AF_DISPATCH_DTYPE(y_dtype, TY, if (vec) AF_ATN(add_tanh_norm4_kernel, TA, TY); else AF_ATN(add_tanh_norm_kernel, TA, TY)));
+  auto launch = [&](auto kernel, auto* ap, auto* yp) {
+    af_launch(kernel, dim3((unsigned)blocks), dim3(block), 0, stream, x, ap, n_parts, (size_t)part_stride, w_post, b_post, alpha_post, yp, w_next,
+              b_next, alpha_next, hidden, total);
+  };
+#define AF_ATN(...) launch(__VA_ARGS__, (const TA*)a, (TY*)y)
+  AF_DISPATCH_DTYPE(a_dtype, TA, AF_DISPATCH_DTYPE(y_dtype, TY, if (!vec) AF_ATN(add_tanh_norm_kernel<TA, TY>);
+                                                   else if (few) AF_ATN(add_tanh_norm4_kernel<TA, TY, 16>);
+                                                   else AF_ATN(add_tanh_norm4_kernel<TA, TY, 1>)));
 #undef AF_ATN
   AF_CHECK_LAUNCH("af_add_tanh_norm");
 }
