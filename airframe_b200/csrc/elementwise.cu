@@ -167,7 +167,7 @@ rmsnorm_row_kernel(TY* __restrict__ y, const float* __restrict__ x, const float*
     }
     ss += xv[v].x * xv[v].x + xv[v].y * xv[v].y + xv[v].z * xv[v].z + xv[v].w * xv[v].w;
   }
-  ss = block_sum(ss, scratch);
+  ss = block_sum<false, true>(ss, scratch);
   const float inv = rsqrtf(ss / (float)hidden + eps);
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
@@ -636,7 +636,7 @@ add_scaled_rmsnorm_row_kernel(float* __restrict__ x, const void* __restrict__ a,
     ss += xv[v][0] * xv[v][0] + xv[v][1] * xv[v][1] + xv[v][2] * xv[v][2] + xv[v][3] * xv[v][3];
   }
   if (y == nullptr) return;
-  ss = block_sum(ss, scratch);
+  ss = block_sum<false, true>(ss, scratch);
   const float inv = rsqrtf(ss / (float)hidden + eps);
 #pragma unroll
   for (int v = 0; v < NV; ++v) {

@@ -195,10 +195,11 @@ norm_of_sum_kernel(LnSumArgs p) {
 // Rows of whole groups of four: a thread keeps NV groups in registers and every load of a group is in flight before
 // the first sum.  Few rows (a decode step): one group a thread, the weights and the state asked for before the wait for
 // the kernel in front; many rows (MANY): two groups a thread, the weights read where they are used (L1 holds them).
-// IN: partial sums in flight at once (16 where the block leaves room for them: rows of up to 1,280; MANY: the first, then four at
-// a time: with four from the first on 999 rows of 2,304 took 17.5 us against 15.9).
-template <typename TY, int NV, bool MANY, bool POST, int IN = MANY ? 0 : 4>
-__global__ void __launch_bounds__(MANY ? 512 : IN > 4 ? 320 : 1024, MANY ? 3 : 1)
+// IN: partial sums in flight at once: 16 where the block and the SMs leave room for them (a decode step's rows of up to 1,280), else 0:
+// the first, then four at a time (with four from the first on 999 rows of 2,304 took 17.5 us against 15.9, 16 rows of 4,096 with nine sums 4.8
+// against 4.3, and with sixteen 255 rows of 1,024 with five 4.6 against 3.6).
+template <typename TY, int NV, bool MANY, bool POST, int IN = 0>
+__global__ void __launch_bounds__(MANY ? 512 : IN > 0 ? 320 : 1024, MANY ? 3 : 1)
 norm_of_sum_row_kernel(LnSumArgs p) {
   pdl_launch_dependents();
   __shared__ float scratch[2][32];
@@ -247,7 +248,7 @@ norm_of_sum_row_kernel(LnSumArgs p) {
       s += v[n][u];
     }
   }
-  const float mean = block_sum<true>(s, scratch[0]) / (float)hidden;
+  const float mean = block_sum<true, !MANY>(s, scratch[0]) / (float)hidden;
   float ss = 0.f;
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
@@ -258,7 +259,7 @@ norm_of_sum_row_kernel(LnSumArgs p) {
       ss += on ? v[n][u] * v[n][u] : 0.f;
     }
   }
-  const float inv = 1.f / sqrtf(block_sum<true>(ss, scratch[1]) / (float)hidden + p.eps);
+  const float inv = 1.f / sqrtf(block_sum<true, !MANY>(ss, scratch[1]) / (float)hidden + p.eps);
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
     const int i = (threadIdx.x + n * blockDim.x) * 4;
@@ -425,7 +426,7 @@ AF_EXPORT int af_norm_of_sum(float* x, const void* a, int a_dtype, int a_parts, 
   do {                                                                                                                \
     if (many) af_launch(norm_of_sum_row_kernel<TY, 2, true, P>, dim3(n_rows), dim3(threads), 0, stream, p);           \
     else if (nv == 2) af_launch(norm_of_sum_row_kernel<TY, 2, false, P>, dim3(n_rows), dim3(threads), 0, stream, p);  \
-    else if (threads <= 320 && most > 4) af_launch(norm_of_sum_row_kernel<TY, 1, false, P, 16>, dim3(n_rows), dim3(threads), 0, stream, p); \
+    else if (threads <= 320 && most > 4 && n_rows <= af_sm_count()) af_launch(norm_of_sum_row_kernel<TY, 1, false, P, 16>, dim3(n_rows), dim3(threads), 0, stream, p); \
     else af_launch(norm_of_sum_row_kernel<TY, 1, false, P>, dim3(n_rows), dim3(threads), 0, stream, p);               \
   } while (0)
     if (post) AF_DISPATCH_DTYPE(y_dtype, TY, LN_LAUNCH(TY, true));
