@@ -288,8 +288,25 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const TA* __restrict__ a, int n_pa
     if (!on[v]) continue;
     const size_t at = (size_t)r * hidden + i;
     if constexpr (sizeof(TA) == 4) {
-      const float4 t = sum_parts4<MANY ? 1 : 8>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
-      av[v][0] = t.x, av[v][1] = t.y, av[v][2] = t.z, av[v][3] = t.w;
+      if constexpr (MANY) {
+        const float4 t = sum_parts4<1>(reinterpret_cast<const float*>(a) + at, n_parts, part_stride);
+        av[v][0] = t.x, av[v][1] = t.y, av[v][2] = t.z, av[v][3] = t.w;
+      } else {
+      const float* ap = reinterpret_cast<const float*>(a) + at;
+      for (int p0 = 0; p0 < n_parts; p0 += 8) {
+        float4 t[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          t[u] = p0 + u < n_parts ? *reinterpret_cast<const float4*>(ap + (size_t)(p0 + u) * part_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          av[v][0] += t[u].x;
+          av[v][1] += t[u].y;
+          av[v][2] += t[u].z;
+          av[v][3] += t[u].w;
+        }
+      }
+      }
     } else {
       const uint2 raw = *reinterpret_cast<const uint2*>(a + at);
       av[v][0] = __uint_as_float(raw.x << 16);
@@ -593,8 +610,18 @@ __device__ __forceinline__ void term_group(float* acc, float scale, const void* 
     acc[3] += scale * __uint_as_float(raw.y & 0xffff0000u);
     return;
   }
-  const float4 v = sum_parts4<IN>(static_cast<const float*>(p) + at, n_parts, part_stride);
-  acc[0] += scale * v.x, acc[1] += scale * v.y, acc[2] += scale * v.z, acc[3] += scale * v.w;
+  const float* f = static_cast<const float*>(p) + at;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int p0 = 0; p0 < n_parts; p0 += IN) {
+    float4 t[IN];
+#pragma unroll
+    for (int u = 0; u < IN; ++u)
+      t[u] = p0 + u < n_parts ? *reinterpret_cast<const float4*>(f + (size_t)(p0 + u) * part_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < IN; ++u) v[0] += t[u].x, v[1] += t[u].y, v[2] += t[u].z, v[3] += t[u].w;
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) acc[u] += scale * v[u];
 }
 
 template <typename TY, int NV>
@@ -733,7 +760,7 @@ add_normed_terms_kernel(float* __restrict__ x, const void* __restrict__ a, int a
 // of the terms is issued before the first reduction, and the norms' weights are asked for before the wait for the
 // kernel in front.
 // MANY (the rows of a prompt): as in add_rmsnorm_row_kernel, 32 registers a thread and the weights read where they are
-// used, so that an SM holds seven rows of 2,304 instead of three (20.7 -> 16.8 us).
+// used, so that an SM holds seven rows of 2,304 instead of three (1,700 rows 20.9 -> 17.0 us).
 template <typename TY, int NV, bool MANY = false>
 __global__ void __launch_bounds__(MANY ? 512 : 1024, MANY ? 4 : 1)
 add_normed_terms_row_kernel(float* __restrict__ x, const void* __restrict__ a, int a_dtype, int a_parts, float scale_a,
@@ -836,7 +863,9 @@ AF_EXPORT int af_add_normed_terms(float* x, const void* a, int a_dtype, int a_pa
     // (many rows: two groups a thread, so that more rows share an SM and their phases overlap)
     const int nv = (n_rows >= 256 && hidden >= 1024) || hidden > 4096 ? 2 : 1;
     const int row_threads = ((hidden / 4 + nv - 1) / nv + 31) / 32 * 32;
-    if (nv == 2 && n_rows >= 256 && row_threads <= 512) {
+    // (as soon as the SMs do not hold all rows at once with 64 registers a thread; until then the weights are better asked for at the start:
+    // 300 rows of 2,304 6.9 against 8.4 us, 900 of 1,024 the same, 2,048 11.7 and 10.6)
+    if (nv == 2 && row_threads <= 512 && n_rows > af_sm_count() * (1024 / row_threads)) {
       AF_DISPATCH_DTYPE(y_dtype, TY,
                         af_launch(add_normed_terms_row_kernel<TY, 2, true>, dim3(n_rows), dim3(row_threads), 0, stream, x, a,
                                   a_dtype, a_parts, scale_a, b, b_dtype, b_parts, scale_b, part_stride, w_post, eps_post,
