@@ -1384,7 +1384,8 @@ struct LatentPrepArgs {
   int max_pages, ring_rows;
 };
 
-template <typename T>
+// FEW: a decode step's tokens, several blocks each.
+template <typename T, bool FEW>
 __global__ void __launch_bounds__(256)
 latent_prep_kernel(LatentPrepArgs<T> p) {
   pdl_launch_dependents();
@@ -1392,9 +1393,9 @@ latent_prep_kernel(LatentPrepArgs<T> p) {
   const int t = blockIdx.x, rot = p.rot, rank = p.rank, dim = p.dim;
   // (few tokens: the first of a token's blocks takes the latent row and what goes beside it, the others the heads'
   // queries: 8 tokens 5.8 -> 3.0 us)
-  const bool rows = blockIdx.y == 0, queries = gridDim.y == 1 || blockIdx.y > 0;
-  const int u0 = gridDim.y == 1 ? 0 : ((int)blockIdx.y - 1) * p.heads / ((int)gridDim.y - 1);
-  const int heads = gridDim.y == 1 ? p.heads : (int)blockIdx.y * p.heads / ((int)gridDim.y - 1) - u0;
+  const bool rows = !FEW || blockIdx.y == 0, queries = !FEW || blockIdx.y > 0;
+  const int u0 = FEW ? ((int)blockIdx.y - 1) * p.heads / ((int)gridDim.y - 1) : 0;
+  const int heads = FEW ? (int)blockIdx.y * p.heads / ((int)gridDim.y - 1) - u0 : p.heads;
   const int pos = p.positions[t];
   T* kdst = nullptr;
   if (rows && p.kcache != nullptr && p.kv_src != nullptr) {
@@ -1454,13 +1455,13 @@ latent_prep_kernel(LatentPrepArgs<T> p) {
   const float* x = p.q_src + (size_t)t * p.q_ld;
   auto q_at = [&](int i) {
     float s = x[i];
-#pragma unroll 8
+#pragma unroll FEW ? 8 : 4
     for (int u = 1; u < p.q_parts; ++u) s += x[(size_t)u * p.q_part_stride + i];
     return s;
   };
   T* qr = p.q + (size_t)t * p.q_stride;
   for (int i = threadIdx.x; i < heads * half; i += blockDim.x) {
-    const int u = u0 + i / half, e = i % half;
+    const int w = i / half, e = i - w * half, u = u0 + w;
     const float2 cs = turn(e);
     const int e0 = first_of(e), e1 = second_of(e);
     const float a = q_at(u * (dim + rot) + dim + e0), b = q_at(u * (dim + rot) + dim + e1);
@@ -1468,12 +1469,12 @@ latent_prep_kernel(LatentPrepArgs<T> p) {
     d[e0] = from_f32<T>(a * cs.x - b * cs.y), d[e1] = from_f32<T>(b * cs.x + a * cs.y);
   }
   for (int i = threadIdx.x; i < heads * dim; i += blockDim.x) {
-    const int u = u0 + i / dim, e = i % dim;
+    const int w = i / dim, e = i - w * dim, u = u0 + w;
     qr[(size_t)u * p.pitch + e] = from_f32<T>(q_at(u * (dim + rot) + e));
   }
   const int pad = p.pitch - dim - rot;
   for (int i = threadIdx.x; i < heads * pad; i += blockDim.x) {
-    const int u = u0 + i / pad, e = i % pad;
+    const int w = i / pad, e = i - w * pad, u = u0 + w;
     qr[(size_t)u * p.pitch + dim + rot + e] = from_f32<T>(0.f);
   }
 }
@@ -1506,7 +1507,7 @@ AF_EXPORT int af_latent_prep(void* q, long long q_stride, const float* q_src, lo
     p.table = (const float2*)table, p.positions = positions, p.seq_of_token = seq_of_token, p.slots = slots;            \
     p.len_after = len_after, p.kcache = (T*)kcache, p.page_table = page_table, p.max_pages = max_pages;                 \
     p.ring_rows = ring_rows;                                                                                            \
-    af_launch(latent_prep_kernel<T>, dim3(n_tokens, blocks), dim3(256), 0, stream, p);                                          \
+    af_launch(blocks > 1 ? latent_prep_kernel<T, true> : latent_prep_kernel<T, false>, dim3(n_tokens, blocks), dim3(256), 0, stream, p);   \
   } while (0)
   AF_DISPATCH_DTYPE(dtype, T, LATENT_PREP(T));
 #undef LATENT_PREP
