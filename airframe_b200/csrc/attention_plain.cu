@@ -1566,10 +1566,9 @@ head_project_kernel(T* __restrict__ out, long long out_stride, const T* __restri
 // The same for the few rows of a decode step: a block takes 32 outputs of a head for eight tokens at once, so a
 // weight is read once for all of them; its 256 threads are 8 groups that each take a stretch of the inputs
 // (short chains side by side), joined in group order through shared memory.  Grid (head, 32 outputs, 8 tokens).
-// The first AF_HPF_AHEAD weights of a thread, which are cold, are asked for before the wait for the kernel in front: in
+// The first AHEAD weights of a thread, which are cold, are asked for before the wait for the kernel in front: in
 // memory order behind it, a few at a time, they were most of the kernel's time (9 us at eight tokens, 18 heads).
-#define AF_HPF_AHEAD 32
-template <typename T>
+template <typename T, int AHEAD>
 __global__ void __launch_bounds__(256)
 head_project_few_kernel(T* __restrict__ out, long long out_stride, const T* __restrict__ x, long long x_stride,
                         const T* __restrict__ w, int D, int N, int extra, int x_pitch, int n_tokens,
@@ -1581,9 +1580,9 @@ head_project_few_kernel(T* __restrict__ out, long long out_stride, const T* __re
   const int grp = threadIdx.x >> 5;
   const int per = (D + 7) / 8, d0 = grp * per, d1 = min(D, d0 + per);
   const T* wh = w + (size_t)h * D * N + (n < N ? n : 0);
-  T ahead[AF_HPF_AHEAD];
+  T ahead[AHEAD];
 #pragma unroll
-  for (int i = 0; i < AF_HPF_AHEAD; ++i) ahead[i] = d0 + i < d1 ? wh[(size_t)(d0 + i) * N] : from_f32<T>(0.f);
+  for (int i = 0; i < AHEAD; ++i) ahead[i] = d0 + i < d1 ? wh[(size_t)(d0 + i) * N] : from_f32<T>(0.f);
   pdl_wait();
   x = pdl_fresh(x);
   gate = pdl_fresh(gate);
@@ -1600,7 +1599,7 @@ head_project_few_kernel(T* __restrict__ out, long long out_stride, const T* __re
   __syncthreads();
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < AF_HPF_AHEAD; ++i) {
+  for (int i = 0; i < AHEAD; ++i) {
     if (d0 + i >= d1) break;
     const float wv = to_f32(ahead[i]);
 #pragma unroll
@@ -1608,7 +1607,7 @@ head_project_few_kernel(T* __restrict__ out, long long out_stride, const T* __re
   }
   if (n < N) {
 #pragma unroll 4
-    for (int d = d0 + AF_HPF_AHEAD; d < d1; ++d) {
+    for (int d = d0 + AHEAD; d < d1; ++d) {
       const float wv = to_f32(wh[(size_t)d * N]);
 #pragma unroll
       for (int u = 0; u < 8; ++u) acc[u] += xs[u * D + d] * wv;
@@ -1635,8 +1634,12 @@ AF_EXPORT int af_head_project(void* out, long long out_stride, const void* x, lo
              "af_head_project: bad sizes");
   AF_REQUIRE((size_t)(D + 256) * sizeof(float) <= 48 * 1024, "af_head_project: %d inputs a head beyond 12032", D);
   if (n_tokens <= 64 && (size_t)(8 * D + 2048) * sizeof(float) <= 48 * 1024 && (N + 31) / 32 < 65536) {
+    // (32 weights ahead where a thread has as many and one round of blocks holds all: 4,096 wide, two tokens, both products 19.6 -> 10.1 us a layer, with
+    // eight 12.6; more blocks than that stand behind one another and want their registers: 33 tokens of 18 heads 6.3, with 32 7.3)
+    const dim3 grid(heads, (N + 31) / 32, (n_tokens + 7) / 8);
+    const bool one_round = (long long)grid.x * grid.y * grid.z <= af_sm_count();
     AF_DISPATCH_DTYPE(dtype, T,
-                      af_launch(head_project_few_kernel<T>, dim3(heads, (N + 31) / 32, (n_tokens + 7) / 8), dim3(256),
+                      af_launch(one_round && D > 128 ? head_project_few_kernel<T, 32> : head_project_few_kernel<T, 8>, grid, dim3(256),
                                 (size_t)(8 * D + 2048) * sizeof(float), stream, (T*)out, out_stride, (const T*)x, x_stride,
                                 (const T*)w, D, N, extra, x_pitch, n_tokens, gate, gate_stride));
     AF_CHECK_LAUNCH("af_head_project");

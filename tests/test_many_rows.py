@@ -202,3 +202,61 @@ def test_rotated_rows_behind_two_to_the_31st_cache_row(K):
     assert last * 64 >= 2 ** 31
     assert torch.equal(memory[last, 0], qkv[:, 2 * hd:3 * hd]) and torch.equal(memory[last + 1, 0], qkv[:, 3 * hd:])
     assert bool((memory[last - 1] == 7.0).all()) and bool((memory[last + 2:] == 7.0).all())
+
+
+@pytest.mark.parametrize("what, M, piece, H, parts", [("tanh", 260, 100, 1024, 5), ("normed", 900, 300, 2304, 2), ("of_sum", 200, 90, 1024, 9),
+                                                    ("of_sum", 70, 64, 4096, 3), ("normed", 70, 64, 4096, 3)])
+def test_norms_of_sums_in_steps_of_any_size(K, what, M, piece, H, parts):
+    """Rows of a step together and in pieces that other variants take (registers, loads in flight, blocks): the same bits, and 64 bits
+    beside them."""
+    g = torch.Generator().manual_seed(M)
+    x, a, b = torch.randn(M, H, generator=g), torch.randn(parts, M, H, generator=g), torch.randn(M, H, generator=g).to(torch.bfloat16)
+    w, w2 = torch.randn(H, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
+
+    def run(lo, hi):
+        xd, y = x[lo:hi].to(DEV), torch.empty(hi - lo, H, dtype=torch.bfloat16, device=DEV)
+        ad, bd = a[:, lo:hi].contiguous().to(DEV), b[lo:hi].to(DEV)
+        if what == "tanh":
+            K.add_tanh_norm(xd, ad, w, w2, 0.4, y=y, w_next=w2, b_next=w, alpha_next=1.1)
+        elif what == "normed":
+            K.add_normed_terms(xd, [(ad, 1.0), (bd, 0.5)], w, 1e-5, y=y, w_next=w2, eps_next=1e-6)
+        else:
+            K.norm_of_sum(xd, [(ad, 1.0), (bd, 0.5)], 2.0, w, w2, 1e-5, y=y)
+        return xd, y
+
+    together = run(0, M)
+    for whole, pieces in zip(together, zip(*[run(lo, min(M, lo + piece)) for lo in range(0, M, piece)])):
+        assert torch.equal(whole, torch.cat(pieces))
+    s, w64, v64 = a.double().sum(0), w.double().cpu(), w2.double().cpu()
+    if what == "tanh":
+        want = x.double() + torch.tanh(0.4 * s) * w64 + v64
+    elif what == "normed":
+        s = s + 0.5 * b.double()
+        want = x.double() + s / (s.square().mean(1, keepdim=True) + 1e-5).sqrt() * w64
+    else:
+        s = 2.0 * x.double() + s + 0.5 * b.double()
+        want = (s - s.mean(1, keepdim=True)) / (s.var(1, keepdim=True, unbiased=False) + 1e-5).sqrt() * w64 + v64
+    # (a row's sums of H values in 32 bits, a few roundings)
+    assert (together[0].double().cpu() - want).abs().max() < 1e-5 * want.abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads, D, N", [(18, 64, 192), (4, 520, 128), (3, 129, 40), (18, 192, 128)])
+def test_products_of_heads_of_few_tokens(K, dtype, heads, D, N):
+    """Eight or 32 weights asked for ahead, as the blocks fit one round of the SMs and the inputs are long: the same bits from steps of
+    any number of tokens, and the sums in 64 bits."""
+    g = torch.Generator().manual_seed(D)
+    T = 64
+    x, w = torch.randn(T, heads * D, generator=g).to(dtype), torch.randn(heads, D, N, generator=g).to(dtype)
+
+    def run(lo, hi):
+        out = torch.full((hi - lo, heads * N), float("nan"), dtype=dtype, device=DEV)
+        K.head_project(out, x[lo:hi].to(DEV), w.to(DEV), heads, D, N)
+        return out
+
+    whole = run(0, T)
+    for piece in (1, 8, 33):
+        assert torch.equal(whole, torch.cat([run(lo, min(T, lo + piece)) for lo in range(0, T, piece)]))
+    want = torch.einsum("thd,hdn->thn", x.double().view(T, heads, D), w.double()).reshape(T, -1)
+    # (sums of D products of size one in 32 bits, and the output's rounding)
+    assert (whole.double().cpu() - want).abs().max() < (2e-6 if dtype == torch.float32 else 2.0 ** -7) * D ** 0.5 * 4
