@@ -106,8 +106,8 @@ __global__ void rope_cache_kernel(T* __restrict__ qkv, int row_stride, const flo
 
 // The same for bfloat16 rows without partial sums and half-split pairs over the whole head (head_dim % 8 == 0): a block
 // takes TOK tokens, a thread four pairs of the same place in every head it turns, so that the pairs' angles serve all of them and the
-// loads of all its tokens are under way together.  What bounds a long prompt are latencies, those of the chain slot - page - row in
-// front of a token among them: few blocks of several tokens, all on the chip at once (2,048 tokens, 8 + 4 heads of 256: 15.9 -> 10.0 us).
+// loads of all its tokens are under way together.  What bounds it are latencies, those of the chain slot - page - row in front of a token
+// among them (in steps of 26 layers, 8 + 4 heads of 256, eight pairs a thread before: 900 tokens 8.1 -> 5.1 us a layer, 2,000 15.7 -> 9.0).
 template <int TOK>
 __global__ void __launch_bounds__(256, TOK == 1 ? 6 : 4)
 rope_cache_vec_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride, const int* __restrict__ positions,
@@ -283,8 +283,9 @@ AF_EXPORT int af_rope_cache_write(void* qkv, int dtype, int row_stride, const fl
       ((uintptr_t)vcache & 15) == 0 && n_tokens >= 64) {
     const int per_head = hd / 8, block = 256 / per_head * per_head;
     const float2* tab = ((uintptr_t)table & 15) == 0 ? reinterpret_cast<const float2*>(table) : nullptr;
-    // (several tokens a block as soon as a token a block would take more than one round of the SMs)
-    if (n_tokens > 6 * af_sm_count())
+    // (several tokens a block where the rows come out of memory; before that a block a token is faster, in whatever number of rounds: 2,048 tokens
+    // in a step 9.0 against 10.6 us, 5,120 alone 15.1 and 18.4, 8,192 37 and 34, 16,384 72 and 64)
+    if (n_tokens > 48 * af_sm_count())
       af_launch(rope_cache_vec_kernel<4>, dim3((n_tokens + 3) / 4), dim3(block), 0, stream, (__nv_bfloat16*)qkv, (long long)row_stride,
                 positions, seq_of_token, slots, len_after, inv_freq, tab, nq, nkv, hd, n_tokens, (__nv_bfloat16*)kcache,
                 (__nv_bfloat16*)vcache, page_table, max_pages, ring_rows, keep);
