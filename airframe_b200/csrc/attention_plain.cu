@@ -295,10 +295,10 @@ AF_EXPORT int af_rope_cache_write(void* qkv, int dtype, int row_stride, const fl
                 (__nv_bfloat16*)vcache, page_table, max_pages, ring_rows, keep);
     AF_CHECK_LAUNCH("af_rope_cache_write");
   }
-  // (fewer tokens: a block a token and head keeps more SMs busy and its chains are shorter: 8 tokens of 16 heads of 256 0.7 against 1.6 us,
-  // 63 1.6 and 1.75, 100 2.65 and 2.64, 150 3.5 and 2.3; 24 heads of 64 1.1 and 1.15 at 8 tokens, 1.75 and 1.5 at 64)
+  // (fewer tokens: a block a token and head keeps more SMs busy and its chains are shorter: 8 tokens of 16 heads of 256 0.7 against 1.6 us alone,
+  // 63 1.6 and 1.75, 150 3.5 and 2.3; in steps of 26 layers 100 tokens 5,369 against 5,391 us, 14 prompts of 2 to 21 5,834 and 5,874, 150 tokens 6,259 and 6,235)
   if (dtype == AF_F32 && parts == nullptr && pairing == AF_PAIR_HALF && rot_dim == hd && hd % 8 == 0 && hd <= 2048 && row_stride % 4 == 0 &&
-      (((uintptr_t)qkv | (uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0 && (long long)n_tokens * (nq + 2 * nkv) >= 1536) {
+      (((uintptr_t)qkv | (uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0 && (long long)n_tokens * (nq + 2 * nkv) >= 2400) {
     const int per_head = hd / 8, block = 256 / per_head * per_head;
     af_launch(rope_cache_vec_f32_kernel, dim3(n_tokens), dim3(block), 0, stream, (float*)qkv, (long long)row_stride, positions,
               seq_of_token, slots, len_after, inv_freq,

@@ -29,7 +29,7 @@ def rope_step(K, qkv, pos, nq, nkv, hd, table):
     return qkv, kc, vc
 
 
-@pytest.mark.parametrize("dtype, T, piece", [(torch.bfloat16, 1001, 500), (torch.float32, 400, 1), (torch.float32, 400, 95), (torch.float32, 7, 3)])
+@pytest.mark.parametrize("dtype, T, piece", [(torch.bfloat16, 1001, 500), (torch.float32, 400, 1), (torch.float32, 400, 149), (torch.float32, 7, 3)])
 @pytest.mark.parametrize("nq, nkv, hd", [(4, 2, 64), (3, 1, 8), (8, 4, 256)])
 def test_rotated_rows(K, dtype, T, piece, nq, nkv, hd):
     """Bits do not depend on how many rows a step has nor on where the angles come from; 64 bits beside them."""
