@@ -174,9 +174,10 @@ AF_EXPORT int af_conv_rows(float* u, void* u16, const float* proj, long long ld,
   // (a decode step's few tokens each begin in their slot's history: a value a thread serves them better)
   const bool vec = width % 4 == 0 && ld % 4 == 0 && off_x % 4 == 0 &&
                    (((uintptr_t)u | (uintptr_t)u16 | (uintptr_t)proj | (uintptr_t)bx | (uintptr_t)cw | (uintptr_t)cb | (uintptr_t)state) & 15) == 0;
-  if (taps <= AF_CV_TAPS && n_tokens >= 64 && vec) {
-    af_launch(conv_rows_window4_kernel, dim3((unsigned)((n_tokens + AF_CV_TOKENS - 1) / AF_CV_TOKENS), (unsigned)((width + 511) / 512)),
-              dim3(128), 0, stream, u, (__nv_bfloat16*)u16, proj, ld, off_x, bx, cw, cb, state, seq_of_token, seq_starts,
+  // (fewer of its blocks than SMs: a channel a thread reaches more of them; 64 tokens of 1,024 channels 3.9 against 5.3 us)
+  const dim3 grid4((unsigned)((n_tokens + AF_CV_TOKENS - 1) / AF_CV_TOKENS), (unsigned)((width + 511) / 512));
+  if (taps <= AF_CV_TAPS && n_tokens >= 64 && vec && (long long)grid4.x * grid4.y >= af_sm_count()) {
+    af_launch(conv_rows_window4_kernel, grid4, dim3(128), 0, stream, u, (__nv_bfloat16*)u16, proj, ld, off_x, bx, cw, cb, state, seq_of_token, seq_starts,
               slots, n_tokens, width, taps);
     AF_CHECK_LAUNCH("af_conv_rows");
   }
