@@ -687,6 +687,30 @@ def test_attention_decode_many_short_sequences_share_blocks(K, hd, nq, nkv, wind
 
 
 @pytest.mark.parametrize("plan", [False, True])
+@pytest.mark.parametrize("hd,nq,nkv,n_seq,pages", [(64, 24, 2, 80, (1,)), (128, 8, 4, 40, (1, 2)), (256, 8, 4, 39, (1, 3, 2, 1)), (64, 40, 2, 50, (2, 1, 1))])
+def test_attention_decode_runs_that_begin_and_end_in_a_break(K, hd, nq, nkv, n_seq, pages, plan):
+    """Units of a few pages in runs that count two pages more for every unit: runs begin at either page of a unit's break and
+    behind it, and end there (up to 8 heads a tile and more of them)."""
+    dtype = torch.bfloat16
+    of = [pages[b % len(pages)] for b in range(n_seq)]
+    units, blocks = nkv * ((nq // nkv + 15) // 16), K.sm_count()
+    assert n_seq * units > blocks                                         # (more units than blocks: no even cut)
+    starts = [u for P in of for _ in range(units) for u in range(P + 2)]  # (every position's place in its unit)
+    share = -(-len(starts) // blocks)
+    begins = {starts[g] for g in range(0, len(starts), share)}
+    ends = {starts[g] for g in range(share - 1, len(starts), share)}      # (the last place of a run)
+    assert {0, 1, 2} <= begins and {0, 1, 2} <= ends
+    g = torch.Generator().manual_seed(hd + nq)
+    lens = [64 * (P - 1) + 1 + (13 * b) % 64 for b, P in enumerate(of)]
+    scale = 1.0 / math.sqrt(hd)
+    q = torch.randn(n_seq, nq * hd, generator=g).to(dtype)
+    ks = [(torch.randn(n, nkv, hd, generator=g) * 0.5).to(dtype) for n in lens]
+    vs = [torch.randn(n, nkv, hd, generator=g).to(dtype) for n in lens]
+    out = _decode_case(K, dtype, hd, nq, nkv, 0, 30.0, lens, q, ks, vs, scale, plan=plan)
+    _check_decode(K, out, lens, q, ks, vs, nq, hd, scale, 30.0, 0)
+
+
+@pytest.mark.parametrize("plan", [False, True])
 @pytest.mark.parametrize("n_splits", [1, 2, 3, 5, 9, 64])
 def test_attention_decode_with_any_room_for_partial_results(K, n_splits, plan):
     """The caller says how many partial results a unit may leave; with little room fewer blocks work, and the

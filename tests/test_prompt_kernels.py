@@ -35,6 +35,46 @@ def test_gemm_tensor_cores_token_tiles(K, N, Kd, out_dtype):
                 assert torch.equal(out, first), (M, n_acc, tile)
 
 
+@pytest.mark.parametrize("act", ["gelu_tanh", "silu"])
+@pytest.mark.parametrize("inter, Kd", [(200, 72), (448, 320)])
+def test_gated_products_of_any_token_tile(K, act, inter, Kd):
+    """Every width of a token tile under the gated epilogue, whose halves meet by shuffles: the same bits whatever the tile, and the
+    product in 64 bits within the roundings of its output and the activation's."""
+    gen = torch.Generator().manual_seed(inter)
+    w = (torch.randn(2 * inter, Kd, generator=gen) * 0.05).to(torch.bfloat16)
+    wi = K.interleave_gate_up(w[:inter].to(DEV), w[inter:].to(DEV))
+    f = {"gelu_tanh": lambda z: torch.nn.functional.gelu(z, approximate="tanh"), "silu": torch.nn.functional.silu}[act]
+    for M in (65, 257, 700):
+        x = torch.randn(M, Kd, generator=gen).to(torch.bfloat16)
+        want = f(x.double() @ w[:inter].double().T) * (x.double() @ w[inter:].double().T)
+        x = x.to(DEV)
+        first = torch.full((M, wi.shape[0] // 2), float("nan"), device=DEV, dtype=torch.bfloat16)
+        K.gemm_tc(first, x, wi, gated=True, activation=act)
+        err = (first[:, :inter].double().cpu() - want).abs()
+        assert (err <= 2.0 ** -8 * want.abs() + 1e-5).all(), float(err.max())
+        for n_acc in (1, 2, 4):
+            for tile in range(32, 257, 32 if n_acc == 4 else 16):
+                out = torch.full_like(first, float("nan"))
+                K.gemm_tc(out, x, wi, gated=True, activation=act, n_acc=n_acc, token_tile=tile)
+                assert torch.equal(out[:, :inter], first[:, :inter]), (M, n_acc, tile)
+    K.check_device_errors(DEV)
+
+
+@pytest.mark.parametrize("M, splits", [(129, 3), (300, 2), (520, 4)])
+def test_split_products_of_a_prompt(K, M, splits):
+    """Partial sums of prompts' rows: equal token tiles, as many as of 256, against tiles of 256 and the sums in 64 bits."""
+    N, Kd = 300, 1032
+    gen = torch.Generator().manual_seed(M)
+    x, w = torch.randn(M, Kd, generator=gen).to(torch.bfloat16), (torch.randn(N, Kd, generator=gen) * 0.05).to(torch.bfloat16)
+    out, twin = (torch.full((splits, M, N), float("nan"), device=DEV) for _ in range(2))
+    K.gemm_tc(out, x.to(DEV), w.to(DEV), splits=splits)
+    K.gemm_tc(twin, x.to(DEV), w.to(DEV), splits=splits, n_acc=1, token_tile=256)
+    assert torch.equal(out, twin)
+    want = x.double() @ w.double().T
+    assert ((out.double().sum(0).cpu() - want).abs() <= 2e-6 * want.abs() + 2e-5).all()
+    K.check_device_errors(DEV)
+
+
 def _attend(q, k, v, scale, cap, seen, slopes, sinks, gate):
     """One sequence in 64 bits: q [n, H, d], k [n, G, d], v [n, G, dv]."""
     n, H = q.shape[:2]

@@ -186,6 +186,38 @@ def test_latents_queries_and_cache_rows(K, heads, dim, rot, rank, q_rank, pitch,
     close(again, rows, max(tol, 2e-5))
 
 
+@pytest.mark.parametrize("T", [1, 13, 64])
+@pytest.mark.parametrize("heads,dim,rot,rank,pitch", [(1, 10, 6, 20, 0), (3, 64, 16, 112, 128), (4, 5, 4, 11, 12), (18, 32, 64, 40, 104)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_latents_of_few_tokens(K, heads, dim, rot, rank, pitch, T, dtype):
+    """A token's heads dealt over several blocks, from partial sums and with padding: the same bits as in a step of more than 64 tokens,
+    which gives a token one block, and the sums in 64 bits."""
+    P, more = pitch or dim + rot, 66
+    g = torch.Generator().manual_seed(heads + T)
+    parts, kv_src = torch.randn(3, more, heads * (dim + rot), generator=g).to(DEV), torch.randn(more, rank + rot, generator=g).to(DEV)
+    norm_w, inv = torch.randn(rank, generator=g).to(DEV), (50.0 ** (-torch.arange(0, rot, 2) / rot)).float().to(DEV)
+
+    def run(n):
+        batch = batch_of([n], [0])
+        q = torch.full((n, heads * P), float("nan"), dtype=dtype, device=DEV)
+        row = torch.full((n, rank + rot), float("nan"), dtype=dtype, device=DEV)
+        kv = SimpleNamespace(k=torch.full((2, 1, PAGE, rank + rot), 7.0, dtype=dtype, device=DEV), v=None, page_table=i32([[1, 0]]), ring_rows=0)
+        K.latent_prep(batch, heads, dim, rot, rank, 1e-5, inv, q=q, q_src=parts[:, :n].contiguous(), pitch=pitch, kvrow=row,
+                      kv_src=kv_src[:n], norm_w=norm_w, kv=kv)
+        assert torch.equal(kv.k[1, 0, :n], row[:64]) and bool((kv.k[1, 0, n:] == 7.0).all())
+        return q, row
+
+    few, many = run(T), run(more)
+    for a, b in zip(few, many):
+        assert torch.equal(a, b[:T])
+    x = parts[:, :T].double().cpu().sum(0).view(T, heads, dim + rot)
+    turn = torch.arange(T, dtype=F64)[:, None, None] * inv.double().cpu()
+    lo, hi = x[..., dim: dim + rot // 2], x[..., dim + rot // 2:]
+    ref = torch.zeros(T, heads, P, dtype=F64)
+    ref[..., :dim + rot] = torch.cat([x[..., :dim], lo * turn.cos() - hi * turn.sin(), hi * turn.cos() + lo * turn.sin()], -1)
+    close(few[0].view(T, heads, P), ref, 2e-5 if dtype == torch.float32 else 8e-3)
+
+
 # ---------------------------------------------------------------- retention
 
 def _retention_case(heads, dk, dv, n_rot, lens, seed, scaling=None):
