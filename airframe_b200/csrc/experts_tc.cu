@@ -16,7 +16,7 @@
 //
 //   warp 0      TMA producer (one lane)
 //   warp 1      TMEM allocation, MMA issue (one lane), TMEM release
-//   warps 2..5  epilogue: TMEM -> registers -> global
+//   warps 2..5  epilogue: TMEM -> registers -> global (GATES: 2..9)
 //
 // GATES is the same grouped product put to another use: the two gates of a gated linear recurrence, whose
 // matrices are block-diagonal.  An "expert" is a block of channels, every block takes all rows, its columns of

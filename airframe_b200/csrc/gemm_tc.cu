@@ -43,6 +43,10 @@
 // copies in flight land, releases its TMEM and returns.
 #include "umma.cuh"
 
+extern "C" int af_gemm_tc_pair(void* out, int out_dtype, long long ldo, const void* x, long long ldx, const void* w, long long ldw,
+                               long long n_w_rows, int M, int K, int gated, int act, float cap, int token_tile, int* err,
+                               cudaStream_t stream);
+
 namespace {
 
 constexpr int TC_BM = 128;  // features per CTA = UMMA M
@@ -536,8 +540,8 @@ struct TcPlan {
 // The estimated time in us.  A grid takes whole rounds of its blocks, so that a tile of 256 tokens leaves up to half of the chip
 // or of the last tile idle: 301 rows in two tiles of 256 were 1.7 times the products, 18 x 4 tiles of 999 x 2304 half the
 // SMs.  The constants are a least-squares fit of 120 sizes (M 100 .. 3,000; N x K 1024 x 1024 .. 28672 x 4096) in up to 24 shapes
-// each, within 5 %: a launch, a round, a K block of 64 and what a token adds to it.  Tiles of 64 run two blocks an SM.  Over
-// those sizes the choice takes 0.896 of the time of tiles of 256 (the best shape of each 0.883): 2304 x 2304 at 301 rows 18.8 -> 13.8 us,
+// each (7 % root mean square, short products up to 40 %): a launch, a round, a K block of 64 and what a token adds to it.  Tiles of 64 run two blocks an SM.  Over
+// those sizes the choice takes 0.90 of the time of tiles of 256 (the best shape of each 0.88): 2304 x 2304 at 301 rows 18.8 -> 13.8 us,
 // 3840 x 2304 at 1,712 33.0 -> 27.5, gated 18432 x 2304 at 700 60.9 -> 50.2, 4096 x 2304 at 3,000 57.1 -> 42.3, 11520 x 2304 at 2,048
 // 86.0 -> 76.1.
 float tc_estimate(int n_acc, int bn, int M, long long rows, int K, int sms) {
@@ -614,10 +618,6 @@ AF_EXPORT int af_gemm_tc_token_tile(int M) {
 // blocks of the next product in the stream fit beside it and fetch their first weight tiles while this one still
 // runs; 1 gives it the whole SM; 0 chooses (2 for grids of more than one wave).
 // err: device word set to 1 when a wait inside the kernel ran out of time.
-extern "C" int af_gemm_tc_pair(void* out, int out_dtype, long long ldo, const void* x, long long ldx, const void* w, long long ldw,
-                               long long n_w_rows, int M, int K, int gated, int act, float cap, int token_tile, int* err,
-                               cudaStream_t stream);
-
 AF_EXPORT int af_gemm_tc(void* out, int out_dtype, long long ldo, long long part_stride, const void* x,
                          long long ldx, const void* w, long long ldw, long long n_w_rows, int M, int K, int gated,
                          int act, int n_acc, float cap, int splits, int per_sm, int token_tile, int* err, cudaStream_t stream) {
